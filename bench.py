@@ -494,30 +494,30 @@ def launch_share(profile: str, kernel: str, among: tuple):
 
 
 def cg_roofline(p, prof):
-    """Roofline of the plain path's dominant kernel (CG kernel A) and of a whole CG iteration.
-    Both CG kernels run inside one device-side graph loop, so CUDA events time the iteration;
-    kernel A's duration is that time times its share of the two kernels in the committed ncu
-    launch list of this workload."""
+    """Roofline of the plain path's dominant pass (p, q = A p and p.q) and of a whole CG iteration.
+    The solve is one cooperative launch, so CUDA events time the iteration; the pass's duration
+    is that time times the share of the same work (k_cg_spmv2) in the committed ncu launch list
+    of the form with two kernels an iteration (SULI_NO_COOP=1)."""
     N = p.nx * p.ny * p.nz
     faces = (p.nx + 1) * p.ny * p.nz + p.nx * (p.ny + 1) * p.nz + p.nx * p.ny * (p.nz + 1)
     bytes_spmv = 8 * (4 * N + faces)
-    bytes_upd = 8 * 6 * N
+    bytes_upd = 8 * 5 * N   # e, r, q in, e, r out: the e update's p is read by the first pass
     n_it = max(prof["cg_iterations"], 1)
     t_it = (prof["cg_spmv"]["ms"] + prof["cg_update"]["ms"]) / n_it / 1e3
     share = launch_share("launches_sloshing_256x128x128_fp64", "k_cg_spmv2", ("k_cg_spmv2", "k_cg_update"))
     peak, peak_kind = measured_peaks()
-    it = {"kernels": "k_cg_spmv2 + k_cg_update (one graph loop)", "bytes": bytes_spmv + bytes_upd, "us": t_it * 1e6,
+    it = {"kernels": "k_cg_two (both passes, one cooperative launch a solve)", "bytes": bytes_spmv + bytes_upd, "us": t_it * 1e6,
           "achieved_gbs": (bytes_spmv + bytes_upd) / t_it / 1e9,
           "frac": (bytes_spmv + bytes_upd) / t_it / 1e9 / peak}
     t_spmv = t_it * (share if share else 1.0)
     ach = bytes_spmv / t_spmv / 1e9
     return {
-        "kernel": "k_cg_spmv2 (FP64 CG kernel A, two cells a thread: p = r + beta p, q = A p, p.q)",
+        "kernel": "k_cg_two, first pass (FP64 CG, two cells a thread: p = r + beta p, q = A p, p.q)",
         "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
         "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback 6.65 TB/s",
         "traffic": profiled_traffic("cg_spmv2_256x128x128", N), "algorithmic_bytes_per_launch": bytes_spmv,
         "avg_launch_us": t_spmv * 1e6,
-        "duration": ("CUDA-event time of a CG iteration x k_cg_spmv2's share of the two CG kernels in "
+        "duration": ("CUDA-event time of a CG iteration x k_cg_spmv2's share of the two-kernel form in "
                      "profiles/launches_sloshing_256x128x128_fp64.txt" if share else
                      "CUDA-event time of a whole CG iteration (no launch list to apportion it)"),
         "cg_iteration": it,

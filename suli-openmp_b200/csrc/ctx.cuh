@@ -169,7 +169,12 @@ struct suli_ctx {
     // the inner PCG loop as one graph: a WHILE node repeats two iterations (ping-pong) and a
     // kernel that clears the condition once the inner solve is done
     cudaGraphExec_t pcg_loop = nullptr;
-    cudaGraphExec_t cg_loop = nullptr;   // the plain FP64 CG iterations as one device-side loop
+    // the plain FP64 CG as one cooperative launch (k_cg_coop.cuh): CTAs the device holds at once and
+    // their inboxes; 0 CTAs (the device cannot launch it, or SULI_NO_COOP=1): two kernels an
+    // iteration, launched from the host, whose sums are grouped differently
+    int coop_ctas = 0;
+    long long* coop_slots = nullptr;   // in the arena
+    size_t coop_slot_bytes = 0;
     int pcg_graph_kernels = 0;   // kernels of one inner iteration
     // learned initial guess (suli_attach_nn) and training-pair recording (suli_graddin_record)
     suli_nn* nn = nullptr;
@@ -178,7 +183,7 @@ struct suli_ctx {
     double* nn_e0 = nullptr;                     // e0 of a recorded solve (box layout)
     suli::NNScale* nn_scale = nullptr;
     float *rec_in = nullptr, *rec_target = nullptr;
-    // false (environment SULI_EAGER_LOOPS=1, for per-kernel profiling): the CG and inner PCG
+    // false (environment SULI_EAGER_LOOPS=1, for per-kernel profiling): the inner PCG
     // iterations are launched one by one from the host, two at a time with a check of the
     // device state after each pair, in place of the device-side graph loop; same kernels, same
     // order, same results
@@ -265,7 +270,8 @@ void launch_tempo(suli_ctx* c, int tt, int it);
 void launch_contorno(suli_ctx* c, int nlock);
 void launch_cg_setup(suli_ctx* c);
 void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new);
-void launch_cg_cond(suli_ctx* c, cudaGraphConditionalHandle h);
+size_t coop_ready(suli_ctx* c);
+cudaError_t launch_cg_coop(suli_ctx* c);
 void launch_cg_divcheck(suli_ctx* c);
 int cluster_ready(suli_ctx* c);
 int stream_ready(suli_ctx* c);

@@ -9,7 +9,10 @@
 // deterministic: fixed warp-shuffle trees per block and a fixed-order sum of the block
 // partials done by the last block to finish (no floating-point atomics).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
+#include <cstring>
 #include "advect.cuh"
 #include "ctx.cuh"
 #include "obstacle.cuh"
@@ -1301,12 +1304,6 @@ __global__ void __launch_bounds__(256) k_cg_divcheck(Geo G, const double* __rest
     }
 }
 
-// loop condition of the CG iteration graph: repeat until the state says done
-__global__ void k_cg_cond(cudaGraphConditionalHandle h, const CGState* st) {
-    pdl_wait();
-    cudaGraphSetConditional(h, st->done ? 0u : 1u);
-}
-
 // de-normalisation over the halo box (:268-274)
 __global__ void k_cg_final(Geo G, BC bc, const double* __restrict__ sdv, const double* __restrict__ e,
                            double* prd1, const CGState* st) {
@@ -1392,6 +1389,10 @@ __global__ void k_fill(double* a, long long n, double v) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n) a[q] = v;
 }
+
+}  // namespace suli
+#include "k_cg_coop.cuh"
+namespace suli {
 
 // ------------------------------------------------------------------------------------
 // launchers
@@ -1665,7 +1666,50 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
     pdl_launch(k_cg_update, gb, b, c->stream, G, c->cg_e, c->cg_r, (const double*)p_new, (const double*)c->cg_q, c->cg,
                c->red_partial, c->red_counter);
 }
-void launch_cg_cond(suli_ctx* c, cudaGraphConditionalHandle h) { pdl_launch(k_cg_cond, 1, 1, c->stream, h, c->cg); }
+// The cooperative solve: the register kernel while every cell fits the device's threads, else the
+// two-pass kernel.  Measured per iteration (B200): 25x50x45 5.1 us (17.5 with two launches an
+// iteration), 64x32x48 6.0 (16.5), 57x49x53 7.3 (17.9); above its 151,552 cells the two-pass kernel
+// takes 12.4 us at 64x64x48 (16.8), 15.2 at 80^3 (20.4), 30.7 at 111x110x110 (41.8), 48.5 at 128^3
+// (55.8), 83.8 at 256x128x128 (103.4) and 611 at 512x256x256 (708).
+constexpr int kRegU = 4, kRegNT = 256, kTwoKZ = 2, kTwoNT = 1024;
+// whether the device runs them; returns the inboxes' 8-byte elements
+size_t coop_ready(suli_ctx* c) {
+    c->coop_ctas = 0;
+    c->coop_slot_bytes = 0;
+    if (const char* ev = std::getenv("SULI_NO_COOP"))
+        if (std::strcmp(ev, "1") == 0) return 0;
+    int ok = 0, nsm = 0, a = 0, b = 0;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !ok ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_cg_reg<kRegU, kRegNT>, kRegNT, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_two<kTwoKZ, kTwoNT>, kTwoNT, 0) != cudaSuccess ||
+        a < 1 || b < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    c->coop_ctas = nsm;
+    const size_t n = 3 * (size_t)nsm * coop_pitch(nsm);
+    c->coop_slot_bytes = n * sizeof(long long);
+    return n;
+}
+cudaError_t launch_cg_coop(suli_ctx* c) {
+    const Geo& G = c->g;
+    ProfScope ps(c, SULI_K_CG_SPMV, 1);
+    cudaError_t e = cudaMemsetAsync(c->coop_slots, 0xff, c->coop_slot_bytes, c->stream);   // every slot empty
+    if (e != cudaSuccess) return e;
+    const double *ax = c->cg_ax, *ay = c->cg_ay, *az = c->cg_az;
+    const long long cells = (long long)G.nx * G.ny * G.nz, per = (long long)kRegU * kRegNT;
+    if (cells <= per * c->coop_ctas) {
+        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_slots};
+        return cudaLaunchCooperativeKernel(k_cg_reg<kRegU, kRegNT>, dim3((unsigned)((cells + per - 1) / per)),
+                                           dim3(kRegNT), args, 0, c->stream);
+    }
+    const long long units = (long long)((G.nx + 1) / 2) * G.ny * ((G.nz + kTwoKZ - 1) / kTwoKZ);
+    const long long ctas = std::min<long long>(c->coop_ctas, (units + kTwoNT - 1) / kTwoNT);
+    void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_pb, &c->cg_q, &c->cg_e, &ax, &ay, &az, &c->cg,
+                    &c->coop_slots};
+    return cudaLaunchCooperativeKernel(k_cg_two<kTwoKZ, kTwoNT>, dim3((unsigned)ctas), dim3(kTwoNT), args, 0, c->stream);
+}
 void launch_cg_divcheck(suli_ctx* c) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_CG_FINAL, 1);

@@ -227,9 +227,11 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
     const int n3d = SULI_F_BXX0;
     const int nwork = 18;
     const size_t per = (size_t)c->g.n;
-    c->arena_elems = per * (size_t)(n3d + nwork);
+    const size_t coop = coop_ready(c);   // the cooperative CG's inboxes, after the fields
+    c->arena_elems = per * (size_t)(n3d + nwork) + coop;
     if ((e = cudaMalloc(&c->arena, c->arena_elems * sizeof(double))) != cudaSuccess) return bail(e, "arena");
     if ((e = cudaMemsetAsync(c->arena, 0, c->arena_elems * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
+    c->coop_slots = reinterpret_cast<long long*>(c->arena + per * (size_t)(n3d + nwork));
     for (int f = 0; f < n3d; ++f) c->f[f] = c->arena + per * f;
     double* wk = c->arena + per * n3d;
     double** work[18] = {&c->ls1, &c->ls2, &c->funcs, &c->nrmx, &c->nrmy, &c->nrmz, &c->cg_d, &c->cg_e,
@@ -301,7 +303,6 @@ int suli_destroy(suli_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->pcg_loop) cudaGraphExecDestroy(c->pcg_loop);
-    if (c->cg_loop) cudaGraphExecDestroy(c->cg_loop);
     for (auto& e : c->prof.ev) cudaEventDestroy(e);
     cudaFree(c->arena);
     cudaFree(c->obst_k);
@@ -649,7 +650,7 @@ int suli_contorno(suli_ctx* c, int nlock) {
 }  // extern "C"
 
 namespace {
-// A solver's iterations as one graph launch: a WHILE conditional node whose body is two
+// The inner solve's iterations as one graph launch: a WHILE conditional node whose body is two
 // iterations (the direction vector ping-pongs between two buffers; every kernel reads its
 // scalars from device memory, so the captured parameters never change) and a kernel that clears
 // the condition once the solve has converged or hit its cap.  The GPU iterates without host
@@ -700,18 +701,6 @@ int ensure_pcg_loop(suli_ctx* c) {
     return SULI_OK;
 }
 
-// the plain FP64 CG
-int ensure_cg_loop(suli_ctx* c) {
-    if (c->cg_loop) return SULI_OK;
-    return make_loop_graph(
-        c, &c->cg_loop,
-        [&] {
-            launch_cg_iter(c, c->cg_pa, c->cg_pb);
-            launch_cg_iter(c, c->cg_pb, c->cg_pa);
-        },
-        [&](cudaGraphConditionalHandle h) { launch_cg_cond(c, h); }, "CG graph");
-}
-
 // Mixed-precision solve: FP64 refinement around an FP32 multigrid-preconditioned CG.
 // Buffers of the learned guess and of recorded solves (allocated on first use).
 int ensure_nn_buffers(suli_ctx* c, bool net) {
@@ -751,21 +740,25 @@ void nn_begin(suli_ctx* c) {
 // the divergence test's resumptions, de-normalisation.  `record` takes a training pair
 // (suli_graddin_record).
 int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
-    if (int rg = ensure_cg_loop(c)) return rg;
     launch_cg_setup(c);
     if (record) nn_begin(c);   // recording only: the learned guess needs the refinement loop
     CHECK_LAUNCH(c);
-    // iteration 1 uses p_old = r with beta = 0 (erroppr = erropr, :172); then the device loop
-    launch_cg_iter(c, c->cg_r, c->cg_pa);
+    int done_iters = 0;   // iterations before this run of the loop (resumed solves)
     auto run_loop = [&]() -> int {
-        if (c->use_graphs) {
-            ProfScope ps(c, SULI_K_CG_SPMV, 0);   // kernel launches are counted below, once known
-            CUDA_TRY(c, cudaGraphLaunch(c->cg_loop, c->stream));
-            return SULI_OK;
+        if (c->coop_ctas > 0) {
+            const cudaError_t e = launch_cg_coop(c);
+            if (e == cudaSuccess) return SULI_OK;
+            if (e != cudaErrorCooperativeLaunchTooLarge) CUDA_TRY(c, e);
+            cudaGetLastError();   // a context with fewer SMs than the device (MPS, green contexts)
+            c->coop_ctas = 0;
         }
-        for (;;) {
-            launch_cg_iter(c, c->cg_pa, c->cg_pb);
-            launch_cg_iter(c, c->cg_pb, c->cg_pa);
+        // iteration 1 uses p_old = r with beta = 0 (erroppr = erropr, :172); iteration n writes its
+        // direction to cg_pa for odd n, cg_pb for even n
+        for (int n = done_iters;; n += 2) {
+            double* cur = (n & 1) ? c->cg_pa : c->cg_pb;    // direction n (n >= 1), then n + 2
+            double* nxt = (n & 1) ? c->cg_pb : c->cg_pa;   // direction n + 1
+            launch_cg_iter(c, n == 0 ? c->cg_r : cur, nxt);
+            launch_cg_iter(c, nxt, cur);
             CHECK_LAUNCH(c);
             if (int rr = sync_read(c, c->cg, c->cg_host, sizeof(CGState))) return rr;
             if (c->cg_host[0].done) return SULI_OK;
@@ -779,16 +772,8 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
         CHECK_LAUNCH(c);
         int rr = sync_read(c, c->cg, c->cg_host, sizeof(CGState));
         if (rr != SULI_OK) return rr;
-        const CGState& s = c->cg_host[0];
-        if (s.done) break;
-        // after n iterations the last direction is in cg_pa for odd n, cg_pb for even n; the loop
-        // body starts from cg_pa
-        if (s.iters == 0) {
-            launch_cg_iter(c, c->cg_r, c->cg_pa);
-        } else if (s.iters % 2 == 0) {
-            CUDA_TRY(c, cudaMemcpyAsync(c->cg_pa, c->cg_pb, c->g.n * sizeof(double), cudaMemcpyDeviceToDevice,
-                                        c->stream));
-        }
+        if (c->cg_host[0].done) break;
+        done_iters = c->cg_host[0].iters;
         if (int rl = run_loop()) return rl;
         CHECK_LAUNCH(c);
     }
@@ -799,14 +784,10 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
     if (r != SULI_OK) return r;
     const CGState& s = c->cg_host[0];
     c->prof.cg_iters += s.iters;
-    if (c->use_graphs) {   // the loop ran ceil((iters - 1) / 2) two-iteration bodies (at least one)
-        const long long bodies = std::max(1, s.iters / 2);
-        c->prof.launches[SULI_K_CG_SPMV] += 2 * bodies;
-        c->prof.launches[SULI_K_CG_UPDATE] += 2 * bodies;
-    }
     if (iters) *iters = s.iters;
     if (resid) *resid = (s.bb > 0.) ? std::sqrt(s.rr / s.bb) : 0.;
     if (s.status == SULI_ERR_NAN) return fail(c, SULI_ERR_NAN, "graddin: NaN/Inf in the Poisson solve");
+    if (s.status == SULI_ERR_CUDA) return fail(c, SULI_ERR_CUDA, "graddin: a grid-wide sum's wait ran out");
     return s.status;
 }
 

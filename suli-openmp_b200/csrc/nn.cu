@@ -5,7 +5,7 @@
 // input-gradient (dgrad) convolutions run on the tensor cores: by default the persistent
 // TMA + tcgen05 pipeline (nn_tp.cuh), which also computes the encoder's pooling and the head in
 // its epilogues; the one-tile tcgen05 kernel (nn_tc.cuh) and mma.sync (nn_conv.cuh) remain
-// selectable.  Weight gradients accumulate in FP32 on the CUDA cores.
+// selectable.  Weight gradients run on the tensor cores too (nn_wgrad.cuh).
 //
 // The network maps (residual r~0/s, density feature, previous pressure e0/s) to the scaled
 // correction (e* - e0)/s of the pressure solve, so it is both an initial guess
@@ -25,6 +25,7 @@
 #include "nn_conv.cuh"
 #include "nn_tc.cuh"
 #include "nn_tp.cuh"
+#include "nn_wgrad.cuh"
 
 namespace suli {
 namespace nn {
@@ -161,16 +162,6 @@ __global__ void k_head_bwd(long long V, const __nv_bfloat16* __restrict__ x, con
         for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += sh[threadIdx.x][q];
         part[(long long)blockIdx.x * 17 + threadIdx.x] = s;   // summed in block order by k_sum_parts
     }
-}
-
-// out[q] += sum over the nparts rows of part[row][q], rows in order (a fixed summation order,
-// so a gradient is the same from run to run)
-__global__ void k_sum_parts(long long nparts, long long width, const float* __restrict__ part, float* out) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= width) return;
-    float s = 0.f;
-    for (long long r = 0; r < nparts; ++r) s += part[r * width + q];
-    out[q] += s;
 }
 
 // W'[tap'][ci][co] = W[26 - tap'][co][ci]: weights of the input-gradient convolution
@@ -547,135 +538,6 @@ void conv(suli_nn* N, const Vol& vol, const ConvIn& in, const __nv_bfloat16* W, 
     }
 }
 
-// The weight gradient on the tensor cores (mma.sync m16n8k16, BF16 x BF16 -> FP32).  Per tap it
-// is the GEMM dW_tap (COUT x CIN) += dZ^T (COUT x V) X_tap (V x CIN) over the CTA's chunk of
-// voxels: dZ and the shifted input of kWgTcSub voxels are staged as BF16 rows (voxel-major, rows
-// padded by 8 elements so that ldmatrix reads are free of bank conflicts), A fragments (COUT rows,
-// voxels along K) and B fragments (voxels along K, CIN columns) come from ldmatrix.trans of those
-// rows.  The warps split the 16 x 8 output tiles and, where a layer has fewer tiles than warps,
-// the voxels; the voxel-split partials are added in warp order through shared memory.  Each CTA
-// writes its row of part exactly as k_wgrad does, so the sum over rows is as reproducible.
-constexpr int kWgTcSub = 64;
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2,
-                                                  uint32_t& r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t addr, uint32_t& r0, uint32_t& r1) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-template <int CO16, int CI16>
-__global__ void __launch_bounds__(256) k_wgrad_tc(Vol vol, ConvIn in, const __nv_bfloat16* __restrict__ dz,
-                                                  float* part) {
-    constexpr int COUT = CO16 * 16, CIN = CI16 * 16;
-    constexpr int TN = CIN / 8, TILES = CO16 * TN;
-    constexpr int KW = (TILES < 8 && 8 % TILES == 0) ? 8 / TILES : 1;   // warps sharing a tile's voxels
-    constexpr int TW = 8 / KW;                                           // warps splitting the tiles
-    constexpr int TPW = (TILES + TW - 1) / TW;                           // tiles a warp owns
-    constexpr int RZ = COUT + 8, RX = CIN + 8;
-    __shared__ __align__(16) __nv_bfloat16 sz[kWgTcSub][RZ];
-    __shared__ __align__(16) __nv_bfloat16 sx[kWgTcSub][RX];
-    __shared__ float red[KW > 1 ? (KW - 1) * TW * TPW * 128 : 1];
-    const int tap = blockIdx.y;
-    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dzz = tap / 9 - 1;
-    const long long V = (long long)vol.nx * vol.ny * vol.nz;
-    const long long v0 = (long long)blockIdx.x * kWgChunk;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tw = warp % TW, kw = warp / TW;
-    float acc[TPW][4];
-#pragma unroll
-    for (int i = 0; i < TPW; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    float bacc = 0.f;   // the bias gradient of channel tid (tap 13)
-    const int hxn = (vol.nx + 1) / 2, hyn = (vol.ny + 1) / 2;
-    const uint32_t szu = smem_u32(&sz[0][0]), sxu = smem_u32(&sx[0][0]);
-    for (long long vs = v0; vs < v0 + kWgChunk && vs < V; vs += kWgTcSub) {
-        // stage dZ and the shifted input of kWgTcSub voxels (16-byte vectors, zero outside)
-        for (int q = tid; q < kWgTcSub * (COUT / 8); q += 256) {
-            const int m = q / (COUT / 8), c = (q % (COUT / 8)) * 8;
-            const long long v = vs + m;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (v < V) val = *reinterpret_cast<const uint4*>(dz + v * COUT + c);
-            *reinterpret_cast<uint4*>(&sz[m][c]) = val;
-        }
-        for (int q = tid; q < kWgTcSub * (CIN / 8); q += 256) {
-            const int m = q / (CIN / 8), c = (q % (CIN / 8)) * 8;
-            const long long v = vs + m;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (v < V) {
-                const int x = (int)(v % vol.nx) + dx, y = (int)((v / vol.nx) % vol.ny) + dy,
-                          z = (int)(v / ((long long)vol.nx * vol.ny)) + dzz;
-                if (x >= 0 && x < vol.nx && y >= 0 && y < vol.ny && z >= 0 && z < vol.nz) {
-                    if (c < in.ca) {
-                        const long long vi = in.a_half ? ((long long)(x >> 1) + hxn * ((long long)(y >> 1) + (long long)hyn * (z >> 1)))
-                                                       : ((long long)x + vol.nx * ((long long)y + (long long)vol.ny * z));
-                        val = *reinterpret_cast<const uint4*>(in.a + vi * in.ca + c);
-                    } else {
-                        const long long vi = (long long)x + vol.nx * ((long long)y + (long long)vol.ny * z);
-                        val = *reinterpret_cast<const uint4*>(in.b + vi * in.cb + (c - in.ca));
-                    }
-                }
-            }
-            *reinterpret_cast<uint4*>(&sx[m][c]) = val;
-        }
-        __syncthreads();
-        if (tap == 13 && tid < COUT)
-            for (int m = 0; m < kWgTcSub; ++m) bacc += __bfloat162float(sz[m][tid]);
-        // this warp's K steps (16 voxels each) of the staged block
-        for (int ks = kw; ks < kWgTcSub / 16; ks += KW) {
-            const int vb = ks * 16;
-            // A: lane -> matrix mi = lane / 8 (co + 8 (mi & 1), voxels + 8 (mi >> 1)), row lane % 8
-            const int ar = vb + (lane & 7) + 8 * (lane >> 4), ac = 8 * ((lane >> 3) & 1);
-            // B: lanes 0-15 give the rows of the two 8-voxel halves (x2)
-            const int br = vb + (lane & 15);
-#pragma unroll
-            for (int i = 0; i < TPW; ++i) {
-                const int t = tw + TW * i;
-                if (t < TILES) {
-                    const int co0 = 16 * (t / TN), ci0 = 8 * (t % TN);
-                    uint32_t a0, a1, a2, a3, b0, b1;
-                    ldmatrix_x4_trans(szu + (uint32_t)((ar * RZ + co0 + ac) * 2), a0, a1, a2, a3);
-                    ldmatrix_x2_trans(sxu + (uint32_t)((br * RX + ci0) * 2), b0, b1);
-                    mma_bf16(acc[i], a0, a1, a2, a3, b0, b1);
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // voxel-split warps: add the partials in warp order (kw = 1 .. KW - 1 into kw = 0)
-    if (KW > 1) {
-        if (kw > 0)
-#pragma unroll
-            for (int i = 0; i < TPW; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) red[(((kw - 1) * TW + tw) * TPW + i) * 128 + e * 32 + lane] = acc[i][e];
-        __syncthreads();
-        if (kw == 0)
-            for (int w = 1; w < KW; ++w)
-#pragma unroll
-                for (int i = 0; i < TPW; ++i)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[i][e] += red[(((w - 1) * TW + tw) * TPW + i) * 128 + e * 32 + lane];
-    }
-    float* row = part + (long long)blockIdx.x * (27LL * COUT * CIN + COUT);
-    if (kw == 0) {
-#pragma unroll
-        for (int i = 0; i < TPW; ++i) {
-            const int t = tw + TW * i;
-            if (t >= TILES) continue;
-            const int co0 = 16 * (t / TN), ci0 = 8 * (t % TN);
-            // accumulator: rows lane / 4 (+ 8), columns 2 (lane % 4) + {0, 1}
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int co = co0 + (lane >> 2) + 8 * half, ci = ci0 + 2 * (lane & 3);
-                row[((long long)tap * COUT + co) * CIN + ci] = acc[i][2 * half];
-                row[((long long)tap * COUT + co) * CIN + ci + 1] = acc[i][2 * half + 1];
-            }
-        }
-    }
-    if (tap == 13 && tid < COUT) row[27LL * COUT * CIN + tid] = bacc;
-}
-
 // per-CTA rows of partial sums (k_wgrad, k_head_bwd), grown on demand (training only)
 float* part_buffer(suli_nn* N, long long floats) {
     if (floats > N->part_floats) {
@@ -693,36 +555,68 @@ static bool wgrad_cuda_cores() {
     const char* ev = std::getenv("SULI_WGRAD_CUDA_CORES");
     return ev && std::strcmp(ev, "1") == 0;
 }
+// out[0 .. width) += the sum of the rows of N->part
+void sum_parts(suli_nn* N, long long rows, long long width, float* out) {
+    k_sum_parts<<<(unsigned)((width + 31) / 32), dim3(32, 8), 0, N->stream>>>((int)rows, width, N->part, out);
+}
+// The tensor-core kernel with blocks of 16 MB x 16 NB channels: every column of the volume, cut
+// into as many segments of at least four planes as fill the SMs once
+template <int MB, int NB>
+void wgrad_tc(suli_nn* N, const Vol& vol, const ConvIn& in, int cout, const __nv_bfloat16* dz, float* dw) {
+    using G = WgGeo<MB, NB>;
+    const int cin = in.ca + in.cb;
+    const long long width = 27LL * cout * cin + cout;   // dw then db, contiguous
+    static int ctas[64] = {0};   // CTAs an SM holds
+    if (!ctas[N->device]) {
+        cudaFuncSetAttribute(k_wgrad_tc<MB, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_wgrad_tc<MB, NB>, kWgThreads, G::SMEM) != cudaSuccess)
+            cudaGetLastError();
+        ctas[N->device] = std::max(n, 1);
+    }
+    const int blocks = (cout / (16 * MB)) * (cin / (16 * NB));
+    const long long columns = (long long)((vol.nx + kWgX - 1) / kWgX) * ((vol.ny + kWgY - 1) / kWgY);
+    const long long want = (long long)ctas[N->device] * sm_count(N->device) / (columns * blocks);
+    const int segs = (int)std::max<long long>(1, std::min<long long>(want, vol.nz / 4));
+    int seg = (vol.nz + segs - 1) / segs;
+    if (!G::TOTALS) seg = std::min(seg, G::CHAIN);
+    const long long rows = columns * ((vol.nz + seg - 1) / seg);
+    if (!part_buffer(N, rows * width)) { N->grad_error = true; return; }
+    k_wgrad_tc<MB, NB><<<dim3((unsigned)rows, blocks), kWgThreads, G::SMEM, N->stream>>>(vol, in, cout, dz, seg, N->part);
+    sum_parts(N, rows, width, dw);
+}
 template <int CO16, int CI16>
-void wgrad_launch(suli_nn* N, const Vol& vol, const ConvIn& in, const __nv_bfloat16* dz, float* dw, float* db) {
+void wgrad_cores(suli_nn* N, const Vol& vol, const ConvIn& in, const __nv_bfloat16* dz, float* dw) {
     const long long V = (long long)vol.nx * vol.ny * vol.nz;
     const long long chunks = (V + kWgChunk - 1) / kWgChunk;
-    const long long width = 27LL * (CO16 * 16) * (CI16 * 16) + CO16 * 16;   // dw then db, contiguous
+    const long long width = 27LL * (CO16 * 16) * (CI16 * 16) + CO16 * 16;
     float* part = part_buffer(N, chunks * width);
     if (!part) { N->grad_error = true; return; }
-    const dim3 grid((unsigned)chunks, 27);
-    if (wgrad_cuda_cores())
-        k_wgrad<CO16, CI16><<<grid, 256, 0, N->stream>>>(vol, in, dz, part);
-    else
-        k_wgrad_tc<CO16, CI16><<<grid, 256, 0, N->stream>>>(vol, in, dz, part);
-    // the layer's bias follows its weights in the parameter vector (db == dw + 27 COUT CIN)
-    if (db != dw + 27LL * (CO16 * 16) * (CI16 * 16)) { N->grad_error = true; return; }
-    k_sum_parts<<<nb(width), 256, 0, N->stream>>>(chunks, width, part, dw);
+    k_wgrad<CO16, CI16><<<dim3((unsigned)chunks, 27), 256, 0, N->stream>>>(vol, in, dz, part);
+    sum_parts(N, chunks, width, dw);
 }
-void wgrad(suli_nn* N, const Vol& vol, const ConvIn& in, int cout, const __nv_bfloat16* dz, float* dw, float* db) {
+// dw[27][cout][cin] += the weight gradient, db = dw + 27 cout cin the bias gradient.  Blocks of 32
+// x 32 channels where both counts allow, else 16 output channels with 16 or 48 input ones.
+void wgrad(suli_nn* N, const Vol& vol, const ConvIn& in, int cout, const __nv_bfloat16* dz, float* dw) {
     const int cin = in.ca + in.cb;
-    const int key = (cout / 16) * 100 + cin / 16;
-    switch (key) {
-    case 101: wgrad_launch<1, 1>(N, vol, in, dz, dw, db); break;
-    case 201: wgrad_launch<2, 1>(N, vol, in, dz, dw, db); break;
-    case 202: wgrad_launch<2, 2>(N, vol, in, dz, dw, db); break;
-    case 402: wgrad_launch<4, 2>(N, vol, in, dz, dw, db); break;
-    case 404: wgrad_launch<4, 4>(N, vol, in, dz, dw, db); break;
-    case 604: wgrad_launch<6, 4>(N, vol, in, dz, dw, db); break;
-    case 606: wgrad_launch<6, 6>(N, vol, in, dz, dw, db); break;
-    case 410: wgrad_launch<4, 10>(N, vol, in, dz, dw, db); break;
-    case 206: wgrad_launch<2, 6>(N, vol, in, dz, dw, db); break;
-    case 103: wgrad_launch<1, 3>(N, vol, in, dz, dw, db); break;
+    if (!wgrad_cuda_cores()) {
+        if (cout % 32 == 0 && cin % 32 == 0) wgrad_tc<2, 2>(N, vol, in, cout, dz, dw);
+        else if (cout % 32 == 0) wgrad_tc<2, 1>(N, vol, in, cout, dz, dw);
+        else if (cin % 48 == 0) wgrad_tc<1, 3>(N, vol, in, cout, dz, dw);
+        else wgrad_tc<1, 1>(N, vol, in, cout, dz, dw);
+        return;
+    }
+    switch ((cout / 16) * 100 + cin / 16) {
+    case 101: wgrad_cores<1, 1>(N, vol, in, dz, dw); break;
+    case 201: wgrad_cores<2, 1>(N, vol, in, dz, dw); break;
+    case 202: wgrad_cores<2, 2>(N, vol, in, dz, dw); break;
+    case 402: wgrad_cores<4, 2>(N, vol, in, dz, dw); break;
+    case 404: wgrad_cores<4, 4>(N, vol, in, dz, dw); break;
+    case 604: wgrad_cores<6, 4>(N, vol, in, dz, dw); break;
+    case 606: wgrad_cores<6, 6>(N, vol, in, dz, dw); break;
+    case 410: wgrad_cores<4, 10>(N, vol, in, dz, dw); break;
+    case 206: wgrad_cores<2, 6>(N, vol, in, dz, dw); break;
+    case 103: wgrad_cores<1, 3>(N, vol, in, dz, dw); break;
     default: break;
     }
 }
@@ -797,7 +691,7 @@ void backward(suli_nn* N) {
         if (!part) { N->grad_error = true; return; }
         k_head_bwd<<<nb(N->V[0]), 256, 0, N->stream>>>(N->V[0], N->a[13], N->w + N->off[kConv], N->dout,
                                                       N->gact[13], part);
-        k_sum_parts<<<1, 32, 0, N->stream>>>((long long)nb(N->V[0]), 17, part, N->g + N->off[kConv]);
+        sum_parts(N, nb(N->V[0]), 17, N->g + N->off[kConv]);
     }
     for (int l = kConv - 1; l >= 0; --l) {
         const LayerSpec& L = kLayer[l];
@@ -805,7 +699,7 @@ void backward(suli_nn* N) {
         const long long n = N->V[L.level] * L.cout;
         k_relu_bwd<<<nb(n), 256, 0, N->stream>>>(n, N->a[l], N->gact[l]);
         const ConvIn in = layer_input(N, l);
-        wgrad(N, vol, in, L.cout, N->gact[l], N->g + N->off[l], N->g + N->off[l] + 27LL * L.cout * L.cin);
+        wgrad(N, vol, in, L.cout, N->gact[l], N->g + N->off[l]);   // the bias gradient follows the weights' 
         if (l == 0) break;   // no gradient w.r.t. the network input
         // dX = conv(dZ, flipped W) on the tensor cores
         k_flip_weights<<<nb(27LL * L.cin * L.cout), 256, 0, N->stream>>>(L.cin, L.cout, N->wb + N->off[l], N->wflip);

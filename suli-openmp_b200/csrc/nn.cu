@@ -77,48 +77,96 @@ __global__ void k_pool(Vol fine, int C, const __nv_bfloat16* __restrict__ x, __n
     y[q] = __float2bfloat16(0.125f * s);
 }
 
-// gradient of the pooling: dx[fine] += dy[parent] / 8
-__global__ void k_pool_bwd(Vol fine, int C, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* dx) {
+// Eight channels (16 bytes) a thread in the backward pass's element-wise kernels: they move two to
+// four tensors once and are bound by HBM.  Each leaves its result times the ReLU's derivative
+// (y > 0 of the layer that made the tensor), so no tensor is read again only to be masked.
+struct Ch8 {
+    float v[8];
+};
+__device__ __forceinline__ Ch8 unpack8(uint4 t) {
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+    Ch8 o;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        o.v[2 * e] = __uint_as_float(w[e] << 16);
+        o.v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+    }
+    return o;
+}
+__device__ __forceinline__ uint4 pack8(const Ch8& a) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a.v[2 * e], a.v[2 * e + 1]);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ uint4 masked8(uint4 a, uint4 y) {
+    return make_uint4(a.x & positive2(y.x), a.y & positive2(y.y), a.z & positive2(y.z), a.w & positive2(y.w));
+}
+__device__ __forceinline__ uint4 ld16(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ void st16(__nv_bfloat16* p, uint4 v) { *reinterpret_cast<uint4*>(p) = v; }
+
+// gradient of the pooling and of the pooled layer's ReLU: dx[fine] = (dx[fine] + dy[parent] / 8) (y > 0)
+__global__ void __launch_bounds__(256) k_pool_bwd(Vol fine, int C, const __nv_bfloat16* __restrict__ dy,
+                                                  const __nv_bfloat16* __restrict__ y, __nv_bfloat16* dx) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int C8 = C / 8;
     const long long V = (long long)fine.nx * fine.ny * fine.nz;
-    if (q >= V * C) return;
-    const int c = (int)(q % C);
-    const long long v = q / C;
-    const int x = (int)(v % fine.nx), y = (int)((v / fine.nx) % fine.ny), z = (int)(v / ((long long)fine.nx * fine.ny));
+    if (q >= V * C8) return;
+    const int c = (int)(q % C8) * 8;
+    const long long v = q / C8;
+    const int x = (int)(v % fine.nx), yy = (int)((v / fine.nx) % fine.ny), z = (int)(v / ((long long)fine.nx * fine.ny));
     const int cx = fine.nx / 2, cy = fine.ny / 2;
-    const long long vc = (long long)(x >> 1) + cx * ((long long)(y >> 1) + (long long)cy * (z >> 1));
-    dx[q] = __float2bfloat16(__bfloat162float(dx[q]) + 0.125f * __bfloat162float(dy[vc * C + c]));
+    const long long vc = (long long)(x >> 1) + cx * ((long long)(yy >> 1) + (long long)cy * (z >> 1));
+    Ch8 a = unpack8(ld16(dx + v * C + c));
+    const Ch8 b = unpack8(ld16(dy + vc * C + c));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a.v[e] = a.v[e] + 0.125f * b.v[e];
+    st16(dx + v * C + c, masked8(pack8(a), ld16(y + v * C + c)));
 }
 
-// dz = dy * (y > 0) in place
+// dz = dy * (y > 0) in place (the convolutions without a masking epilogue)
 __global__ void k_relu_bwd(long long n, const __nv_bfloat16* __restrict__ y, __nv_bfloat16* dy) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n && !(__bfloat162float(y[q]) > 0.f)) dy[q] = __float2bfloat16(0.f);
 }
 
-// split the gradient of concat(up(A), B): dA[coarse] = sum of the 8 children (channels < ca);
-// dB[fine] += channels >= ca
-__global__ void k_concat_bwd(Vol fine, int ca, int cb, const __nv_bfloat16* __restrict__ dcat,
-                             __nv_bfloat16* __restrict__ da, __nv_bfloat16* db) {
+// split the gradient of concat(up(A), B): dA[coarse] = sum of the 8 children (channels < ca) times
+// A's ReLU derivative (yA > 0); dB[fine] = the channels >= ca
+__global__ void __launch_bounds__(256) k_concat_bwd(Vol fine, int ca, int cb, const __nv_bfloat16* __restrict__ dcat,
+                                                    const __nv_bfloat16* __restrict__ ya, __nv_bfloat16* __restrict__ da,
+                                                    __nv_bfloat16* __restrict__ db) {
     const int cx = fine.nx / 2, cy = fine.ny / 2, cz = fine.nz / 2;
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long Vc = (long long)cx * cy * cz, Vf = (long long)fine.nx * fine.ny * fine.nz;
-    const int C = ca + cb;
-    if (q < Vc * ca) {
-        const int c = (int)(q % ca);
-        const long long vc = q / ca;
+    const int C = ca + cb, A8 = ca / 8, B8 = cb / 8;
+    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < Vc * A8) {
+        const int c = (int)(q % A8) * 8;
+        const long long vc = q / A8;
         const int X = (int)(vc % cx), Y = (int)((vc / cx) % cy), Z = (int)(vc / ((long long)cx * cy));
-        float s = 0.f;
+        uint4 t[8];
+#pragma unroll
         for (int d = 0; d < 8; ++d) {
             const int fx = 2 * X + (d & 1), fy = 2 * Y + ((d >> 1) & 1), fz = 2 * Z + (d >> 2);
-            s += __bfloat162float(dcat[((long long)fx + fine.nx * ((long long)fy + (long long)fine.ny * fz)) * C + c]);
+            t[d] = ld16(dcat + ((long long)fx + fine.nx * ((long long)fy + (long long)fine.ny * fz)) * C + c);
         }
-        da[q] = __float2bfloat16(s);
+        Ch8 s = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int d = 0; d < 8; ++d) {
+            const Ch8 a = unpack8(t[d]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s.v[e] += a.v[e];
+        }
+        st16(da + vc * ca + c, masked8(pack8(s), ld16(ya + vc * ca + c)));
+        return;
     }
-    if (q < Vf * cb) {
-        const int c = (int)(q % cb);
-        const long long v = q / cb;
-        db[q] = __float2bfloat16(__bfloat162float(db[q]) + __bfloat162float(dcat[v * C + ca + c]));
+    q -= Vc * A8;
+    if (q < Vf * B8) {
+        const int c = (int)(q % B8) * 8;
+        const long long v = q / B8;
+        st16(db + v * cb + c, ld16(dcat + v * C + ca + c));
     }
 }
 
@@ -132,47 +180,64 @@ __global__ void k_head_fwd(long long V, const __nv_bfloat16* __restrict__ x, con
     for (int c = 0; c < 16; ++c) s += w[c] * __bfloat162float(x[v * 16 + c]);
     out[v] = s;
 }
-// head backward: dx[v][c] = w[c] dout[v]; the block's sums of x[v][c] dout[v] and of dout into
-// part[block][0..16] (k_sum_parts adds them to dw, db)
-__global__ void k_head_bwd(long long V, const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                           const float* __restrict__ dout, __nv_bfloat16* __restrict__ dx, float* part) {
+// head backward: dx[v][c] = w[c] dout[v] times the last layer's ReLU derivative (x > 0); the
+// block's sums of x[v][c] dout[v] and of dout into part[block][0..16] (k_sum_parts adds them to
+// dw, db)
+constexpr int kHeadBlocks = 592;   // four blocks an SM: few rows to add, each thread many voxels
+__global__ void __launch_bounds__(256) k_head_bwd(long long V, const __nv_bfloat16* __restrict__ x,
+                                                  const float* __restrict__ w, const float* __restrict__ dout,
+                                                  __nv_bfloat16* __restrict__ dx, float* part) {
     __shared__ float sh[17][8];
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float g[17];
+    float g[17], wr[16];
 #pragma unroll
     for (int c = 0; c < 17; ++c) g[c] = 0.f;
-    if (v < V) {
-        const float d = dout[v];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            dx[v * 16 + c] = __float2bfloat16(w[c] * d);
-            g[c] = __bfloat162float(x[v * 16 + c]) * d;
+    for (int c = 0; c < 16; ++c) wr[c] = w[c];
+    for (long long v = (long long)blockIdx.x * 256 + threadIdx.x; v < V; v += (long long)gridDim.x * 256) {
+        const float d = dout[v];
+        const uint4 y0 = ld16(x + v * 16), y1 = ld16(x + v * 16 + 8);
+        const Ch8 a = unpack8(y0), b = unpack8(y1);
+        Ch8 o0, o1;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            o0.v[c] = wr[c] * d;
+            o1.v[c] = wr[8 + c] * d;
+            g[c] += a.v[c] * d;
+            g[8 + c] += b.v[c] * d;
         }
-        g[16] = d;
+        st16(dx + v * 16, masked8(pack8(o0), y0));
+        st16(dx + v * 16 + 8, masked8(pack8(o1), y1));
+        g[16] += d;
     }
 #pragma unroll
     for (int c = 0; c < 17; ++c)
         for (int o = 16; o > 0; o >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], o);
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     if (lane == 0)
+#pragma unroll
         for (int c = 0; c < 17; ++c) sh[c][wp] = g[c];
     __syncthreads();
     if (threadIdx.x < 17) {
         float s = 0.f;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += sh[threadIdx.x][q];
-        part[(long long)blockIdx.x * 17 + threadIdx.x] = s;   // summed in block order by k_sum_parts
+        for (int q = 0; q < 8; ++q) s += sh[threadIdx.x][q];
+        part[(long long)blockIdx.x * 17 + threadIdx.x] = s;
     }
 }
 
-// W'[tap'][ci][co] = W[26 - tap'][co][ci]: weights of the input-gradient convolution
-__global__ void k_flip_weights(int cin, int cout, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long n = 27LL * cin * cout;
-    if (q >= n) return;
-    const int co = (int)(q % cout);
-    const int ci = (int)((q / cout) % cin);
-    const int tp = (int)(q / ((long long)cout * cin));
-    wt[q] = w[((long long)(26 - tp) * cout + co) * cin + ci];
+// W'[tap'][ci][co] = W[26 - tap'][co][ci]: weights of the input-gradient convolutions, every layer
+// (blockIdx.y) at its own offset
+struct FlipArgs {
+    int off[kConv], cin[kConv], cout[kConv];
+};
+__global__ void __launch_bounds__(256) k_flip_weights(const __grid_constant__ FlipArgs A, const __nv_bfloat16* __restrict__ w,
+                                                      __nv_bfloat16* __restrict__ wt) {
+    const int l = blockIdx.y, cin = A.cin[l], cout = A.cout[l], n = 27 * cin * cout;
+    w += A.off[l];
+    wt += A.off[l];
+    for (int q = blockIdx.x * 256 + threadIdx.x; q < n; q += gridDim.x * 256) {
+        const int co = q % cout, ci = (q / cout) % cin, tp = q / (cout * cin);
+        wt[q] = w[((26 - tp) * cout + co) * cin + ci];
+    }
 }
 
 // weight gradient of one layer: dW[tap][co][ci] += sum_v X[v + off(tap)][ci] dZ[v][co];
@@ -257,13 +322,14 @@ __global__ void __launch_bounds__(256) k_wgrad(Vol vol, ConvIn in, const __nv_bf
 // squared error L = mean(e^2), e = pred - target; dout = 2 e / V.  The sums are block partials
 // (fixed warp-shuffle tree) folded in block order by k_loss_fold, so the loss is reproducible.
 __global__ void k_loss_sums(long long V, const float* __restrict__ pred, const float* __restrict__ tgt,
-                            double* __restrict__ part) {
+                            double* __restrict__ part, float* __restrict__ dout) {
     __shared__ double sh[2][8];
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double e = 0., e2 = 0.;
     if (v < V) {
         e = (double)pred[v] - (double)tgt[v];
         e2 = e * e;
+        dout[v] = (float)(2.0 / (double)V * e);   // the mean squared error's gradient
     }
     for (int o = 16; o > 0; o >>= 1) {
         e += __shfl_xor_sync(0xffffffffu, e, o);
@@ -296,13 +362,6 @@ __global__ void __launch_bounds__(256) k_loss_fold(int nparts, const double* __r
     }
     if (threadIdx.x == 0) { sums[0] = sh[0][0]; sums[1] = sh[1][0]; }
 }
-__global__ void k_loss_grad(long long V, const float* __restrict__ pred, const float* __restrict__ tgt,
-                            float* __restrict__ dout) {
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= V) return;
-    dout[v] = (float)(2.0 / (double)V * ((double)pred[v] - (double)tgt[v]));
-}
-
 // Adam on the FP32 master weights, then the BF16 copy the convolutions read
 __global__ void k_adam(long long n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, __nv_bfloat16* __restrict__ wb, float lr, float b1, float b2, float eps,
@@ -318,11 +377,6 @@ __global__ void k_adam(long long n, float* __restrict__ w, const float* __restri
         w[q] -= lr * (mq / c1) / (sqrtf(vq / c2) + eps);
     }
     wb[q] = __float2bfloat16(w[q]);
-}
-
-__global__ void k_zero_bf(long long n, __nv_bfloat16* a) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n) a[q] = __float2bfloat16(0.f);
 }
 
 }  // namespace nn
@@ -342,7 +396,7 @@ struct suli_nn {
     long long off[kConv + 1];   // parameter offsets (head at off[kConv])
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     __nv_bfloat16* wb = nullptr;     // BF16 copy, same layout
-    __nv_bfloat16* wflip = nullptr;  // scratch: flipped weights for dgrad
+    __nv_bfloat16* wflip = nullptr;  // flipped weights for dgrad, same offsets
     unsigned char* frozen = nullptr;
     long long step = 0;
     // activations (BF16, channels last)
@@ -522,7 +576,7 @@ bool conv_tp(suli_nn* N, const Vol& vol, const ConvIn& in, const __nv_bfloat16* 
 
 void conv(suli_nn* N, const Vol& vol, const ConvIn& in, const __nv_bfloat16* W, const float* bias, int relu, int cout,
           __nv_bfloat16* out) {
-    if (N->kernel == 0 && conv_tp(N, vol, in, W, bias, relu, cout, out, TpEpi{nullptr, nullptr, nullptr, 1})) return;
+    if (N->kernel == 0 && conv_tp(N, vol, in, W, bias, relu, cout, out, TpEpi{nullptr, nullptr, nullptr, 1, nullptr})) return;
     if (N->kernel == 0 || N->kernel == 2) {
         conv_tc(N, vol, in, W, bias, relu, cout, out);
         return;
@@ -657,7 +711,7 @@ int forward(suli_nn* N, float* out, bool keep) {
         const bool pools = (l == 1 || l == 3 || l == 5);   // pooling after each encoder level but the last
         const __nv_bfloat16* W = N->wb + N->off[l];
         const float* b = N->w + N->off[l] + 27LL * L.cout * L.cin;
-        TpEpi epi{pools ? N->pool[lv] : nullptr, nullptr, nullptr, 1};
+        TpEpi epi{pools ? N->pool[lv] : nullptr, nullptr, nullptr, 1, nullptr};
         if (l == kConv - 1) {
             epi.head_w = N->w + N->off[kConv];
             epi.head_out = out;
@@ -681,47 +735,61 @@ int forward(suli_nn* N, float* out, bool keep) {
     return launches;
 }
 
-// backward from N->dout; accumulates parameter gradients into N->g (zeroed by the caller)
+// dX = conv(dZ, flipped W) of layer l into out, times the ReLU derivative of the layer whose
+// output out's gradient is (mask > 0; null: none): in the pipelined kernel's epilogue
+void dgrad(suli_nn* N, int l, __nv_bfloat16* out, const __nv_bfloat16* mask) {
+    const LayerSpec& L = kLayer[l];
+    const Vol& vol = N->vol[L.level];
+    const ConvIn gin{N->gact[l], L.cout, 0, nullptr, 0};
+    const __nv_bfloat16* W = N->wflip + N->off[l];
+    if (N->kernel == 0 && conv_tp(N, vol, gin, W, nullptr, 0, L.cin, out, TpEpi{nullptr, nullptr, nullptr, 1, mask})) return;
+    conv(N, vol, gin, W, nullptr, 0, L.cin, out);
+    const long long n = N->V[L.level] * L.cin;
+    if (mask) k_relu_bwd<<<nb(n), 256, 0, N->stream>>>(n, mask, out);
+}
+
+// backward from N->dout; accumulates parameter gradients into N->g (zeroed by the caller).
+// N->gact[l] holds the gradient with respect to layer l's convolution output (its ReLU applied).
 void backward(suli_nn* N) {
-    // gradients w.r.t. each layer's output, accumulated where a tensor feeds two consumers
-    for (int l = 0; l < kConv; ++l)
-        k_zero_bf<<<nb(N->V[kLayer[l].level] * kLayer[l].cout), 256, 0, N->stream>>>(N->V[kLayer[l].level] * kLayer[l].cout, N->gact[l]);
+    FlipArgs fa;
+    for (int l = 0; l < kConv; ++l) {
+        fa.off[l] = (int)N->off[l];
+        fa.cin[l] = kLayer[l].cin;
+        fa.cout[l] = kLayer[l].cout;
+    }
+    k_flip_weights<<<dim3(64, kConv), 256, 0, N->stream>>>(fa, N->wb, N->wflip);
     {
-        float* part = part_buffer(N, (long long)nb(N->V[0]) * 17);
+        const int rows = (int)std::min<long long>(kHeadBlocks, nb(N->V[0]));
+        float* part = part_buffer(N, (long long)rows * 17);
         if (!part) { N->grad_error = true; return; }
-        k_head_bwd<<<nb(N->V[0]), 256, 0, N->stream>>>(N->V[0], N->a[13], N->w + N->off[kConv], N->dout,
-                                                      N->gact[13], part);
-        sum_parts(N, nb(N->V[0]), 17, N->g + N->off[kConv]);
+        k_head_bwd<<<rows, 256, 0, N->stream>>>(N->V[0], N->a[13], N->w + N->off[kConv], N->dout, N->gact[13], part);
+        sum_parts(N, rows, 17, N->g + N->off[kConv]);
     }
     for (int l = kConv - 1; l >= 0; --l) {
         const LayerSpec& L = kLayer[l];
         const Vol& vol = N->vol[L.level];
-        const long long n = N->V[L.level] * L.cout;
-        k_relu_bwd<<<nb(n), 256, 0, N->stream>>>(n, N->a[l], N->gact[l]);
         const ConvIn in = layer_input(N, l);
-        wgrad(N, vol, in, L.cout, N->gact[l], N->g + N->off[l]);   // the bias gradient follows the weights' 
+        wgrad(N, vol, in, L.cout, N->gact[l], N->g + N->off[l]);   // the bias gradient follows the weights'
         if (l == 0) break;   // no gradient w.r.t. the network input
-        // dX = conv(dZ, flipped W) on the tensor cores
-        k_flip_weights<<<nb(27LL * L.cin * L.cout), 256, 0, N->stream>>>(L.cin, L.cout, N->wb + N->off[l], N->wflip);
-        ConvIn gin{N->gact[l], L.cout, 0, nullptr, 0};
         if (in.cb > 0) {
             // decoder concat(up(coarse), skip): coarse part -> sum over the 8 children (its only
-            // consumer), skip part accumulates (the skip also feeds the pooling)
-            conv(N, vol, gin, N->wflip, nullptr, 0, L.cin, N->gcat);
+            // consumer); the skip also feeds the pooling, whose gradient is added (and the ReLU
+            // applied) when the encoder's backward reaches it
+            dgrad(N, l, N->gcat, nullptr);
             const int coarse = (l == 8) ? 7 : (l == 10 ? 9 : 11);
             const int skip = (l == 8) ? 5 : (l == 10 ? 3 : 1);
-            const long long nf = N->V[L.level] * in.cb, nc = N->V[L.level + 1] * in.ca;
-            k_concat_bwd<<<nb(nf > nc ? nf : nc), 256, 0, N->stream>>>(vol, in.ca, in.cb, N->gcat, N->gact[coarse],
-                                                                       N->gact[skip]);
+            const long long n = (N->V[L.level + 1] * in.ca + N->V[L.level] * in.cb) / 8;
+            k_concat_bwd<<<nb(n), 256, 0, N->stream>>>(vol, in.ca, in.cb, N->gcat, N->a[coarse], N->gact[coarse],
+                                                       N->gact[skip]);
         } else if (l == 2 || l == 4 || l == 6) {
             // the input was pooled: gradient through the pooling into the encoder output
-            conv(N, vol, gin, N->wflip, nullptr, 0, L.cin, N->gtmp);
+            dgrad(N, l, N->gtmp, nullptr);
             const int src = l - 1, lv = kLayer[src].level;
-            k_pool_bwd<<<nb(N->V[lv] * kLayer[src].cout), 256, 0, N->stream>>>(N->vol[lv], kLayer[src].cout, N->gtmp,
-                                                                             N->gact[src]);
+            k_pool_bwd<<<nb(N->V[lv] * kLayer[src].cout / 8), 256, 0, N->stream>>>(N->vol[lv], kLayer[src].cout, N->gtmp,
+                                                                                 N->a[src], N->gact[src]);
         } else {
             // plain chain: this layer is the only consumer of the previous output
-            conv(N, vol, gin, N->wflip, nullptr, 0, L.cin, N->gact[l - 1]);
+            dgrad(N, l, N->gact[l - 1], N->a[l - 1]);
         }
     }
 }
@@ -817,9 +885,7 @@ int suli_nn_create(int nx, int ny, int nz, int device, suli_nn** out) {
     auto A = [&](cudaError_t e) { ok = ok && (e == cudaSuccess); };
     A(alloc(&N->w, N->nparam)); A(alloc(&N->g, N->nparam)); A(alloc(&N->m, N->nparam)); A(alloc(&N->v, N->nparam));
     A(alloc(&N->wb, N->nparam));
-    long long wmax = 0;
-    for (int l = 0; l < kConv; ++l) wmax = std::max(wmax, 27LL * kLayer[l].cin * kLayer[l].cout);
-    A(alloc(&N->wflip, wmax));
+    A(alloc(&N->wflip, N->nparam));
     A(alloc(&N->in0, N->V[0] * 16));
     for (int l = 0; l < kConv; ++l) {
         A(alloc(&N->a[l], N->V[kLayer[l].level] * kLayer[l].cout));
@@ -905,9 +971,8 @@ int suli_nn_loss_grad(suli_nn* N, const float* d_in3, const float* d_target, dou
     cudaSetDevice(N->device);
     k_pack_input<<<nb(N->V[0]), 256, 0, N->stream>>>(N->V[0], d_in3, N->in0);
     forward(N, N->out, true);
-    k_loss_sums<<<nb(N->V[0]), 256, 0, N->stream>>>(N->V[0], N->out, d_target, N->loss_part);
+    k_loss_sums<<<nb(N->V[0]), 256, 0, N->stream>>>(N->V[0], N->out, d_target, N->loss_part, N->dout);
     k_loss_fold<<<1, 256, 0, N->stream>>>((int)nb(N->V[0]), N->loss_part, N->sums);
-    k_loss_grad<<<nb(N->V[0]), 256, 0, N->stream>>>(N->V[0], N->out, d_target, N->dout);
     cudaMemsetAsync(N->g, 0, N->nparam * 4, N->stream);
     N->grad_error = false;
     backward(N);
@@ -960,7 +1025,7 @@ int suli_nn_conv3d_ex(int nx, int ny, int nz, const void* x, int cin, const void
     const auto* W = static_cast<const __nv_bfloat16*>(w);
     auto* o = static_cast<__nv_bfloat16*>(out);
     auto* po = static_cast<__nv_bfloat16*>(pool_out);
-    const TpEpi epi{po, head_w, head_out, 1};
+    const TpEpi epi{po, head_w, head_out, 1, nullptr};
     if (!(kernel == 0 && conv_tp(&tmp, vol, in, W, bias, relu, cout, o, epi))) {
         conv(&tmp, vol, in, W, bias, relu, cout, o);
         if (po) k_pool<<<nb(V / 8 * cout), 256>>>(vol, cout, o, po);

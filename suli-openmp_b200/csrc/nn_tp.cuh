@@ -78,6 +78,8 @@ struct TpEpi {
     const float* head_w;   // 1x1x1 head, 16 weights + bias (null: none; Cout = 16 only)
     float* head_out;       // head output [V] FP32
     int store;             // 1: store the BF16 activation
+    const __nv_bfloat16* mask;   // backward: the stored values are zeroed where this tensor is not
+                                 // positive (a ReLU's derivative; null: none)
 };
 
 struct TpCfg {
@@ -117,6 +119,11 @@ __device__ __forceinline__ void tp_tma3(uint32_t dst, const CUtensorMap* map, in
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
         : "memory");
+}
+
+// all bits set in each half whose BF16 value is positive
+__device__ __forceinline__ uint32_t positive2(uint32_t v) {
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&v), __nv_bfloat162(__float2bfloat16(0.f), __float2bfloat16(0.f)));
 }
 
 // bounded wait on a phase parity; gives up when another role has aborted
@@ -395,6 +402,13 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
                         rv[2 * e + 1] = __high2float(h2);
                     }
                     const long long vo = (long long)ox + vol.nx * ((long long)oy + (long long)vol.ny * oz);
+                    if (inside && epi.mask) {
+                        const uint4* mp = reinterpret_cast<const uint4*>(epi.mask + vo * cfg.cout + cb);
+                        const uint4 m0 = mp[0], m1 = mp[1];
+                        const uint32_t mm[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) packed[e] &= positive2(mm[e]);
+                    }
                     if (inside && epi.store) {
                         uint4* o = reinterpret_cast<uint4*>(out + vo * cfg.cout + cb);
                         o[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);

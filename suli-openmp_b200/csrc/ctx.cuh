@@ -170,11 +170,10 @@ struct suli_ctx {
     // kernel that clears the condition once the inner solve is done
     cudaGraphExec_t pcg_loop = nullptr;
     // the plain FP64 CG as one cooperative launch (k_cg_coop.cuh): CTAs the device holds at once and
-    // their inboxes; 0 CTAs (the device cannot launch it, or SULI_NO_COOP=1): two kernels an
+    // their work area; 0 CTAs (the device cannot launch it, or SULI_NO_COOP=1): two kernels an
     // iteration, launched from the host, whose sums are grouped differently
     int coop_ctas = 0;
-    long long* coop_slots = nullptr;   // in the arena
-    size_t coop_slot_bytes = 0;
+    double* coop_area = nullptr;   // in the arena
     int pcg_graph_kernels = 0;   // kernels of one inner iteration
     // learned initial guess (suli_attach_nn) and training-pair recording (suli_graddin_record)
     suli_nn* nn = nullptr;

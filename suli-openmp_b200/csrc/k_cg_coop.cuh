@@ -5,104 +5,10 @@
 // whose arithmetic takes 1-2 us.  Here every CTA stays resident for the whole solve and an
 // iteration is two grid-wide sums (p.q, r.r), each also the barrier that publishes r (or p).
 //
-// Grid-wide sum: every CTA has an inbox with one 8-byte slot a CTA.  A CTA writes its partial into
-// its slot of every inbox (release), polls its own inbox until no slot holds the "empty" pattern
-// and adds the partials in CTA order (fixed order, so a run is bit-reproducible): one store and
-// one load latency a sum, no atomics, and no two CTAs poll the same lines (with one shared slot
-// a CTA, polled by all, a sum took 2 us longer at 110 CTAs than at 55).  Three inbox sets take
-// turns: before a CTA publishes in one set it empties its own inbox of the next, which it read two
-// sums ago and which nobody writes before having seen that publication.  Each wait is bounded; a
-// wait that runs out ends the solve with SULI_ERR_CUDA.
 #pragma once
+#include "k_coop.cuh"
 
 namespace suli {
-
-constexpr long long kSlotEmpty = -1;          // all bits set: no partial sum is published as this NaN
-constexpr int kCoopSpin = 1 << 22;            // polls of a bounded wait (each about an L2 latency)
-
-struct CoopSum {
-    long long* slots;   // [3][nctas][pitch], all empty at launch
-    int n;              // CTAs
-    int pitch;          // slots an inbox, rounded up to whole 128-byte lines
-    int round;          // sums done, modulo 3
-    double* sh;         // shared scratch: warp partials, the total, the failure flag
-    bool failed;
-};
-constexpr int kCoopShared = 34;
-__host__ __device__ inline int coop_pitch(int n) { return (n + 15) & ~15; }
-
-template <bool ACQUIRE>
-__device__ __forceinline__ long long slot_load(const long long* p) {
-    long long v;
-    if (ACQUIRE) asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    else asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void slot_store(long long* p, long long v) {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// Sum of v over the grid; every thread gets it.  PUBLISH: every global store of the CTA before the
-// call is visible to every CTA's loads (from L2) after it; without it the sum orders nothing (and
-// waits for no store).  Of two successive sums at least one publishes: its fence also orders the
-// emptied slots, which are emptied one sum after they were read and written again one sum later.
-template <bool PUBLISH>
-__device__ __forceinline__ double coop_sum(CoopSum& S, double v) {
-    const int tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) S.sh[tid >> 5] = v;
-    __syncthreads();
-    if (tid < 32) {
-        v = (lane < nw) ? S.sh[lane] : 0.;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        const int prev = (S.round == 0) ? 2 : S.round - 1;
-        const long long mine = isnan(v) ? 0x7ff8000000000000ll : __double_as_longlong(v);
-        long long* set = S.slots + (long long)S.round * S.n * S.pitch;
-        long long* clear = S.slots + ((long long)prev * S.n + blockIdx.x) * S.pitch;
-        if (!PUBLISH)
-            for (int q = lane; q < S.n; q += 32) slot_store(set + (long long)q * S.pitch + blockIdx.x, mine);
-        for (int q = lane; q < S.n; q += 32) slot_store(clear + q, kSlotEmpty);
-        if (PUBLISH) {
-            __threadfence();
-            for (int q = lane; q < S.n; q += 32) slot_store(set + (long long)q * S.pitch + blockIdx.x, mine);
-        }
-        set += (long long)blockIdx.x * S.pitch;
-        double t = 0.;
-        bool ok = true;
-        for (int q0 = lane; q0 < S.n; q0 += 5 * 32) {   // five slots a lane in flight
-            long long w[5];
-            int spin = 0;
-            bool all;
-            do {
-                all = true;
-#pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    const int q = q0 + 32 * m;
-                    w[m] = (q < S.n) ? slot_load<PUBLISH>(set + q) : 0;
-                }
-#pragma unroll
-                for (int m = 0; m < 5; ++m) all = all && (w[m] != kSlotEmpty);
-            } while (!all && ++spin < kCoopSpin);
-            ok = ok && all;
-#pragma unroll
-            for (int m = 0; m < 5; ++m)
-                if (q0 + 32 * m < S.n) t += __longlong_as_double(w[m]);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        ok = __all_sync(0xffffffffu, ok);
-        if (lane == 0) {
-            S.sh[32] = t;
-            S.sh[33] = ok ? 0. : 1.;
-        }
-    }
-    __syncthreads();
-    S.round = (S.round == 2) ? 0 : S.round + 1;
-    S.failed = S.failed || S.sh[33] != 0.;
-    return S.sh[32];
-}
 
 // the scalars of the solve, the same in every thread
 struct CoopCG {
@@ -141,18 +47,17 @@ __device__ __forceinline__ void coop_store(const CoopCG& s, bool failed, CGState
 // advances itself (p_nb = r_nb + beta p_nb, the owner's expression), so an iteration loads only r
 // at the neighbours and stores only r.  The directions end in cg_pa (resumed solves read it).
 // Cells are numbered along x, so the loads of a warp run along rows.  Bound by the latencies of
-// its two sums and of the neighbours' loads (25x50x45: 5.1 us an iteration, 17.5 with two kernels);
-// four cells a thread, so that fewer CTAs (55 there) take part in the sums.
+// its two sums and of the neighbours' loads (25x50x45: 5.5 us an iteration, 17.5 with two kernels).
 template <int U, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, double* pa, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
-                                                  const double* __restrict__ az, CGState* st, long long* slots) {
+                                                  const double* __restrict__ az, CGState* st, double* work) {
     __shared__ double sh[kCoopShared];
     CoopCG s = coop_load(st);
     if (s.done) return;
     const double thr = st->thr;
     const int mode = st->mode, maxit = st->maxit;
-    CoopSum S{slots, (int)gridDim.x, coop_pitch((int)gridDim.x), 0, sh, false};
+    CoopGrid S(work, sh);
     const int px = G.px, pxy = (int)G.pxy;
     const int total = G.nx * G.ny * G.nz, step = gridDim.x * NT;
     int c[U], nb[U][6];
@@ -203,7 +108,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
                        pn[u][4] * a[u][4] - pn[u][5] * a[u][5];
                 dot += p[u] * q[u];
             }
-        s.dot(coop_sum<false>(S, dot));
+        s.dot(coop_sum(S, dot));
         if (s.done || S.failed) break;
         double rr = 0.;
 #pragma unroll
@@ -214,7 +119,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
                 __stcg(r + c[u], rc[u]);
                 rr += rc[u] * rc[u];
             }
-        s.residual(coop_sum<true>(S, rr), mode, thr, maxit);
+        s.residual(coop_sum(S, rr), mode, thr, maxit);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -225,23 +130,151 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
     if (blockIdx.x == 0 && threadIdx.x == 0) coop_store(s, S.failed, st);
 }
 
+// Small grids whose operator is symmetric: the same iteration in Chronopoulos and Gear's form
+// (J. Comput. Appl. Math. 25, 1989), which needs one grid-wide sum: with w = A~ r,
+//   s = w + beta s (= A~ p),  alpha = r.r / (r.w - beta r.r / alpha_old),
+// r.r and r.w come from one sum after the updates.  A thread keeps e, r, p, s and w of its U cells
+// and r and s at their six neighbours, which it advances itself (the owner's expressions), so an
+// iteration loads only w at the neighbours and stores only w, in two arrays in turn (a CTA may be
+// one sum ahead).  e, p and the coefficients sit in shared memory, the rest in registers.
+// In exact arithmetic the iterates are k_cg_reg's; measured on tanks with density ratio 833, the
+// iteration counts and the true residuals agree down to a relative residual of 1e-12.  An
+// asymmetric operator (a periodic axis with the reference's clamped end faces, 8_derivadas.f90:318-323,
+// when the density varies across it) makes p.A~p another number, so those solves keep k_cg_reg.
+// A resumed solve reads p and s, which end in cg_pa and cg_q.
+// Bound by the latency of its one sum, whose last part the neighbours' loads overlap: 3.9 us an
+// iteration at 25x50x45 where k_cg_reg takes 5.5, 4.1 at 64x32x48 against 6.0.
+template <int U, int NT>
+__global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, double* pa, double* wa, double* wb, double* e,
+                                                  const double* __restrict__ ax, const double* __restrict__ ay,
+                                                  const double* __restrict__ az, CGState* st, double* work) {
+    extern __shared__ double cells[];   // [8 U][NT]: six coefficients, e, p
+    __shared__ double sh[kCoopShared];
+    CoopCG t = coop_load(st);
+    if (t.done) return;
+    const double thr = st->thr;
+    const int mode = st->mode, maxit = st->maxit;
+    CoopGrid S(work, sh);
+    const int px = G.px, pxy = (int)G.pxy;
+    const int total = G.nx * G.ny * G.nz, step = gridDim.x * NT;
+    const bool fresh = (t.iters == 0);
+    int c[U], nb[U][6];
+    double rn[U][6], sn[U][6], rc[U], sc[U], wc[U];
+    double* own = cells + threadIdx.x;   // value v of cell u: own[(8 u + v) NT]
+    double dot = 0.;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int id = blockIdx.x * NT + threadIdx.x + u * step;
+        c[u] = -1;
+        rc[u] = sc[u] = wc[u] = 0.;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) { nb[u][m] = 0; rn[u][m] = sn[u][m] = 0.; }
+        if (id < total) {
+            const int i = id % G.nx + 1, j = (id / G.nx) % G.ny + 1, k = id / (G.nx * G.ny) + 1;
+            const int cc = G.idx32(i, j, k);
+            const Nb o = neighbours(G, bc, i, j, k);
+            c[u] = cc;
+            nb[u][0] = cc + o.xp; nb[u][1] = cc + o.xm; nb[u][2] = cc + o.yp;
+            nb[u][3] = cc + o.ym; nb[u][4] = cc + o.zp; nb[u][5] = cc + o.zm;
+            const double a[6] = {ax[cc + 1], ax[cc], ay[cc + px], ay[cc], az[cc + pxy], az[cc]};
+            rc[u] = r[cc];
+            double q = rc[u];
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                own[(8 * u + m) * NT] = a[m];
+                rn[u][m] = r[nb[u][m]];
+                q = q - rn[u][m] * a[m];
+                if (!fresh) sn[u][m] = wa[nb[u][m]];
+            }
+            if (!fresh) sc[u] = wa[cc];
+            own[(8 * u + 6) * NT] = e[cc];
+            own[(8 * u + 7) * NT] = fresh ? 0. : pa[cc];
+            wc[u] = q;
+            dot += rc[u] * q;
+        }
+    }
+    // w goes to cg_pb first: other CTAs may still read s of a resumed solve in cg_q
+    double *w = wb, *wnext = wa;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (c[u] >= 0) __stcg(w + c[u], wc[u]);
+    double alpha_old = t.alpha;
+    bool first = true;
+    coop_begin(S, 0., dot);
+    for (;;) {
+        double wn[U][6];   // in flight while the partials are added
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c[u] >= 0) {
+#pragma unroll
+                for (int m = 0; m < 6; ++m) wn[u][m] = __ldcg(w + nb[u][m]);
+            }
+        const double2 d = coop_end(S);
+        if (S.failed) break;
+        if (!first) t.residual(d.x, mode, thr, maxit);
+        else if (fresh) t.beta = 0.;
+        first = false;
+        if (t.done) break;
+        t.rr_start = t.rr;
+        t.pq = (t.iters == 0) ? d.y : d.y - t.beta * t.rr / alpha_old;   // p.A~p
+        t.alpha = t.rr / t.pq;
+        if (!isfinite(t.alpha)) { t.status = SULI_ERR_NAN; break; }
+        const double alpha = t.alpha, beta = t.beta;
+        double rr = 0., rw = 0.;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c[u] >= 0) {
+                const double p = rc[u] + beta * own[(8 * u + 7) * NT];
+                own[(8 * u + 7) * NT] = p;
+                own[(8 * u + 6) * NT] = own[(8 * u + 6) * NT] - alpha * p;
+                sc[u] = wc[u] + beta * sc[u];
+                rc[u] = rc[u] - alpha * sc[u];
+                double q = rc[u];
+#pragma unroll
+                for (int m = 0; m < 6; ++m) {
+                    sn[u][m] = wn[u][m] + beta * sn[u][m];
+                    rn[u][m] = rn[u][m] - alpha * sn[u][m];
+                    q = q - rn[u][m] * own[(8 * u + m) * NT];
+                }
+                wc[u] = q;
+                __stcg(wnext + c[u], q);
+                rr += rc[u] * rc[u];
+                rw += rc[u] * q;
+            }
+        alpha_old = alpha;
+        double* x = w;
+        w = wnext;
+        wnext = x;
+        coop_begin(S, rr, rw);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (c[u] >= 0) {
+            r[c[u]] = rc[u];
+            e[c[u]] = own[(8 * u + 6) * NT];
+            pa[c[u]] = own[(8 * u + 7) * NT];
+            wa[c[u]] = sc[u];
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) coop_store(t, S.failed, st);
+}
+
 // Larger grids: the iteration's two passes over units dealt to the threads in turn (a unit is a
 // pair of x cells, 16-byte loads, and a column of KZ planes).  The first pass also applies the
 // previous iteration's e -= alpha p, whose p it reads anyway, so the second only forms r; it
 // takes the units in reverse order, newest in the L2 first.  Iteration n (from 1) writes its
 // direction into pa for odd n, pb for even n.  Bound by the loads a thread's 64 registers keep in
-// flight: 12 passes in 83.8 us at 256x128x128, 4.8 TB/s (the two kernels' 13 passes: 103.4 us).
+// flight: 12 passes in 83.4 us at 256x128x128, 4.8 TB/s (the two kernels' 13 passes: 103.4 us).
 // Measured there: 512 threads of the same 87.7-97, 4 planes a unit 96, 8 planes 105, 1 plane 89.
 template <int KZ, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, double* pa, double* pb, double* q, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
-                                                  const double* __restrict__ az, CGState* st, long long* slots) {
+                                                  const double* __restrict__ az, CGState* st, double* work) {
     __shared__ double sh[kCoopShared];
     CoopCG s = coop_load(st);
     if (s.done) return;
     const double thr = st->thr;
     const int mode = st->mode, maxit = st->maxit;
-    CoopSum S{slots, (int)gridDim.x, coop_pitch((int)gridDim.x), 0, sh, false};
+    CoopGrid S(work, sh);
     const int nx = G.nx, ny = G.ny, nz = G.nz, px = G.px, pxy = (int)G.pxy;
     const int ux = (nx + 1) / 2, uxy = ux * ny, units = uxy * ((nz + KZ - 1) / KZ);
     const int first = blockIdx.x * NT + threadIdx.x, step = gridDim.x * NT;
@@ -306,7 +339,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, doubl
             }
         }
         pending = false;
-        s.dot(coop_sum<true>(S, dot));
+        s.dot(coop_sum(S, dot));
         if (s.done || S.failed) break;
         const double alpha = s.alpha;
         double rr = 0.;
@@ -329,7 +362,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, doubl
             }
         }
         pending = true;
-        s.residual(coop_sum<true>(S, rr), mode, thr, maxit);
+        s.residual(coop_sum(S, rr), mode, thr, maxit);
     }
     if (pending) {   // the last iteration's e -= alpha p
         const double* p = (s.iters & 1) ? pa : pb;

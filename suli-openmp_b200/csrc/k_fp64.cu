@@ -1666,48 +1666,57 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
     pdl_launch(k_cg_update, gb, b, c->stream, G, c->cg_e, c->cg_r, (const double*)p_new, (const double*)c->cg_q, c->cg,
                c->red_partial, c->red_counter);
 }
-// The cooperative solve: the register kernel while every cell fits the device's threads, else the
-// two-pass kernel.  Measured per iteration (B200): 25x50x45 5.1 us (17.5 with two launches an
-// iteration), 64x32x48 6.0 (16.5), 57x49x53 7.3 (17.9); above its 151,552 cells the two-pass kernel
-// takes 12.4 us at 64x64x48 (16.8), 15.2 at 80^3 (20.4), 30.7 at 111x110x110 (41.8), 48.5 at 128^3
-// (55.8), 83.8 at 256x128x128 (103.4) and 611 at 512x256x256 (708).
-constexpr int kRegU = 4, kRegNT = 256, kTwoKZ = 2, kTwoNT = 1024;
-// whether the device runs them; returns the inboxes' 8-byte elements
+// The cooperative solve: a register kernel while every cell fits the device's threads (one sum an
+// iteration where the operator is symmetric, else two), else the two-pass kernel.  Measured per
+// iteration on a B200 (two kernels an iteration in a graph loop in brackets): k_cg_one 3.9 us at
+// 25x50x45 (17.5; k_cg_reg 5.5), 4.1 at 64x32x48 (16.5; 6.0), 5.4 at 57x49x53 (17.9); above its
+// 151,552 cells on 148 SMs k_cg_two 12.9 at 64x64x48 (16.8), 14.9 at 80^3 (20.4), 31.0 at
+// 111x110x110 (41.8), 47.2 at 128^3 (55.8), 83.4 at 256x128x128 (103.4), 617 at 512x256x256 (708).
+constexpr int kRegU = 4, kRegNT = 256, kOneU = 4, kOneNT = 256, kTwoKZ = 2, kTwoNT = 1024;
+static_assert(kRegU * kRegNT == kOneU * kOneNT, "the register kernels hold the same grids");
+constexpr int kOneSmem = 8 * kOneU * kOneNT * (int)sizeof(double);
+static bool cg_symmetric(const suli_ctx* c) { return c->bc.wrapf || !(c->bc.perx || c->bc.pery || c->bc.perz); }
+// whether the device runs them; returns their work area's 8-byte elements
 size_t coop_ready(suli_ctx* c) {
     c->coop_ctas = 0;
-    c->coop_slot_bytes = 0;
     if (const char* ev = std::getenv("SULI_NO_COOP"))
         if (std::strcmp(ev, "1") == 0) return 0;
-    int ok = 0, nsm = 0, a = 0, b = 0;
+    int ok = 0, nsm = 0, a = 0, b = 0, d = 0;
     if (cudaDeviceGetAttribute(&ok, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !ok ||
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_cg_reg<kRegU, kRegNT>, kRegNT, 0) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_two<kTwoKZ, kTwoNT>, kTwoNT, 0) != cudaSuccess ||
-        a < 1 || b < 1) {
+        cudaFuncSetAttribute(k_cg_one<kOneU, kOneNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_cg_one<kOneU, kOneNT>, kOneNT, kOneSmem) != cudaSuccess ||
+        a < 1 || b < 1 || d < 1) {
         cudaGetLastError();
         return 0;
     }
     c->coop_ctas = nsm;
-    const size_t n = 3 * (size_t)nsm * coop_pitch(nsm);
-    c->coop_slot_bytes = n * sizeof(long long);
-    return n;
+    return coop_work(nsm);
 }
 cudaError_t launch_cg_coop(suli_ctx* c) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_CG_SPMV, 1);
-    cudaError_t e = cudaMemsetAsync(c->coop_slots, 0xff, c->coop_slot_bytes, c->stream);   // every slot empty
+    cudaError_t e = cudaMemsetAsync(c->coop_area, 0, sizeof(double), c->stream);   // the arrival counter
     if (e != cudaSuccess) return e;
     const double *ax = c->cg_ax, *ay = c->cg_ay, *az = c->cg_az;
     const long long cells = (long long)G.nx * G.ny * G.nz, per = (long long)kRegU * kRegNT;
+    if (cells <= per * c->coop_ctas && cg_symmetric(c)) {
+        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_q, &c->cg_pb, &c->cg_e, &ax, &ay, &az, &c->cg,
+                        &c->coop_area};
+        return cudaLaunchCooperativeKernel(k_cg_one<kOneU, kOneNT>, dim3((unsigned)((cells + per - 1) / per)),
+                                           dim3(kOneNT), args, kOneSmem, c->stream);
+    }
     if (cells <= per * c->coop_ctas) {
-        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_slots};
+        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_area};
         return cudaLaunchCooperativeKernel(k_cg_reg<kRegU, kRegNT>, dim3((unsigned)((cells + per - 1) / per)),
                                            dim3(kRegNT), args, 0, c->stream);
     }
     const long long units = (long long)((G.nx + 1) / 2) * G.ny * ((G.nz + kTwoKZ - 1) / kTwoKZ);
     const long long ctas = std::min<long long>(c->coop_ctas, (units + kTwoNT - 1) / kTwoNT);
     void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_pb, &c->cg_q, &c->cg_e, &ax, &ay, &az, &c->cg,
-                    &c->coop_slots};
+                    &c->coop_area};
     return cudaLaunchCooperativeKernel(k_cg_two<kTwoKZ, kTwoNT>, dim3((unsigned)ctas), dim3(kTwoNT), args, 0, c->stream);
 }
 void launch_cg_divcheck(suli_ctx* c) {

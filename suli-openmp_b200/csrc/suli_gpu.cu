@@ -227,11 +227,11 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
     const int n3d = SULI_F_BXX0;
     const int nwork = 18;
     const size_t per = (size_t)c->g.n;
-    const size_t coop = coop_ready(c);   // the cooperative CG's inboxes, after the fields
+    const size_t coop = coop_ready(c);   // the cooperative CG's work area, after the fields
     c->arena_elems = per * (size_t)(n3d + nwork) + coop;
     if ((e = cudaMalloc(&c->arena, c->arena_elems * sizeof(double))) != cudaSuccess) return bail(e, "arena");
     if ((e = cudaMemsetAsync(c->arena, 0, c->arena_elems * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
-    c->coop_slots = reinterpret_cast<long long*>(c->arena + per * (size_t)(n3d + nwork));
+    c->coop_area = c->arena + per * (size_t)(n3d + nwork);
     for (int f = 0; f < n3d; ++f) c->f[f] = c->arena + per * f;
     double* wk = c->arena + per * n3d;
     double** work[18] = {&c->ls1, &c->ls2, &c->funcs, &c->nrmx, &c->nrmy, &c->nrmz, &c->cg_d, &c->cg_e,

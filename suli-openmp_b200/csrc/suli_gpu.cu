@@ -75,26 +75,29 @@ int extent(const suli_params* p, int f, int lo[3], int hi[3]) {
     }
 }
 
-// Scatter a dense Fortran-layout block into the padded box and back.
-__global__ void k_scatter(Geo G, const double* __restrict__ src, double* dst, int l0, int l1, int l2, int n0, int n1,
-                          int n2) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long tot = (long long)n0 * n1 * n2;
-    if (q >= tot) return;
-    const int a = (int)(q % n0);
-    const int b = (int)((q / n0) % n1);
-    const int cc = (int)(q / ((long long)n0 * n1));
-    dst[G.idx(l0 + a, l1 + b, l2 + cc)] = src[q];
+// Scatter a dense Fortran-layout block into the padded box and back: a thread a point of 4 rows x 64
+// (no division a point), bound by HBM.
+struct Block3 {
+    int l0, l1, l2, n0, n1, n2;   // first indices, extents
+};
+template <bool SCATTER>
+__global__ void __launch_bounds__(256) k_repack(Geo G, Block3 B, const double* __restrict__ src, double* __restrict__ dst) {
+    const int a = blockIdx.x * 64 + threadIdx.x;
+    if (a >= B.n0) return;
+    for (int cc = blockIdx.z; cc < B.n2; cc += gridDim.z)
+        for (int b = blockIdx.y * 4 + threadIdx.y; b < B.n1; b += gridDim.y * 4) {
+            const long long q = a + (long long)B.n0 * (b + (long long)B.n1 * cc), p = G.idx(B.l0 + a, B.l1 + b, B.l2 + cc);
+            if (SCATTER) dst[p] = src[q];
+            else dst[q] = src[p];
+        }
 }
-__global__ void k_gather(Geo G, const double* __restrict__ src, double* dst, int l0, int l1, int l2, int n0, int n1,
-                         int n2) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long tot = (long long)n0 * n1 * n2;
-    if (q >= tot) return;
-    const int a = (int)(q % n0);
-    const int b = (int)((q / n0) % n1);
-    const int cc = (int)(q / ((long long)n0 * n1));
-    dst[q] = src[G.idx(l0 + a, l1 + b, l2 + cc)];
+template <bool SCATTER>
+void repack(suli_ctx* c, int field, const double* src, double* dst) {
+    int lo[3], hi[3];
+    extent(&c->P, field, lo, hi);
+    const Block3 B{lo[0], lo[1], lo[2], hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1};
+    const dim3 grid((B.n0 + 63) / 64, std::min((B.n1 + 3) / 4, 65535), std::min(B.n2, 65535));
+    k_repack<SCATTER><<<grid, dim3(64, 4), 0, c->stream>>>(c->g, B, src, dst);
 }
 
 int sync_read(suli_ctx* c, const void* dev, void* host, size_t bytes) {
@@ -349,6 +352,17 @@ static bool host_memory(const void* p) {
     return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
 }
 
+// memory of the context's own GPU that a kernel can read and write in place of a staged copy
+static bool own_memory(const suli_ctx* c, const void* p) {
+    cudaPointerAttributes a{};
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(double) != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == c->device;
+}
+
 int suli_upload(suli_ctx* c, int field, const double* host) {
     if (!c || !host || field < 0 || field >= SULI_F_COUNT) return fail(c, SULI_ERR_ARG, "upload: bad field");
     cudaSetDevice(c->device);
@@ -369,10 +383,12 @@ int suli_upload(suli_ctx* c, int field, const double* host) {
                 if (host[q] != 0.0) { c->tf_active = true; break; }
         }
     }
-    // stage through the CG q buffer (same size class as any field, free between calls)
-    double* stage = c->cg_q;
-    CUDA_TRY(c, cudaMemcpyAsync(stage, host, n * sizeof(double), cudaMemcpyDefault, c->stream));
-    k_scatter<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->g, stage, c->f[field], lo[0], lo[1], lo[2], n0, n1, n2);
+    if (own_memory(c, host)) {
+        repack<true>(c, field, host, c->f[field]);
+    } else {   // stage through the CG q buffer (same size class as any field, free between calls)
+        CUDA_TRY(c, cudaMemcpyAsync(c->cg_q, host, n * sizeof(double), cudaMemcpyDefault, c->stream));
+        repack<true>(c, field, c->cg_q, c->f[field]);
+    }
     CHECK_LAUNCH(c);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return SULI_OK;
@@ -390,10 +406,10 @@ int suli_download(suli_ctx* c, int field, double* host) {
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         return SULI_OK;
     }
-    double* stage = c->cg_q;
-    k_gather<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->g, c->f[field], stage, lo[0], lo[1], lo[2], n0, n1, n2);
+    const bool direct = own_memory(c, host);
+    repack<false>(c, field, c->f[field], direct ? host : c->cg_q);
     CHECK_LAUNCH(c);
-    CUDA_TRY(c, cudaMemcpyAsync(host, stage, n * sizeof(double), cudaMemcpyDefault, c->stream));
+    if (!direct) CUDA_TRY(c, cudaMemcpyAsync(host, c->cg_q, n * sizeof(double), cudaMemcpyDefault, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return SULI_OK;
 }
@@ -1029,13 +1045,8 @@ struct StepIO {
 };
 
 static int io_scatter(suli_ctx* c, int slot, int field) {
-    int lo[3], hi[3];
-    extent(&c->P, field, lo, hi);
-    const int n0 = hi[0] - lo[0] + 1, n1 = hi[1] - lo[1] + 1, n2 = hi[2] - lo[2] + 1;
-    const size_t n = (size_t)n0 * n1 * n2;
     CUDA_TRY(c, cudaStreamWaitEvent(c->stream, c->io_ev[slot], 0));
-    k_scatter<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->g, c->io_stage[slot], c->f[field], lo[0], lo[1],
-                                                                   lo[2], n0, n1, n2);
+    repack<true>(c, field, c->io_stage[slot], c->f[field]);
     CHECK_LAUNCH(c);
     return SULI_OK;
 }
@@ -1045,8 +1056,7 @@ static int io_send(suli_ctx* c, int slot, int field, double* host) {
     extent(&c->P, field, lo, hi);
     const int n0 = hi[0] - lo[0] + 1, n1 = hi[1] - lo[1] + 1, n2 = hi[2] - lo[2] + 1;
     const size_t n = (size_t)n0 * n1 * n2;
-    k_gather<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->g, c->f[field], c->io_stage[slot], lo[0], lo[1],
-                                                                  lo[2], n0, n1, n2);
+    repack<false>(c, field, c->f[field], c->io_stage[slot]);
     CHECK_LAUNCH(c);
     CUDA_TRY(c, cudaEventRecord(c->io_ev[slot], c->stream));
     CUDA_TRY(c, cudaStreamWaitEvent(c->io_out, c->io_ev[slot], 0));

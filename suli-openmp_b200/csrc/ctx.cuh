@@ -136,7 +136,7 @@ struct suli_ctx {
     // mixed-precision solve (precision = 1)
     std::vector<suli::MGLevel> mg;
     float *pc_x = nullptr, *pc_r = nullptr, *pc_pa = nullptr, *pc_pb = nullptr, *pc_q = nullptr;
-    float* pc_r2 = nullptr;   // the inner residual is updated from one buffer into the other
+    float* pc_r2 = nullptr;   // second inner residual, where the update runs inside the pre-smoothing
     double* cg_e2 = nullptr;
     double* cg_sd = nullptr;    // sqrt(d), stored once per solve (ghost values, the refinement's scaling)
     double* cg_isd = nullptr;   // 1/sqrt(d) (the coefficient scaling)
@@ -279,7 +279,9 @@ void launch_cg_final(suli_ctx* c, const double* e);
 // ---- mixed-precision solve (k_mixed.cu) ----
 void launch_mx_setup(suli_ctx* c);
 void launch_mx_residual(suli_ctx* c, const double* e_in, double* e_out, bool apply);
-void launch_pcg_init(suli_ctx* c, int maxit);
+void launch_pcg_begin(suli_ctx* c, int maxit);
+void launch_pcg_pair(suli_ctx* c);
+int pcg_bodies(const suli_ctx* c, int iters);
 // the loop condition of the inner-solve graph: non-zero while the inner solve is not done
 void launch_pcg_cond(suli_ctx* c, cudaGraphConditionalHandle h);
 void launch_vcycle(suli_ctx* c, const float* f0, bool pre_done = false);
@@ -289,8 +291,6 @@ void launch_nn_features16(suli_ctx* c, void* in16);
 void launch_nn_features16_at(suli_ctx* c, void* in16, const double* r, const double* e);
 void launch_nn_step(suli_ctx* c, const float* out, double* e);
 void launch_nn_target(suli_ctx* c, const double* e_star, float* target);
-void launch_pcg_iter(suli_ctx* c, const float* p_old, float* p_new, const float* r_old, float* r_new,
-                     bool x_zero = false);
 int pcg_iter_kernels(const suli_ctx* c);
 int vcycle_kernels(const suli_ctx* c);
 void launch_posdin(suli_ctx* c);

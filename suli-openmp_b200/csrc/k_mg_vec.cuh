@@ -403,15 +403,15 @@ __global__ void __launch_bounds__(256, KZ == 2 ? 4 : 3) k_pcgv_spmvc(Geo G, BC b
     }
 }
 
-// x += alpha p (x_zero: x = alpha p, the pass's first update), r -= alpha q, r.r and the inner stop
-// test (k_pcg_updc)
-__global__ void __launch_bounds__(256) k_pcgv_updc(Geo G, float* __restrict__ x, const float* __restrict__ r,
-                                                   float* __restrict__ r_out, const float* __restrict__ p,
-                                                   const float* __restrict__ qv, PCGState* st, double* partial,
-                                                   unsigned int* counter, int x_zero) {
+// x += alpha p (the first iteration: x = alpha p), r -= alpha q, r.r and the inner stop test
+// (k_pcg_updc)
+__global__ void __launch_bounds__(256) k_pcgv_updc(Geo G, float* __restrict__ x, float* __restrict__ r,
+                                                   const float* __restrict__ p, const float* __restrict__ qv,
+                                                   PCGState* st, double* partial, unsigned int* counter) {
     pdl_wait();
     if (st->done) return;
     const float alpha = (float)st->alpha;
+    const bool x_zero = st->iters == 0;
     const int i0 = kVX * (blockIdx.x * blockDim.x + threadIdx.x) + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k0 = blockIdx.z * kKZU + 1;
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256) k_pcgv_updc(Geo G, float* __restrict__ x,
                 rr += (double)ro[e] * (double)ro[e];
             }
             st4(x, c, xo);
-            st4(r_out, c, ro);
+            st4(r, c, ro);
         }
     }
     double t, u;

@@ -508,13 +508,14 @@ __global__ void __launch_bounds__(256) k_pcg_spmvc(Geo G, BC bc, const float* __
 }
 
 constexpr int kKZU = 8;
-__global__ void __launch_bounds__(256) k_pcg_updc(Geo G, float* __restrict__ x, const float* __restrict__ r,
-                                                  float* __restrict__ r_out, const float* __restrict__ p,
-                                                  const float* __restrict__ q, PCGState* st, double* partial,
-                                                  unsigned int* counter, int x_zero) {
+// x += alpha p (the first iteration: x = alpha p), r -= alpha q, r.r and the inner stop test
+__global__ void __launch_bounds__(256) k_pcg_updc(Geo G, float* __restrict__ x, float* __restrict__ r,
+                                                  const float* __restrict__ p, const float* __restrict__ q,
+                                                  PCGState* st, double* partial, unsigned int* counter) {
     pdl_wait();
     if (st->done) return;
     const float alpha = (float)st->alpha;
+    const bool x_zero = st->iters == 0;
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k0 = blockIdx.z * kKZU + 1;
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(256) k_pcg_updc(Geo G, float* __restrict__ x, 
             const int c = c0 + pxy * k;
             x[c] = (x_zero ? 0.f : x[c]) + alpha * p[c];
             const float rv = r[c] - alpha * q[c];
-            r_out[c] = rv;
+            r[c] = rv;
             rr += (double)rv * (double)rv;
         }
     }
@@ -733,10 +734,10 @@ void launch_mx_residual(suli_ctx* c, const double* e_in, double* e_out, bool app
 
 void launch_pcg_cond(suli_ctx* c, cudaGraphConditionalHandle h) { pdl_launch(k_pcg_cond, 1, 1, c->stream, h, c->pcg); }
 
-// The pass's first PCG update writes x = alpha p (launch_pcg_iter with x_zero), so x needs no
-// zero fill, except where the update runs inside the pre-smoothing kernel (SULI_FUSED_UPDATE=1).
+// The pass's first PCG update writes x = alpha p, so x needs no zero fill, except where the update
+// runs inside the pre-smoothing kernel (SULI_FUSED_UPDATE=1).
 static bool fused_update(const suli_ctx* c);
-void launch_pcg_init(suli_ctx* c, int maxit) {
+static void launch_pcg_init(suli_ctx* c, int maxit) {
     k_pcg_init<<<1, 1, 0, c->stream>>>(c->pcg, c->P.inner_tol, maxit);
     if (!fused_update(c)) return;
     const long long n = (long long)c->g.n;
@@ -1209,12 +1210,21 @@ void launch_vcycle(suli_ctx* c, const float* f0, bool pre_done) {
 // and q at the neighbours), so it is not the default.
 static bool fused_update(const suli_ctx* c) { return c->fuse_update && c->mg.size() > 1 && vec_level(c, c->g); }
 
-// one inner PCG iteration: p = z + beta p_old, q = A p (p.q -> alpha); x += alpha p,
-// r_new = r_old - alpha q (r.r -> stop test); z = M r_new (r.z -> beta)
-void launch_pcg_iter(suli_ctx* c, const float* p_old, float* p_new, const float* r_old, float* r_new, bool x_zero) {
+// One inner PCG iteration.  By default z = M r (r.z -> beta), p = z + beta p_old, q = A p (p.q ->
+// alpha), x += alpha p, r -= alpha q (r.r -> stop test): the test ends the iteration, so the loop
+// stops right behind it: with z formed last, after the update, every converged solve ran one more
+// V-cycle or pair of them as kernels that only read the done flag, about 34 us a solve (one
+// pressure solve of a 128^3 tank 4.30 -> 3.96 ms, a 144x80x112 step 7.14 -> 6.83).  The first iteration
+// (iters = 0) has beta = 0, any finite p_old, and writes x.  With the update fused into the pre-smoothing (r_new != r_old) the V-cycle comes last:
+// p, q, [update, z = M r_new], after a first V-cycle by the caller.
+void launch_pcg_iter(suli_ctx* c, const float* p_old, float* p_new, const float* r_old, float* r_new) {
     const Geo& G = c->g;
     MGLevel& M0 = c->mg[0];
-    const bool vec = vec_level(c, G);
+    const bool vec = vec_level(c, G), fused = fused_update(c);
+    if (!fused) {
+        ProfScope ps(c, SULI_K_MG, vcycle_kernels(c));
+        launch_vcycle(c, r_old);
+    }
     {
         ProfScope ps(c, SULI_K_CG_SPMV, 1);
         if (c->mg.size() > 1) {
@@ -1231,27 +1241,47 @@ void launch_pcg_iter(suli_ctx* c, const float* p_old, float* p_new, const float*
                        stored(M0), c->pcg, c->red_partial, c->red_counter);
         }
     }
-    if (fused_update(c)) {
+    if (fused) {
         ProfScope ps(c, SULI_K_MG, vcycle_kernels(c));
         VLAUNCH(k_mgv_preu, OpRho4, G, G, c->bc, c->pc_x, p_new, r_old, c->pc_q, r_new, from_rho4(M0), M0.y,
                 (float)c->P.mg_omega, (float)c->P.mg_omega2, c->pcg, c->red_partial, c->red_counter);
         launch_vcycle(c, r_new, true);
         return;
     }
-    {
-        ProfScope ps(c, SULI_K_CG_UPDATE, 1);
-        if (vec) {
-            pdl_launch(k_pcgv_updc, vgrid_upd(G), kB2, c->stream, G, c->pc_x, r_old, r_new, p_new, c->pc_q, c->pcg,
-                       c->red_partial, c->red_counter, x_zero ? 1 : 0);
-        } else {
-            const dim3 gu((G.nx + 31) / 32, (G.ny + 7) / 8, (G.nz + kKZU - 1) / kKZU);
-            pdl_launch(k_pcg_updc, gu, kB2, c->stream, G, c->pc_x, r_old, r_new, p_new, c->pc_q, c->pcg,
-                       c->red_partial, c->red_counter, x_zero ? 1 : 0);
-        }
+    ProfScope ps(c, SULI_K_CG_UPDATE, 1);
+    if (vec) {
+        pdl_launch(k_pcgv_updc, vgrid_upd(G), kB2, c->stream, G, c->pc_x, r_new, p_new, c->pc_q, c->pcg,
+                   c->red_partial, c->red_counter);
+    } else {
+        const dim3 gu((G.nx + 31) / 32, (G.ny + 7) / 8, (G.nz + kKZU - 1) / kKZU);
+        pdl_launch(k_pcg_updc, gu, kB2, c->stream, G, c->pc_x, r_new, p_new, c->pc_q, c->pcg, c->red_partial,
+                   c->red_counter);
     }
-    ProfScope ps(c, SULI_K_MG, vcycle_kernels(c));
-    launch_vcycle(c, r_new);
 }
+
+// the body of the inner loop: two iterations, the direction ping-ponging between two buffers (the
+// first reads pc_pb, unless fused, whose first iteration the caller launched into pc_pa)
+void launch_pcg_pair(suli_ctx* c) {
+    if (fused_update(c)) {
+        launch_pcg_iter(c, c->pc_pa, c->pc_pb, c->pc_r2, c->pc_r);
+        launch_pcg_iter(c, c->pc_pb, c->pc_pa, c->pc_r, c->pc_r2);
+    } else {
+        launch_pcg_iter(c, c->pc_pb, c->pc_pa, c->pc_r, c->pc_r);
+        launch_pcg_iter(c, c->pc_pa, c->pc_pb, c->pc_r, c->pc_r);
+    }
+}
+// what a pass launches before the loop: the inner solve's state; fused, also the first iteration
+void launch_pcg_begin(suli_ctx* c, int maxit) {
+    launch_pcg_init(c, maxit);
+    if (!fused_update(c)) return;
+    {
+        ProfScope ps(c, SULI_K_MG, vcycle_kernels(c));
+        launch_vcycle(c, c->pc_r);
+    }
+    launch_pcg_iter(c, c->mg[0].y, c->pc_pa, c->pc_r, c->pc_r2);   // p_old = z with beta = 0
+}
+// two-iteration bodies the loop ran for an inner solve of this many iterations
+int pcg_bodies(const suli_ctx* c, int iters) { return std::max(1, fused_update(c) ? iters / 2 : (iters + 1) / 2); }
 
 int pcg_iter_kernels(const suli_ctx* c) { return fused_update(c) ? 1 + vcycle_kernels(c) : 2 + vcycle_kernels(c); }
 

@@ -707,10 +707,7 @@ int ensure_pcg_loop(suli_ctx* c) {
     if (c->pcg_loop) return SULI_OK;
     if (int r = make_loop_graph(
             c, &c->pcg_loop,
-            [&] {
-                launch_pcg_iter(c, c->pc_pa, c->pc_pb, c->pc_r2, c->pc_r);
-                launch_pcg_iter(c, c->pc_pb, c->pc_pa, c->pc_r, c->pc_r2);
-            },
+            [&] { launch_pcg_pair(c); },
             [&](cudaGraphConditionalHandle h) { launch_pcg_cond(c, h); }, "inner-solve graph"))
         return r;
     c->pcg_graph_kernels = pcg_iter_kernels(c);
@@ -827,14 +824,17 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
     bool pcg_pending = false;
     auto take_inner = [&]() -> int {
         pcg_pending = false;
-        if (c->pcg_host[0].status == SULI_ERR_NAN) return fail(c, SULI_ERR_NAN, "graddin: NaN/Inf in the inner solve");
+        if (c->pcg_host[0].status == SULI_ERR_NAN) {
+            // the next solve's first iteration reads the old direction (times 0): leave it finite
+            cudaMemsetAsync(c->pc_pb, 0, c->g.n * sizeof(float), c->stream);
+            return fail(c, SULI_ERR_NAN, "graddin: NaN/Inf in the inner solve");
+        }
         if (c->pcg_host[0].status == SULI_ERR_CUDA)
             return fail(c, SULI_ERR_CUDA, "graddin: a streaming multigrid kernel's wait for its loads ran out");
         inner_total += c->pcg_host[0].iters;
         inner_capped = (c->pcg_host[0].iters >= c->inner_maxit);
         if (c->use_graphs) {   // eager launches were counted as they went
-            const long long bodies = std::max(1, (c->pcg_host[0].iters - 1 + 1) / 2);
-            c->prof.launches[SULI_K_MG] += bodies * (2LL * c->pcg_graph_kernels + 1);
+            c->prof.launches[SULI_K_MG] += pcg_bodies(c, c->pcg_host[0].iters) * (2LL * c->pcg_graph_kernels + 1);
         }
         return SULI_OK;
     };
@@ -855,19 +855,13 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
         }
         rr_prev = rr_now;
         if (outer >= c->P.refine_maxit) { status = SULI_WARN_CG_MAXIT; break; }
-        launch_pcg_init(c, c->inner_maxit);
-        {
-            ProfScope ps(c, SULI_K_MG, vcycle_kernels(c));
-            launch_vcycle(c, c->pc_r);
-        }
-        launch_pcg_iter(c, c->mg[0].y, c->pc_pa, c->pc_r, c->pc_r2, true);   // p_old = z with beta = 0, x = 0
+        launch_pcg_begin(c, c->inner_maxit);
         if (c->use_graphs) {
             ProfScope ps(c, SULI_K_MG, 0);   // kernel launches are counted below, once known
             CUDA_TRY(c, cudaGraphLaunch(c->pcg_loop, c->stream));
         } else {
             for (int pair = 0; pair < c->inner_maxit; ++pair) {
-                launch_pcg_iter(c, c->pc_pa, c->pc_pb, c->pc_r2, c->pc_r);
-                launch_pcg_iter(c, c->pc_pb, c->pc_pa, c->pc_r, c->pc_r2);
+                launch_pcg_pair(c);
                 CHECK_LAUNCH(c);
                 if (int rr = sync_read(c, c->pcg, c->pcg_host, sizeof(PCGState))) return rr;
                 if (c->pcg_host[0].done) break;

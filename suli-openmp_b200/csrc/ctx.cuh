@@ -54,6 +54,19 @@ struct PCGState {
     int maxit;
     int status;
 };
+#ifdef __CUDACC__
+// the state an inner solve starts from: r.r of its right-hand side, tolf = inner_tol^2
+__device__ __forceinline__ void pcg_start(PCGState* st, double rr0, double tolf, int maxit) {
+    st->rr0 = rr0;
+    st->tol2 = tolf * rr0;
+    st->iters = 0;
+    st->done = 0;
+    st->status = 0;
+    st->maxit = maxit;
+    st->beta = 0.;
+    st->rz = 0.;
+}
+#endif
 
 // Scales of the learned initial guess (device resident): rms of the first scaled residual,
 // mean and rms deviation of e0, the FP64 step length, the null-space coefficient of a
@@ -267,7 +280,7 @@ void launch_visco(suli_ctx* c);
 void launch_convdiff(suli_ctx* c);
 void launch_tempo(suli_ctx* c, int tt, int it);
 void launch_contorno(suli_ctx* c, int nlock);
-void launch_cg_setup(suli_ctx* c);
+void launch_cg_setup(suli_ctx* c, bool mixed = false, bool mixed_residual = false);
 void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new);
 size_t coop_ready(suli_ctx* c);
 cudaError_t launch_cg_coop(suli_ctx* c);
@@ -279,7 +292,7 @@ void launch_cg_final(suli_ctx* c, const double* e);
 // ---- mixed-precision solve (k_mixed.cu) ----
 void launch_mx_setup(suli_ctx* c);
 void launch_mx_residual(suli_ctx* c, const double* e_in, double* e_out, bool apply);
-void launch_pcg_begin(suli_ctx* c, int maxit);
+void launch_pcg_begin(suli_ctx* c);
 void launch_pcg_pair(suli_ctx* c);
 int pcg_bodies(const suli_ctx* c, int iters);
 // the loop condition of the inner-solve graph: non-zero while the inner solve is not done

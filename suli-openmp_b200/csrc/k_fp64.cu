@@ -15,6 +15,7 @@
 #include <cstring>
 #include "advect.cuh"
 #include "ctx.cuh"
+#include "face32.cuh"
 #include "obstacle.cuh"
 #include "pdl.cuh"
 #include "reduce.cuh"
@@ -1009,17 +1010,52 @@ __device__ __forceinline__ double rho_face_z(const Geo& G, const BC& bc, const d
 // sums and the scaled coefficients are the same expressions, in the same order, as forming
 // every face where it is used.
 
+// what the mixed path takes from the set-up besides the FP64 system: level 0 of its multigrid
+// (FP32 density, faces, inverse diagonal and the face constants 2 dt/dx^2, ...) and the inner
+// solve's first right-hand side
+struct MXSetup {
+    float *rho, *sx, *sy, *sz, *idg, *c2, *ru;
+    float cx2, cy2, cz2;
+    PCGState* pst;
+    double tolf;
+    int maxit;
+};
+__device__ __forceinline__ void mx_level0(const Geo& G, const BC& bc, const MXSetup& M, const double* rho, int i, int j,
+                                          int k, int c) {
+    auto fx = [&](int f) { const int fc = clampi(f, 2, G.nx); return face_rho(M.cx2, FIDX(rho, fc, j, k), FIDX(rho, fc - 1, j, k)); };
+    auto fy = [&](int f) { const int fc = clampi(f, 2, G.ny); return face_rho(M.cy2, FIDX(rho, i, fc, k), FIDX(rho, i, fc - 1, k)); };
+    auto fz = [&](int f) { const int fc = clampi(f, 2, G.nz); return face_rho(M.cz2, FIDX(rho, i, j, fc), FIDX(rho, i, j, fc - 1)); };
+    const float xl = fx(i), xh = fx(i + 1), yl = fy(j), yh = fy(j + 1), zl = fz(k), zh = fz(k + 1);
+    M.rho[c] = (float)rho[c];
+    M.sx[c] = xl; M.sy[c] = yl; M.sz[c] = zl;
+    if (i == G.nx) M.sx[c + 1] = xh;
+    if (j == G.ny) M.sy[c + G.px] = yh;
+    if (k == G.nz) M.sz[c + (int)G.pxy] = zh;
+    float d = 0.f;
+    if (i > 1 || bc.perx) d += xl;
+    if (i < G.nx || bc.perx) d += xh;
+    if (j > 1 || bc.pery) d += yl;
+    if (j < G.ny || bc.pery) d += yh;
+    if (k > 1 || bc.perz) d += zl;
+    if (k < G.nz || bc.perz) d += zh;
+    M.idg[c] = 1.f / (d > 0.f ? d : 1.f);
+    if (i == 1 && j == 1 && k == 1) { M.c2[0] = M.cx2; M.c2[1] = M.cy2; M.c2[2] = M.cz2; }
+}
+
 // minus-face conductances of every cell, the reference's c/((rho_a + rho_b)/2) with the clamped
-// end faces (:46-87): sx(i) = face between i-1 and i (at i = 1 the face of i = 2)
+// end faces (:46-87): sx(i) = face between i-1 and i (at i = 1 the face of i = 2); MX: also the
+// multigrid's level 0, from the same density loads
+template <bool MX>
 __global__ void __launch_bounds__(256) k_cg_faces(Geo G, BC bc, CGConst K, const double* __restrict__ rho, double* sx,
-                                                  double* sy, double* sz) {
+                                                  double* sy, double* sz, MXSetup M) {
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k;
     if (i > G.nx || j > G.ny || k > G.nz) return;
-    const long long c = G.idx(i, j, k);
+    const int c = G.idx32(i, j, k);
     sx[c] = K.cx / rho_face_x(G, bc, rho, i, j, k);
     sy[c] = K.cy / rho_face_y(G, bc, rho, i, j, k);
     sz[c] = K.cz / rho_face_z(G, bc, rho, i, j, k);
+    if (MX) mx_level0(G, bc, M, rho, i, j, k, c);
 }
 
 // the plus face of a cell: the next cell's minus face, or at the last cell the same clamped face
@@ -1035,7 +1071,8 @@ __device__ __forceinline__ PlusFaces plus_faces(const Geo& G, const BC& bc, int 
                      (k < G.nz) ? sz[c + G.pxy] : sz[c - (wz ? (long long)(G.nz - 1) * G.pxy : 0)]};
 }
 
-// diagonal d, scaled unknown e = prd1*sqrt(d), scaled right-hand side b = q/sqrt(d) (:46-87, :118-124)
+// diagonal d (kept only for a recorded solve), scaled unknown e = prd1*sqrt(d), scaled right-hand
+// side b = q/sqrt(d) (:46-87, :118-124)
 __global__ void __launch_bounds__(256) k_cg_diag(Geo G, BC bc, CGConst K, const double* __restrict__ sx,
                                                  const double* __restrict__ sy, const double* __restrict__ sz,
                                                  const double* __restrict__ u, const double* __restrict__ v,
@@ -1051,7 +1088,7 @@ __global__ void __launch_bounds__(256) k_cg_diag(Geo G, BC bc, CGConst K, const 
                      (FIDX(w, i, j, k) - FIDX(w, i, j, k + 1)) * K.rdz;
     const double sd = sqrt(dv);
     const double isd = 1.0 / sd;
-    d[c] = dv;
+    if (d) d[c] = dv;
     e[c] = prd1[c] * sd;
     b[c] = q * isd;
     sdo[c] = sd;
@@ -1059,25 +1096,31 @@ __global__ void __launch_bounds__(256) k_cg_diag(Geo G, BC bc, CGConst K, const 
 }
 
 // scaled face coefficients s/sqrt(d_c d_nb) = s * (1/sqrt(d_c)) * (1/sqrt(d_nb)) and the first
-// residual (:126-151); reduction of r.r and b.b
+// residual (:126-151); reduction of r.r and b.b.  Plain: the reference's residual, whose
+// neighbours outside the box are prd1's ghosts.  MX: the refinement's residual (k_mx_outer: ghosts
+// map to cells), rounded to FP32 as the inner solve's right-hand side r_u = sqrt(d) r~, with
+// its sums; the refinement's own first pass over the coefficients is saved (set-up and refinement
+// of a 256x128x128 step 1.86 -> 1.59 ms).  Forming the faces from the density here and in
+// k_cg_diag instead of reading them back was no faster: five more FP64 divisions a cell.
 constexpr int kCoefZ = 4;
+template <bool MX>
 __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, const double* __restrict__ sx,
                                                     const double* __restrict__ sy, const double* __restrict__ sz,
                                                     const double* __restrict__ sd, const double* __restrict__ isd,
                                                     const double* __restrict__ e, const double* __restrict__ b,
                                                     const double* __restrict__ prd1, double* ax, double* ay,
                                                     double* az, double* r, CGState* st, double* partial,
-                                                    unsigned int* counter) {
+                                                    unsigned int* counter, MXSetup M) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
-    double rr = 0.0, bbv = 0.0;
+    double rr = 0.0, bbv = 0.0, ru2 = 0.0, um = 0.0;
     // a thread owns kCoefZ cells of a column: 4x fewer blocks than one cell a thread, whose
     // partials the grid reduction (one counter) would otherwise take in turn
 #pragma unroll
     for (int m = 0; m < kCoefZ; ++m) {
     const int k = blockIdx.z * kCoefZ + 1 + m;
     if (i <= nx && j <= ny && k <= nz) {
-        const int c = (int)G.idx(i, j, k);
+        const int c = G.idx32(i, j, k);
         const int px = G.px, pxy = (int)G.pxy;
         const Nb o = neighbours(G, bc, i, j, k);   // ghost-mapped neighbours (periodic wrap / Neumann self)
         const double ic = isd[c];
@@ -1093,19 +1136,38 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
         if (i == nx) ax[c + 1] = app;
         if (j == ny) ay[c + px] = bpp;
         if (k == nz) az[c + pxy] = cpp;
-        // e at a neighbour: interior value, or the halo value prd1(ghost)*sqrt(d(mapped ghost))
-        auto ee = [&](bool ghost, int cg, int off) { return ghost ? prd1[cg] * sd[c + off] : e[c + off]; };
+        // e at a neighbour: interior value, or the halo value prd1(ghost)*sqrt(d(mapped ghost)).
+        // MX maps ghosts to cells, but a ghost that is not finite still fails the solve.
+        auto ee = [&](bool ghost, int cg, int off) {
+            if (MX && ghost) rr += 0.0 * prd1[cg];
+            return (!MX && ghost) ? prd1[cg] * sd[c + off] : e[c + off];
+        };
         const double bv = b[c];
         const double rv = e[c] - app * ee(i == nx, c + 1, o.xp) - anp * ee(i == 1, c - 1, o.xm) -
                           bpp * ee(j == ny, c + px, o.yp) - bnp * ee(j == 1, c - px, o.ym) -
                           cpp * ee(k == nz, c + pxy, o.zp) - cnp * ee(k == 1, c - pxy, o.zm) - bv;
-        r[c] = rv;
         rr += rv * rv;
         bbv += bv * bv;
+        if (MX) {
+            const double uv = sd[c] * rv;
+            M.ru[c] = (float)uv;
+            ru2 += uv * uv;
+            um = fmax(um, fabs(uv));
+        } else {
+            r[c] = rv;
+        }
     }
     }
-    double trr, tbb;
-    if (reduce2_last(rr, bbv, partial, counter, trr, tbb) && flat_tid() == 0) {
+    double trr, tbb, tru2 = 0.0, tum = 0.0;
+    bool last;
+    if (MX) {
+        double s[3] = {rr, bbv, ru2}, t[3];
+        last = reduce_sums_max_last<3>(s, um, partial, counter, t, tum);
+        trr = t[0]; tbb = t[1]; tru2 = t[2];
+    } else {
+        last = reduce2_last(rr, bbv, partial, counter, trr, tbb);
+    }
+    if (last && flat_tid() == 0) {
         st->rr = trr;
         st->rr_start = trr;
         st->bb = tbb;
@@ -1116,10 +1178,12 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
         st->mode = K.mode;
         st->status = 0;
         st->div_tol = K.div_tol;
-        st->rmax = 0.;
-        const bool go = (fabs(trr) > st->thr) && (K.maxit > 0);
+        st->rmax = tum;
+        const bool go = MX ? (trr > st->thr || (K.div_tol > 0. && !(tum <= K.div_tol)))
+                           : (fabs(trr) > st->thr) && (K.maxit > 0);
         st->done = go ? 0 : 1;
         if (!isfinite(trr)) { st->status = SULI_ERR_NAN; st->done = 1; }
+        if (MX) pcg_start(M.pst, tru2, M.tolf, M.maxit);
     }
 }
 
@@ -1631,18 +1695,29 @@ static CGConst cg_const(const suli_ctx* c) {
     K.maxit = c->P.cg_maxit;
     return K;
 }
-void launch_cg_setup(suli_ctx* c) {
+// mixed: also level 0 of the multigrid; mixed_residual: the refinement's first residual in place of
+// the plain path's
+void launch_cg_setup(suli_ctx* c, bool mixed, bool mixed_residual) {
     const Geo& G = c->g;
     const CGConst K = cg_const(c);
     ProfScope ps(c, SULI_K_CG_SETUP, 3);
+    MXSetup M = {};
+    if (mixed) {
+        const MGLevel& L = c->mg[0];
+        M = MXSetup{L.rho, L.sx, L.sy, L.sz, L.idg, L.c2, c->pc_r, (float)(2. * c->dt / (c->P.dx * c->P.dx)),
+                    (float)(2. * c->dt / (c->P.dy * c->P.dy)), (float)(2. * c->dt / (c->P.dz * c->P.dz)), c->pcg, c->P.inner_tol * c->P.inner_tol, c->inner_maxit};
+    }
     // face scratch: the CG direction and product vectors, written again before the iterations read them
     double *sx = c->cg_pa, *sy = c->cg_pb, *sz = c->cg_q;
-    k_cg_faces<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->bc, K, c->f[SULI_F_RHO], sx, sy, sz);
+    const auto faces = mixed ? k_cg_faces<true> : k_cg_faces<false>;
+    faces<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->bc, K, c->f[SULI_F_RHO], sx, sy, sz, M);
     k_cg_diag<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->bc, K, sx, sy, sz, c->f[SULI_F_U], c->f[SULI_F_V], c->f[SULI_F_W],
-                                                      c->f[SULI_F_PRD1], c->cg_d, c->cg_e, c->cg_b, c->cg_sd, c->cg_isd);
-    k_cg_coef<<<grid3(G.nx, G.ny, (G.nz + kCoefZ - 1) / kCoefZ, kBlk), kBlk, 0, c->stream>>>(G, c->bc, K, sx, sy, sz, c->cg_sd, c->cg_isd, c->cg_e, c->cg_b,
-                                                      c->f[SULI_F_PRD1], c->cg_ax, c->cg_ay, c->cg_az, c->cg_r, c->cg,
-                                                      c->red_partial, c->red_counter);
+                                                      c->f[SULI_F_PRD1], c->rec_in ? c->cg_d : nullptr, c->cg_e, c->cg_b,
+                                                      c->cg_sd, c->cg_isd);
+    const auto coef = mixed_residual ? k_cg_coef<true> : k_cg_coef<false>;
+    coef<<<grid3(G.nx, G.ny, (G.nz + kCoefZ - 1) / kCoefZ, kBlk), kBlk, 0, c->stream>>>(
+        G, c->bc, K, sx, sy, sz, c->cg_sd, c->cg_isd, c->cg_e, c->cg_b, c->f[SULI_F_PRD1], c->cg_ax, c->cg_ay, c->cg_az,
+        c->cg_r, c->cg, c->red_partial, c->red_counter, M);
 }
 void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
     const Geo& G = c->g;

@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <cstring>
 #include "ctx.cuh"
+#include "face32.cuh"
 #include "pdl.cuh"
 #include "reduce.cuh"
 
@@ -85,17 +86,6 @@ struct OpStored {
     __device__ __forceinline__ float inv_diag(int c) const { return idg[c]; }
 };
 
-// c2/(rho_a + rho_b) with the hardware reciprocal (2 ulp): the preconditioner's operator only
-// has to be the same everywhere it is formed, and this is the one formula used for it.  The .ftz
-// form, the same value for normal numbers: __fdividef also rescales subnormal divisors, several
-// instructions for each of the 17 faces a quad forms, and the level-0 kernels are half bound by
-// instruction issue (inner solves of a 256x128x128 step 8.62 -> 8.38 ms).
-__device__ __forceinline__ float face_div(float c2, float rsum) {
-    float q;
-    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(c2), "f"(rsum));
-    return q;
-}
-
 // faces from the FP32 density (level 0); c2[0..2] = 2 dt/dx^2, 2 dt/dy^2, 2 dt/dz^2 in device
 // memory (dt changes per RK stage while the captured graphs stay the same)
 struct OpRho {
@@ -132,41 +122,9 @@ struct OpRho {
     __device__ __forceinline__ float inv_diag(int c) const { return idg[c]; }
 };
 
-// face conductance of the level-0 operator between two cells (FP32, the formula OpRho uses)
-__device__ __forceinline__ float face_rho(float c2, double ra, double rb) {
-    return face_div(c2, (float)ra + (float)rb);
-}
-
 // ------------------------------------------------------------------------------------
-// set-up: FP32 density, the fine faces (for the coarsening) and the inverse diagonal
+// set-up of the coarse levels (level 0's faces come with the FP64 system, k_fp64.cu)
 // ------------------------------------------------------------------------------------
-__global__ void k_mx_faces0(Geo G, BC bc, const double* __restrict__ rho, float cx2, float cy2, float cz2,
-                            float* rho32, float* sx, float* sy, float* sz, float* idg, float* c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z + 1;
-    if (i == 1 && j == 1 && k == 1) { c2[0] = cx2; c2[1] = cy2; c2[2] = cz2; }
-    if (i > G.nx || j > G.ny || k > G.nz) return;
-    auto fx = [&](int f) { const int fc = clampi_m(f, 2, G.nx); return face_rho(cx2, FI(rho, fc, j, k), FI(rho, fc - 1, j, k)); };
-    auto fy = [&](int f) { const int fc = clampi_m(f, 2, G.ny); return face_rho(cy2, FI(rho, i, fc, k), FI(rho, i, fc - 1, k)); };
-    auto fz = [&](int f) { const int fc = clampi_m(f, 2, G.nz); return face_rho(cz2, FI(rho, i, j, fc), FI(rho, i, j, fc - 1)); };
-    const float xl = fx(i), xh = fx(i + 1), yl = fy(j), yh = fy(j + 1), zl = fz(k), zh = fz(k + 1);
-    const long long c = G.idx(i, j, k);
-    rho32[c] = (float)rho[c];
-    sx[c] = xl; sy[c] = yl; sz[c] = zl;
-    if (i == G.nx) FI(sx, i + 1, j, k) = xh;
-    if (j == G.ny) FI(sy, i, j + 1, k) = yh;
-    if (k == G.nz) FI(sz, i, j, k + 1) = zh;
-    float d = 0.f;
-    if (i > 1 || bc.perx) d += xl;
-    if (i < G.nx || bc.perx) d += xh;
-    if (j > 1 || bc.pery) d += yl;
-    if (j < G.ny || bc.pery) d += yh;
-    if (k > 1 || bc.perz) d += zl;
-    if (k < G.nz || bc.perz) d += zh;
-    idg[c] = 1.f / (d > 0.f ? d : 1.f);
-}
-
 // Galerkin coarse faces: (sum of the 4 fine faces covering a coarse face) / 8
 __global__ void k_mg_coarsen(Geo Gf, Geo Gc, BC bc, const float* __restrict__ fx, const float* __restrict__ fy,
                              const float* __restrict__ fz, float* cxs, float* cys, float* czs, float* idg) {
@@ -555,9 +513,10 @@ __global__ void __launch_bounds__(256) k_pcg_updc(Geo G, float* __restrict__ x, 
 // ------------------------------------------------------------------------------------
 // Block partials of the refinement residual: r~.r~, r_u.r_u and max |r_u| (r_u = sqrt(d) r~ is the
 // divergence the projection would leave).  The last block sets the stopping test: r~.r~ within
-// the threshold and, with div_tol > 0, max |r_u| within div_tol.
+// the threshold and, with div_tol > 0, max |r_u| within div_tol; and the next inner solve's state.
 __device__ __forceinline__ void mx_outer_finish(double rr, double ru2, double um, int apply, CGState* cg,
-                                                PCGState* pst, double* partial, unsigned int* counter) {
+                                                PCGState* pst, double tolf, int maxit, double* partial,
+                                                unsigned int* counter) {
     if (isnan(um)) um = INFINITY;
     double t1, t2, tm;
     if (reduce3_last(rr, ru2, um, partial, counter, t1, t2, tm) && flat_tid() == 0) {
@@ -567,7 +526,7 @@ __device__ __forceinline__ void mx_outer_finish(double rr, double ru2, double um
         const bool div_ok = !(cg->div_tol > 0.) || tm <= cg->div_tol;
         cg->done = (t1 > cg->thr || !div_ok) ? 0 : 1;
         if (!isfinite(t1)) { cg->status = SULI_ERR_NAN; cg->done = 1; }
-        pst->rr0 = t2;
+        pcg_start(pst, t2, tolf, maxit);
     }
 }
 
@@ -576,8 +535,8 @@ __global__ void __launch_bounds__(256) k_mx_outer(Geo G, BC bc, const double* __
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
                                                   const double* __restrict__ az, const double* __restrict__ b,
                                                   double* __restrict__ e_out, float* __restrict__ ru, int apply,
-                                                  CGState* cg, PCGState* pst, double* partial, unsigned int* counter,
-                                                  double* __restrict__ r_out) {
+                                                  CGState* cg, PCGState* pst, double tolf, int maxit, double* partial,
+                                                  unsigned int* counter, double* __restrict__ r_out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z + 1;
@@ -597,23 +556,23 @@ __global__ void __launch_bounds__(256) k_mx_outer(Geo G, BC bc, const double* __
         ru2 = u * u;
         um = fabs(u);
     }
-    mx_outer_finish(rr, ru2, um, apply, cg, pst, partial, counter);
+    mx_outer_finish(rr, ru2, um, apply, cg, pst, tolf, maxit, partial, counter);
 }
 
 // k_mx_outer with two x cells a thread (16-byte row loads; needs nx even) and kOuterZ planes of
 // their column (loads from clamped planes, so that the planes' loads are issued together; stores
 // and sums only inside the grid): per cell the same expressions, only the two reductions group
-// their terms differently.  A quarter of the blocks of one plane a thread; measured at
-// 256x128x128 one, two (at 64 registers) and four planes a thread run alike (latency-bound, about
-// 80 us a launch).
+// their terms differently.  A quarter of the blocks of one plane a thread.  Latency-bound: at
+// 256x128x128 12 launches take 0.99 ms at four blocks an SM (64 registers), 1.07 at three; 1.09
+// with two planes a thread, 1.21 with eight.
 constexpr int kOuterZ = 4;
-__global__ void __launch_bounds__(256) k_mx_outer2(Geo G, BC bc, const double* __restrict__ e_in,
+__global__ void __launch_bounds__(256, 4) k_mx_outer2(Geo G, BC bc, const double* __restrict__ e_in,
                                                    const float* __restrict__ dp, const double* __restrict__ sd,
                                                    const double* __restrict__ ax, const double* __restrict__ ay,
                                                    const double* __restrict__ az, const double* __restrict__ b,
                                                    double* __restrict__ e_out, float* __restrict__ ru, int apply,
-                                                   CGState* cg, PCGState* pst, double* partial, unsigned int* counter,
-                                                   double* __restrict__ r_out) {
+                                                   CGState* cg, PCGState* pst, double tolf, int maxit, double* partial,
+                                                   unsigned int* counter, double* __restrict__ r_out) {
     const int i0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k0 = blockIdx.z * kOuterZ + 1;
@@ -666,17 +625,7 @@ __global__ void __launch_bounds__(256) k_mx_outer2(Geo G, BC bc, const double* _
             }
         }
     }
-    mx_outer_finish(rr, ru2, um, apply, cg, pst, partial, counter);
-}
-
-__global__ void k_pcg_init(PCGState* st, double inner_tol, int maxit) {
-    st->tol2 = inner_tol * inner_tol * st->rr0;
-    st->iters = 0;
-    st->done = 0;
-    st->status = 0;
-    st->maxit = maxit;
-    st->beta = 0.;
-    st->rz = 0.;
+    mx_outer_finish(rr, ru2, um, apply, cg, pst, tolf, maxit, partial, counter);
 }
 
 __global__ void k_pcg_cond(cudaGraphConditionalHandle h, const PCGState* st) {
@@ -707,12 +656,7 @@ static inline OpStored stored(const MGLevel& L) { return OpStored{L.sx, L.sy, L.
 static inline OpRho from_rho(const MGLevel& L) { return OpRho{L.rho, L.idg, L.c2}; }
 
 void launch_mx_setup(suli_ctx* c) {
-    ProfScope ps(c, SULI_K_CG_SETUP, (int)c->mg.size());
-    MGLevel& L0 = c->mg[0];
-    const float cx2 = (float)(2. * c->dt / (c->P.dx * c->P.dx)), cy2 = (float)(2. * c->dt / (c->P.dy * c->P.dy)),
-                cz2 = (float)(2. * c->dt / (c->P.dz * c->P.dz));
-    k_mx_faces0<<<cells3(L0.g), kB2, 0, c->stream>>>(L0.g, c->bc, c->f[SULI_F_RHO], cx2, cy2, cz2, L0.rho, L0.sx,
-                                                     L0.sy, L0.sz, L0.idg, L0.c2);
+    ProfScope ps(c, SULI_K_CG_SETUP, (int)c->mg.size() - 1);
     for (size_t l = 1; l < c->mg.size(); ++l) {
         MGLevel& F = c->mg[l - 1];
         MGLevel& C = c->mg[l];
@@ -725,31 +669,22 @@ void launch_mx_setup(suli_ctx* c) {
 // is kept as well, in cg_r, for the network's features and step length.
 void launch_mx_residual(suli_ctx* c, const double* e_in, double* e_out, bool apply) {
     double* r_out = (c->nn && c->nn_mode == 2 && !c->rec_in) ? c->cg_r : nullptr;
+    const double tolf = c->P.inner_tol * c->P.inner_tol;
     ProfScope ps(c, SULI_K_REFINE, 1);
     const Geo& G = c->g;
     if (G.nx % 2 == 0) {
         const dim3 g2((G.nx / 2 + 31) / 32, (G.ny + 7) / 8, (G.nz + kOuterZ - 1) / kOuterZ);
         k_mx_outer2<<<g2, kB2, 0, c->stream>>>(G, c->bc, e_in, c->pc_x, c->cg_sd, c->cg_ax, c->cg_ay, c->cg_az,
-                                               c->cg_b, e_out, c->pc_r, apply ? 1 : 0, c->cg, c->pcg,
+                                               c->cg_b, e_out, c->pc_r, apply ? 1 : 0, c->cg, c->pcg, tolf, c->inner_maxit,
                                                c->red_partial, c->red_counter, r_out);
     } else {
         k_mx_outer<<<cells3(G), kB2, 0, c->stream>>>(G, c->bc, e_in, c->pc_x, c->cg_sd, c->cg_ax, c->cg_ay, c->cg_az,
-                                                     c->cg_b, e_out, c->pc_r, apply ? 1 : 0, c->cg, c->pcg,
+                                                     c->cg_b, e_out, c->pc_r, apply ? 1 : 0, c->cg, c->pcg, tolf, c->inner_maxit,
                                                      c->red_partial, c->red_counter, r_out);
     }
 }
 
 void launch_pcg_cond(suli_ctx* c, cudaGraphConditionalHandle h) { pdl_launch(k_pcg_cond, 1, 1, c->stream, h, c->pcg); }
-
-// The pass's first PCG update writes x = alpha p, so x needs no zero fill, except where the update
-// runs inside the pre-smoothing kernel (SULI_FUSED_UPDATE=1).
-static bool fused_update(const suli_ctx* c);
-static void launch_pcg_init(suli_ctx* c, int maxit) {
-    k_pcg_init<<<1, 1, 0, c->stream>>>(c->pcg, c->P.inner_tol, maxit);
-    if (!fused_update(c)) return;
-    const long long n = (long long)c->g.n;
-    k_zero_f<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->pc_x, n);
-}
 
 static inline OpRho4 from_rho4(const MGLevel& L) { return OpRho4{L.rho, L.idg, L.c2}; }
 // launch a column kernel of the vectorised family with the context's column depth (2 or 4)
@@ -1277,10 +1212,11 @@ void launch_pcg_pair(suli_ctx* c) {
         launch_pcg_iter(c, c->pc_pa, c->pc_pb, c->pc_r, c->pc_r);
     }
 }
-// what a pass launches before the loop: the inner solve's state; fused, also the first iteration
-void launch_pcg_begin(suli_ctx* c, int maxit) {
-    launch_pcg_init(c, maxit);
+// what a pass launches before the loop: nothing, or fused, the first iteration
+void launch_pcg_begin(suli_ctx* c) {
     if (!fused_update(c)) return;
+    const long long n = (long long)c->g.n;
+    k_zero_f<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->pc_x, n);   // its update adds to x
     {
         ProfScope ps(c, SULI_K_MG, vcycle_kernels(c));
         launch_vcycle(c, c->pc_r);

@@ -98,22 +98,24 @@ static __device__ bool reduce2_last(double a, double b, double* partial, unsigne
     return true;
 }
 
-// Three block partials per block: a and b summed, m maxed; the last block to arrive folds all
+// NS + 1 block partials per block: a[] summed, m maxed; the last block to arrive folds all
 // partials in block order and returns true (totals valid in thread 0 of that block).
-static __device__ bool reduce3_last(double a, double b, double m, double* partial, unsigned int* counter, double& ta,
-                                    double& tb, double& tm) {
+template <int NS>
+static __device__ bool reduce_sums_max_last(double (&a)[NS], double m, double* partial, unsigned int* counter,
+                                            double (&ta)[NS], double& tm) {
     __shared__ bool last;
+    constexpr int W = NS + 1;
     const int tid = flat_tid();
     const int nt = blockDim.x * blockDim.y * blockDim.z;
     const int bid = flat_bid();
     const int nb = gridDim.x * gridDim.y * gridDim.z;
-    a = block_sum(a);
-    b = block_sum(b);
+#pragma unroll
+    for (int n = 0; n < NS; ++n) a[n] = block_sum(a[n]);
     m = block_max(m);
     if (tid == 0) {
-        partial[3 * bid] = a;
-        partial[3 * bid + 1] = b;
-        partial[3 * bid + 2] = m;
+#pragma unroll
+        for (int n = 0; n < NS; ++n) partial[W * bid + n] = a[n];
+        partial[W * bid + NS] = m;
         __threadfence();
         const unsigned int t = atomicAdd(counter, 1u);
         last = (t == (unsigned int)(nb - 1));
@@ -121,30 +123,43 @@ static __device__ bool reduce3_last(double a, double b, double m, double* partia
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    // partials tid, tid + nt, ... in that order, eight triples loaded ahead of the folds
+    // partials tid, tid + nt, ... in that order, eight blocks' loads ahead of the folds
     constexpr int U = 8;
-    double sa = 0.0, sb = 0.0, sm = 0.0;
+    double sa[NS] = {}, sm = 0.0;
     for (int q0 = tid; q0 < nb; q0 += U * nt) {
-        double pa[U], pb[U], pm[U];
+        double pa[U][NS], pm[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int q = q0 + u * nt;
-            pa[u] = (q < nb) ? __ldcg(&partial[3 * q]) : 0.0;
-            pb[u] = (q < nb) ? __ldcg(&partial[3 * q + 1]) : 0.0;
-            pm[u] = (q < nb) ? __ldcg(&partial[3 * q + 2]) : 0.0;
+#pragma unroll
+            for (int n = 0; n < NS; ++n) pa[u][n] = (q < nb) ? __ldcg(&partial[W * q + n]) : 0.0;
+            pm[u] = (q < nb) ? __ldcg(&partial[W * q + NS]) : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (q0 + u * nt >= nb) break;
-            sa += pa[u];
-            sb += pb[u];
+#pragma unroll
+            for (int n = 0; n < NS; ++n) sa[n] += pa[u][n];
             sm = fmax(sm, pm[u]);
         }
     }
-    sa = block_sum(sa);
-    sb = block_sum(sb);
+#pragma unroll
+    for (int n = 0; n < NS; ++n) sa[n] = block_sum(sa[n]);
     sm = block_max(sm);
-    if (tid == 0) { ta = sa; tb = sb; tm = sm; *counter = 0u; }
+    if (tid == 0) {
+#pragma unroll
+        for (int n = 0; n < NS; ++n) ta[n] = sa[n];
+        tm = sm;
+        *counter = 0u;
+    }
+    return true;
+}
+static __device__ bool reduce3_last(double a, double b, double m, double* partial, unsigned int* counter, double& ta,
+                                    double& tb, double& tm) {
+    double s[2] = {a, b}, t[2];
+    if (!reduce_sums_max_last<2>(s, m, partial, counter, t, tm)) return false;
+    ta = t[0];
+    tb = t[1];
     return true;
 }
 

@@ -250,7 +250,7 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
         if ((e = cudaMemsetAsync(c->f[f], 0, n * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
     }
     const long long nb = (long long)((p->nx + 1 + 31) / 32) * ((p->ny + 1 + 7) / 8) * (p->nz + 1) + 64;
-    if ((e = cudaMalloc(&c->red_partial, (size_t)nb * 3 * sizeof(double))) != cudaSuccess) return bail(e, "partial");
+    if ((e = cudaMalloc(&c->red_partial, (size_t)nb * 4 * sizeof(double))) != cudaSuccess) return bail(e, "partial");
     if ((e = cudaMalloc(&c->red_counter, 64 * sizeof(unsigned int))) != cudaSuccess) return bail(e, "counter");
     if ((e = cudaMemsetAsync(c->red_counter, 0, 64 * sizeof(unsigned int), c->stream)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMalloc(&c->red_out, 16 * sizeof(double))) != cudaSuccess) return bail(e, "red_out");
@@ -806,13 +806,18 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
 
 int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
     if (int rg = ensure_pcg_loop(c)) return rg;
-    launch_cg_setup(c);   // FP64 diagonal, coefficients, b~, first residual and threshold
-    launch_mx_setup(c);   // FP32 faces of every multigrid level
+    // FP64 diagonal, coefficients, b~, threshold and, where no learned guess or recording comes
+    // between (they read the plain residual), the first refinement residual; level 0's FP32 faces
+    const bool plain_first = c->rec_in || (c->nn && c->nn_mode >= 1);
+    launch_cg_setup(c, true, !plain_first);
+    launch_mx_setup(c);   // FP32 faces of the coarser multigrid levels
     nn_begin(c);
     double* ecur = c->cg_e;
     double* enext = c->cg_e2;
-    launch_mx_residual(c, ecur, enext, false);
-    std::swap(ecur, enext);
+    if (plain_first) {
+        launch_mx_residual(c, ecur, enext, false);
+        std::swap(ecur, enext);
+    }
     CHECK_LAUNCH(c);
     long long inner_total = 0;
     int outer = 0, status = SULI_OK;
@@ -855,7 +860,7 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
         }
         rr_prev = rr_now;
         if (outer >= c->P.refine_maxit) { status = SULI_WARN_CG_MAXIT; break; }
-        launch_pcg_begin(c, c->inner_maxit);
+        launch_pcg_begin(c);
         if (c->use_graphs) {
             ProfScope ps(c, SULI_K_MG, 0);   // kernel launches are counted below, once known
             CUDA_TRY(c, cudaGraphLaunch(c->pcg_loop, c->stream));

@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(256) k_lsprops(Geo G, LsConst L, const double*
                                                  double* hs, double* hsx, double* hsy, double* hsz, double* rho,
                                                  double* ls_nu, int do_mod, int do_hs, int do_vol,
                                                  double* partial, unsigned int* counter, double* out) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const bool in = (t.i <= G.nx && t.j <= G.ny && t.k <= G.nz);
     double vol = 0.0;
@@ -158,6 +159,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_curv(Geo G, LsConst L, const double* __restrict__ nx_,
                                               const double* __restrict__ ny_, const double* __restrict__ nz_,
                                               double* ddx, double* ddy, double* ddz, double* kurv) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     R P[7], dp, dn;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(256) k_ls_advect(Geo G, LsConst L, const doubl
                                                    const double* phi0, double* out,
                                                    const double* __restrict__ u, const double* __restrict__ v,
                                                    const double* __restrict__ w, double a, double b, double gd) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const int i = t.i, j = t.j, k = t.k;
@@ -218,6 +221,7 @@ __device__ __forceinline__ R reinit_mod(R l, const Weno3<R>& W) {
 template <typename R>
 __global__ void __launch_bounds__(256) k_reinit_funcs(Geo G, LsConst L, const double* __restrict__ ls,
                                                       double* funcs) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const Weno3<R> W = der_weno_at<R>(G, ls, t.i, t.j, t.k, L.ihx, L.ihy, L.ihz, L.rcp<R>(0), L.rcp<R>(1), L.rcp<R>(2));
@@ -233,6 +237,7 @@ __global__ void __launch_bounds__(256) k_reinit_stage(Geo G, LsConst L, const do
                                                       const double* phi0, double* out,
                                                       const double* __restrict__ funcs, double a, double b,
                                                       double gd) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const Weno3<R> W = der_weno_at<R>(G, cur, t.i, t.j, t.k, L.ihx, L.ihy, L.ihz, L.rcp<R>(0), L.rcp<R>(1), L.rcp<R>(2));
@@ -248,6 +253,7 @@ __global__ void __launch_bounds__(256) k_reinit_stage(Geo G, LsConst L, const do
 __global__ void __launch_bounds__(256) k_reinit_err(Geo G, const double* __restrict__ after,
                                                     const double* __restrict__ before, double band,
                                                     double* partial, unsigned int* counter, double* out) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     double s = 0.0, n = 0.0;
     if (t.i <= G.nx && t.j <= G.ny && t.k <= G.nz) {
@@ -261,6 +267,7 @@ __global__ void __launch_bounds__(256) k_reinit_err(Geo G, const double* __restr
 
 // ls = ls + ls_m over the cells (14_level_set.f90:196-202)
 __global__ void k_ls_shift(Geo G, double* ls, double shift) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const long long c = G.idx(t.i, t.j, t.k);
@@ -269,6 +276,7 @@ __global__ void k_ls_shift(Geo G, double* ls, double shift) {
 
 // volume correction step (14_level_set.f90:259-265)
 __global__ void k_volfix(Geo G, double* ls, const double* __restrict__ mod_ls, double dt1fac, double vol_ini) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const long long c = G.idx(t.i, t.j, t.k);
@@ -289,6 +297,7 @@ template <typename R, int KZ>
 __global__ void __launch_bounds__(256) k_nut(Geo G, ViscConst V, const double* __restrict__ u,
                                              const double* __restrict__ v, const double* __restrict__ w,
                                              const double* __restrict__ rho, double* __restrict__ nut) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k0 = blockIdx.z * KZ + 1;
     if (i > G.nx || j > G.ny || k0 > G.nz) return;
@@ -324,6 +333,7 @@ __global__ void __launch_bounds__(256) k_nut(Geo G, ViscConst V, const double* _
 __global__ void __launch_bounds__(256) k_facenu(Geo G, int m_turb, const double* __restrict__ ls_nu,
                                                 const double* __restrict__ nut, double* xnut, double* ynut,
                                                 double* znut) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k, nx = G.nx, ny = G.ny, nz = G.nz;
     if (i > nx + 1 || j > ny + 1 || k > nz + 1) return;
@@ -362,6 +372,7 @@ __global__ void __launch_bounds__(256) k_facenu_dir(Geo G, ViscDirConst V, const
                                                     const double* __restrict__ v, const double* __restrict__ w,
                                                     const double* __restrict__ ls_nu, double* xnut, double* ynut,
                                                     double* znut) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k, nx = G.nx, ny = G.ny, nz = G.nz;
     if (i > nx + 1 || j > ny + 1 || k > nz + 1) return;
@@ -414,10 +425,21 @@ struct CDConst {
     int cap_z2, cap_y2, cap_yn;              // planes where ub/vb/wb are captured (3_contorno.f90:247-264)
     int obst;                                // obstacles: captured above each column, friction read everywhere
 };
+// dst = src at face (i, j, k) of 1..n+1, the thread of the first face of an axis also at index 0 of
+// that axis: the halo box 0..n+1 copied by a kernel over the faces
+__device__ __forceinline__ void copy_box(const Geo& G, const double* __restrict__ src, double* __restrict__ dst, int i,
+                                         int j, int k) {
+    for (int kk = (k == 1) ? 0 : k; kk <= k; ++kk)
+        for (int jj = (j == 1) ? 0 : j; jj <= j; ++jj)
+            for (int ii = (i == 1) ? 0 : i; ii <= i; ++ii) FIDX(dst, ii, jj, kk) = FIDX(src, ii, jj, kk);
+}
+
 struct CDFields {
     const double *u, *v, *w, *rho, *hsx, *hsy, *hsz, *kurv, *nut, *xnut, *ynut, *znut, *ub, *vb, *wb;
     const double *tfu, *tfv, *tfw;
     double *Fu, *Fv, *Fw;
+    const double* prd1;   // copied to prd0
+    double* prd0;
 };
 
 // the reference subtracts (gz/C^2)|ub| u at every face (6_convdiff.f90:156,168,183); ub is zero
@@ -462,9 +484,11 @@ __device__ __forceinline__ R classico_hi(const double* __restrict__ a, int c, co
 // DER: classico's scheme (adv_type = 1); ADV: 2 rotacional, 3 antissim (advect.cuh; der = 1)
 template <typename R, int DER, int ADV>
 __global__ void __launch_bounds__(256) k_convdiff(Geo G, CDConst C, CDFields F) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k, nx = G.nx, ny = G.ny, nz = G.nz;
     if (i > nx + 1 || j > ny + 1 || k > nz + 1) return;
+    copy_box(G, F.prd1, F.prd0, i, j, k);
     const R idx = R(C.idx), idy = R(C.idy), idz = R(C.idz);   // 1/dx, 1/dy, 1/dz
     // every load is the face's own index plus a constant offset (32-bit): a field value at
     // (i + di, j + dj, k + dk), read in the compute type R
@@ -627,6 +651,7 @@ struct TempoArgs {
     double dt;
 };
 __global__ void __launch_bounds__(256) k_tempo(Geo G, TempoArgs T) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k;
     if (i > G.nx + 1 || j > G.ny + 1 || k > G.nz + 1) return;
@@ -677,6 +702,7 @@ struct BCArgs {
 // thread per ghost cell of the halo surface: the two x layers (all j, k), the two y layers
 // (interior i, all k), the two z layers (interior i, j); reads touch only interior cells.
 __global__ void k_prd_ghosts(Geo G, BC bc, double* prd1) {
+    pdl_wait();
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     const long long nxf = 2LL * (ny + 2) * (nz + 2), nyf = 2LL * nx * (nz + 2), nzf = 2LL * nx * ny;
@@ -699,6 +725,7 @@ __global__ void k_prd_ghosts(Geo G, BC bc, double* prd1) {
 
 // y walls (:58-114), thread per (i,k)
 __global__ void k_bc_y(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz, ny1 = ny + 1;
     const bool per = (bc.y0 == 0 && bc.yf == 0);
@@ -743,6 +770,7 @@ __global__ void k_bc_y(Geo G, BC bc, BCArgs A) {
 
 // x walls (:116-197), thread per (j,k)
 __global__ void k_bc_x(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz, nx1 = nx + 1;
     const bool per = (bc.x0 == 0 && bc.xf == 0);
@@ -788,6 +816,7 @@ __global__ void k_bc_x(Geo G, BC bc, BCArgs A) {
 
 // z walls (:199-241) and the wall-friction capture (:247-264), thread per (i,j)
 __global__ void k_bc_z(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz, nz1 = nz + 1;
     const bool per = (bc.z0 == 0 && bc.zf == 0);
@@ -835,6 +864,7 @@ __global__ void k_bc_z(Geo G, BC bc, BCArgs A) {
 
 // capture of the j = 2 and j = ny planes (:254-264), after the z phase, thread per (i,k)
 __global__ void k_bc_capture_y(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     for (int side = 0; side < 2; ++side) {
@@ -849,6 +879,7 @@ __global__ void k_bc_capture_y(Geo G, BC bc, BCArgs A) {
 
 // obstacle columns (:266-294) in place of the capture, thread per (i, j), 0..nx+2 x 0..ny+2
 __global__ void k_bc_obst(Geo G, ObstMasks M, BCArgs A) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > G.nx + 2 || j > G.ny + 2) return;
     obst_columns(G, M, A.u, A.v, A.w, A.ub, A.vb, A.wb, i, j);
@@ -856,6 +887,7 @@ __global__ void k_bc_obst(Geo G, ObstMasks M, BCArgs A) {
 
 // contorno(3): level set inside the obstacle (:445-481), thread per column (i, j)
 __global__ void k_ls_obst(Geo G, const int* __restrict__ kw, double* ls) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     if (i > G.nx || j > G.ny) return;
     const int top = kw[i + (G.nx + 2) * j] - 1;
@@ -870,6 +902,7 @@ __global__ void k_ls_obst(Geo G, const int* __restrict__ kw, double* ls) {
 // the level set of column i = 1 from the wave (thread per (j, k), 0..ny+1 x 0..nz+2; k = nz+2
 // is the top row of bxz0, which the reference leaves unset: 0 here).
 __global__ void k_ls_round_float(Geo G, double* ls) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const int c = G.idx32(t.i, t.j, t.k);
@@ -877,6 +910,7 @@ __global__ void k_ls_round_float(Geo G, double* ls) {
 }
 __global__ void k_waves(Geo G, WaveCoef W, double dx, double dz, double time, double* ls, double* bxx0, double* bxx1,
                         double* bxz0) {
+    pdl_wait();
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     const int ny = G.ny, nz = G.nz, row = ny + 2;
     if (j > ny + 1 || k > nz + 2) return;
@@ -890,6 +924,7 @@ __global__ void k_waves(Geo G, WaveCoef W, double dx, double dz, double time, do
 
 // nlock = 2: boundary-normal velocities, y then x then z (:297-441)
 __global__ void k_bc_ny(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz, ny1 = ny + 1, lv = nx + 2;
     if (i > nx + 1 || k > nz + 1) return;
@@ -903,6 +938,7 @@ __global__ void k_bc_ny(Geo G, BC bc, BCArgs A) {
     if (bc.yf == 3) FIDX(v, i, ny1, k) = A.pl.byyf[i + lv * k];
 }
 __global__ void k_bc_nx(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz, nx1 = nx + 1, ly = ny + 2;
     const bool per = (bc.x0 == 0 && bc.xf == 0);
@@ -923,6 +959,7 @@ __global__ void k_bc_nx(Geo G, BC bc, BCArgs A) {
     }
 }
 __global__ void k_bc_nz(Geo G, BC bc, BCArgs A) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = G.nx, ny = G.ny, nz = G.nz, nz1 = nz + 1, lv = nx + 2;
     if (i > nx + 1 || j > ny + 1) return;
@@ -943,6 +980,7 @@ __global__ void k_bc_nz(Geo G, BC bc, BCArgs A) {
 constexpr int kFixThreads = 1024;
 __global__ void __launch_bounds__(kFixThreads) k_outflow_fix(Geo G, BCArgs A, const int* __restrict__ ku, double dx,
                                                             double dy, double dz) {
+    pdl_wait();
     __shared__ double s_delta;
     const int nx = G.nx, ny = G.ny, nz = G.nz, tid = threadIdx.x;
     double fx = 0., fy = 0., fz = 0., open = 0.;
@@ -1048,6 +1086,7 @@ __device__ __forceinline__ void mx_level0(const Geo& G, const BC& bc, const MXSe
 template <bool MX>
 __global__ void __launch_bounds__(256) k_cg_faces(Geo G, BC bc, CGConst K, const double* __restrict__ rho, double* sx,
                                                   double* sy, double* sz, MXSetup M) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k;
     if (i > G.nx || j > G.ny || k > G.nz) return;
@@ -1078,6 +1117,7 @@ __global__ void __launch_bounds__(256) k_cg_diag(Geo G, BC bc, CGConst K, const 
                                                  const double* __restrict__ u, const double* __restrict__ v,
                                                  const double* __restrict__ w, const double* __restrict__ prd1,
                                                  double* d, double* e, double* b, double* sdo, double* isdo) {
+    pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k;
     if (i > G.nx || j > G.ny || k > G.nz) return;
@@ -1111,6 +1151,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
                                                     const double* __restrict__ prd1, double* ax, double* ay,
                                                     double* az, double* r, CGState* st, double* partial,
                                                     unsigned int* counter, MXSetup M) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     double rr = 0.0, bbv = 0.0, ru2 = 0.0, um = 0.0;
@@ -1349,6 +1390,7 @@ __global__ void __launch_bounds__(kTX * kTY) k_cg_update(Geo G, double* __restri
 __global__ void __launch_bounds__(256) k_cg_divcheck(Geo G, const double* __restrict__ sd,
                                                      const double* __restrict__ r, CGState* st, double* partial,
                                                      unsigned int* counter) {
+    pdl_wait();
     if (!st->done || st->status != 0 || !(st->div_tol > 0.)) return;
     const Thread3 t = tid3(1, 1, 1);
     double m = 0.;
@@ -1371,6 +1413,7 @@ __global__ void __launch_bounds__(256) k_cg_divcheck(Geo G, const double* __rest
 // de-normalisation over the halo box (:268-274)
 __global__ void k_cg_final(Geo G, BC bc, const double* __restrict__ sdv, const double* __restrict__ e,
                            double* prd1, const CGState* st) {
+    pdl_wait();
     const Thread3 t = tid3(0, 0, 0);
     const int i = t.i, j = t.j, k = t.k, nx = G.nx, ny = G.ny, nz = G.nz;
     if (i > nx + 1 || j > ny + 1 || k > nz + 1) return;
@@ -1396,13 +1439,15 @@ constexpr int kPosZ = 8;
 __global__ void __launch_bounds__(256) k_posdin(Geo G, BC bc, double aux1, double aux2, double aux3,
                                                 const double* __restrict__ rho, const double* __restrict__ prd1,
                                                 double* __restrict__ u, double* __restrict__ v,
-                                                double* __restrict__ w) {
+                                                double* __restrict__ w, double* __restrict__ prd) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k0 = blockIdx.z * kPosZ + 1;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     if (i > nx + 1 || j > ny + 1) return;
     const int k1 = min(k0 + kPosZ - 1, nz + 1);
     for (int k = k0; k <= k1; ++k) {
+        copy_box(G, prd1, prd, i, j, k);   // prd = prd1
         if (j <= ny && k <= nz) {
             const double rhox = rho_face_x(G, bc, rho, i, j, k);
             FIDX(u, i, j, k) = FIDX(u, i, j, k) - aux1 * (FIDX(prd1, i, j, k) - FIDX(prd1, i - 1, j, k)) / rhox;
@@ -1427,6 +1472,7 @@ constexpr int kEstZ = 4, kEstChunks = 4;
 __global__ void __launch_bounds__(256) k_est(Geo G, double rdx, double rdy, double rdz, const double* __restrict__ u,
                                              const double* __restrict__ v, const double* __restrict__ w,
                                              double* partial, unsigned int* counter, double* out) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     double m = 0.;
     if (i <= G.nx && j <= G.ny) {
@@ -1481,12 +1527,23 @@ static LsConst ls_const(const suli_ctx* c) {
 static dim3 cells_grid(const Geo& g) { return grid3(g.nx, g.ny, g.nz, kBlk); }
 static dim3 faces_grid(const Geo& g) { return grid3(g.nx + 1, g.ny + 1, g.nz + 1, kBlk); }
 
+// Launch a kernel of the step (each calls pdl_wait first).  Behind another kernel of the same call
+// (c->chained) it is a dependent launch, which overlaps its start with the end of the one before:
+// the grids of a small step run shorter than a plain launch takes.  Behind anything else (a copy,
+// a memset, work a caller put on the stream) it is a plain launch.
+template <typename... KArgs, typename... Args>
+static void step_launch(suli_ctx* c, void (*kernel)(KArgs...), dim3 grid, dim3 block, Args... args) {
+    if (c->chained) pdl_launch(kernel, grid, block, c->stream, args...);
+    else kernel<<<grid, block, 0, c->stream>>>(static_cast<KArgs>(args)...);
+    c->chained = true;
+}
+
 // stencil arithmetic in FP32 for the mixed-precision path (precision 1), FP64 otherwise; the
 // fields stay FP64 either way
 #define LAUNCH_R(kern, grid, block, ...)                                                   \
     do {                                                                                   \
-        if (c->P.precision == 1) kern<float><<<(grid), (block), 0, c->stream>>>(__VA_ARGS__);  \
-        else kern<double><<<(grid), (block), 0, c->stream>>>(__VA_ARGS__);                 \
+        if (c->P.precision == 1) step_launch(c, kern<float>, (grid), (block), __VA_ARGS__);  \
+        else step_launch(c, kern<double>, (grid), (block), __VA_ARGS__);                 \
     } while (0)
 
 void launch_lsprops(suli_ctx* c, const double* ls, bool do_mod, bool do_hs, bool do_vol) {
@@ -1522,18 +1579,18 @@ void launch_reinit_stage(suli_ctx* c, const double* cur, const double* phi0, dou
 void launch_reinit_err(suli_ctx* c, const double* after, const double* before, double band) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_REINIT, 1);
-    k_reinit_err<<<cells_grid(G), kBlk, 0, c->stream>>>(G, after, before, band, c->red_partial, c->red_counter,
+    step_launch(c, k_reinit_err, cells_grid(G), kBlk, G, after, before, band, c->red_partial, c->red_counter,
                                                          c->red_out);
 }
 void launch_ls_shift(suli_ctx* c, double shift) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_VOLFIX, 1);
-    k_ls_shift<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->f[SULI_F_LS], shift);
+    step_launch(c, k_ls_shift, cells_grid(G), kBlk, G, c->f[SULI_F_LS], shift);
 }
 void launch_volfix(suli_ctx* c, double dt1fac) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_VOLFIX, 1);
-    k_volfix<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->f[SULI_F_LS], c->f[SULI_F_MOD_LS], dt1fac, c->vol_ini);
+    step_launch(c, k_volfix, cells_grid(G), kBlk, G, c->f[SULI_F_LS], c->f[SULI_F_MOD_LS], dt1fac, c->vol_ini);
 }
 constexpr int kNutZ = 4;   // cells of a column per thread in k_nut
 void launch_visco(suli_ctx* c) {
@@ -1545,12 +1602,12 @@ void launch_visco(suli_ctx* c) {
         V.itdx = 1. / (2. * c->P.dx); V.itdy = 1. / (2. * c->P.dy); V.itdz = 1. / (2. * c->P.dz);
         V.cx = c->P.dx * c->P.dx * cs * cs; V.cy = c->P.dy * c->P.dy * cs * cs; V.cz = c->P.dz * c->P.dz * cs * cs;
         if (c->P.precision == 1)
-            k_facenu_dir<float><<<faces_grid(G), kBlk, 0, c->stream>>>(G, V, c->f[SULI_F_U], c->f[SULI_F_V],
+            step_launch(c, k_facenu_dir<float>, faces_grid(G), kBlk, G, V, c->f[SULI_F_U], c->f[SULI_F_V],
                                                                      c->f[SULI_F_W], c->f[SULI_F_LS_NU],
                                                                      c->f[SULI_F_XNUT], c->f[SULI_F_YNUT],
                                                                      c->f[SULI_F_ZNUT]);
         else
-            k_facenu_dir<double><<<faces_grid(G), kBlk, 0, c->stream>>>(G, V, c->f[SULI_F_U], c->f[SULI_F_V],
+            step_launch(c, k_facenu_dir<double>, faces_grid(G), kBlk, G, V, c->f[SULI_F_U], c->f[SULI_F_V],
                                                                       c->f[SULI_F_W], c->f[SULI_F_LS_NU],
                                                                       c->f[SULI_F_XNUT], c->f[SULI_F_YNUT],
                                                                       c->f[SULI_F_ZNUT]);
@@ -1565,35 +1622,34 @@ void launch_visco(suli_ctx* c) {
         const double *u = c->f[SULI_F_U], *v = c->f[SULI_F_V], *w = c->f[SULI_F_W], *rho = c->f[SULI_F_RHO];
         double* nut = c->f[SULI_F_NUT];
         if (c->P.precision == 1) {   // FP32 arithmetic over the FP64 state
-            if (col) k_nut<float, kNutZ><<<gn, kBlk, 0, c->stream>>>(G, V, u, v, w, rho, nut);
-            else k_nut<float, 1><<<gn, kBlk, 0, c->stream>>>(G, V, u, v, w, rho, nut);
+            if (col) step_launch(c, (k_nut<float, kNutZ>), gn, kBlk, G, V, u, v, w, rho, nut);
+            else step_launch(c, (k_nut<float, 1>), gn, kBlk, G, V, u, v, w, rho, nut);
         } else {
-            if (col) k_nut<double, kNutZ><<<gn, kBlk, 0, c->stream>>>(G, V, u, v, w, rho, nut);
-            else k_nut<double, 1><<<gn, kBlk, 0, c->stream>>>(G, V, u, v, w, rho, nut);
+            if (col) step_launch(c, (k_nut<double, kNutZ>), gn, kBlk, G, V, u, v, w, rho, nut);
+            else step_launch(c, (k_nut<double, 1>), gn, kBlk, G, V, u, v, w, rho, nut);
         }
     }
-    k_facenu<<<faces_grid(G), kBlk, 0, c->stream>>>(G, c->P.m_turb, c->f[SULI_F_LS_NU], c->f[SULI_F_NUT],
+    step_launch(c, k_facenu, faces_grid(G), kBlk, G, c->P.m_turb, c->f[SULI_F_LS_NU], c->f[SULI_F_NUT],
                                                      c->f[SULI_F_XNUT], c->f[SULI_F_YNUT], c->f[SULI_F_ZNUT]);
 }
 template <typename R>
 static void convdiff_der(suli_ctx* c, const CDConst& C, const CDFields& F) {
     const Geo& G = c->g;
     if (c->P.adv_type == 2) {
-        k_convdiff<R, 1, 2><<<faces_grid(G), kBlk, 0, c->stream>>>(G, C, F);
+        step_launch(c, (k_convdiff<R, 1, 2>), faces_grid(G), kBlk, G, C, F);
         return;
     }
     if (c->P.adv_type == 3) {
-        k_convdiff<R, 1, 3><<<faces_grid(G), kBlk, 0, c->stream>>>(G, C, F);
+        step_launch(c, (k_convdiff<R, 1, 3>), faces_grid(G), kBlk, G, C, F);
         return;
     }
     switch (c->P.der) {
-    case 2: k_convdiff<R, 2, 1><<<faces_grid(G), kBlk, 0, c->stream>>>(G, C, F); break;
-    case 3: k_convdiff<R, 3, 1><<<faces_grid(G), kBlk, 0, c->stream>>>(G, C, F); break;
-    default: k_convdiff<R, 1, 1><<<faces_grid(G), kBlk, 0, c->stream>>>(G, C, F); break;
+    case 2: step_launch(c, (k_convdiff<R, 2, 1>), faces_grid(G), kBlk, G, C, F); break;
+    case 3: step_launch(c, (k_convdiff<R, 3, 1>), faces_grid(G), kBlk, G, C, F); break;
+    default: step_launch(c, (k_convdiff<R, 1, 1>), faces_grid(G), kBlk, G, C, F); break;
     }
 }
 void launch_convdiff(suli_ctx* c) {
-    const Geo& G = c->g;
     CDConst C;
     C.idx = 1. / c->P.dx; C.idy = 1. / c->P.dy; C.idz = 1. / c->P.dz;
     C.gx = c->P.gx; C.gz = c->P.gz; C.sigma = c->P.sigma;
@@ -1608,8 +1664,8 @@ void launch_convdiff(suli_ctx* c) {
     F.ub = c->f[SULI_F_UB]; F.vb = c->f[SULI_F_VB]; F.wb = c->f[SULI_F_WB];
     F.tfu = c->f[SULI_F_TF_U]; F.tfv = c->f[SULI_F_TF_V]; F.tfw = c->f[SULI_F_TF_W];
     F.Fu = c->f[SULI_F_FU]; F.Fv = c->f[SULI_F_FV]; F.Fw = c->f[SULI_F_FW];
+    F.prd1 = c->f[SULI_F_PRD1]; F.prd0 = c->f[SULI_F_PRD0];
     ProfScope ps(c, SULI_K_CONVDIFF, 1);
-    cudaMemcpyAsync(c->f[SULI_F_PRD0], c->f[SULI_F_PRD1], G.n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
     if (c->P.precision == 1)   // FP32 arithmetic over the FP64 state
         convdiff_der<float>(c, C, F);
     else
@@ -1625,15 +1681,16 @@ void launch_tempo(suli_ctx* c, int tt, int it) {
     T.f1[0] = c->f[SULI_F_FU1]; T.f1[1] = c->f[SULI_F_FV1]; T.f1[2] = c->f[SULI_F_FW1];
     T.tm = c->P.t_tempo; T.tt = tt; T.it = it; T.dt = c->dt;
     ProfScope ps(c, SULI_K_TEMPO, 1);
-    k_tempo<<<faces_grid(G), kBlk, 0, c->stream>>>(G, T);
+    step_launch(c, k_tempo, faces_grid(G), kBlk, G, T);
 }
 void launch_boundary_waves(suli_ctx* c) {
     const Geo& G = c->g;
     const dim3 b2(32, 8);
     ProfScope ps(c, SULI_K_CONTORNO, 2);
-    k_ls_round_float<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->f[SULI_F_LS]);
+    step_launch(c, k_ls_round_float, cells_grid(G), kBlk, G, c->f[SULI_F_LS]);
     cudaMemsetAsync(c->f[SULI_F_BXY0], 0, c->plane_elems[SULI_F_BXY0] * sizeof(double), c->stream);   // v1 never set
-    k_waves<<<grid3(G.ny + 2, G.nz + 3, 1, b2), b2, 0, c->stream>>>(G, c->wave, c->P.dx, c->P.dz, c->t, c->f[SULI_F_LS],
+    c->chained = false;
+    step_launch(c, k_waves, grid3(G.ny + 2, G.nz + 3, 1, b2), b2, G, c->wave, c->P.dx, c->P.dz, c->t, c->f[SULI_F_LS],
                                                                      c->f[SULI_F_BXX0], c->f[SULI_F_BXX1], c->f[SULI_F_BXZ0]);
 }
 void launch_contorno(suli_ctx* c, int nlock) {
@@ -1644,7 +1701,7 @@ void launch_contorno(suli_ctx* c, int nlock) {
         if (!obst) return;
         {
             ProfScope ps(c, SULI_K_CONTORNO, 1);
-            k_ls_obst<<<grid3(G.nx, G.ny, 1, b2), b2, 0, c->stream>>>(G, c->obst_kw, c->f[SULI_F_LS]);
+            step_launch(c, k_ls_obst, grid3(G.nx, G.ny, 1, b2), b2, G, c->obst_kw, c->f[SULI_F_LS]);
         }
         launch_lsprops(c, c->f[SULI_F_LS], false, true, false);   // heaviside()
         return;
@@ -1662,22 +1719,22 @@ void launch_contorno(suli_ctx* c, int nlock) {
                                          (capy || obst ? 1 : 0));
     {
         const long long ng = 2LL * (G.ny + 2) * (G.nz + 2) + 2LL * G.nx * (G.nz + 2) + 2LL * G.nx * G.ny;
-        k_prd_ghosts<<<(unsigned)((ng + 255) / 256), 256, 0, c->stream>>>(G, c->bc, A.prd1);
+        step_launch(c, k_prd_ghosts, (unsigned)((ng + 255) / 256), 256, G, c->bc, A.prd1);
     }
-    k_bc_y<<<grid3(G.nx + 3, G.nz + 3, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
-    k_bc_x<<<grid3(G.ny + 3, G.nz + 3, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
-    k_bc_z<<<grid3(G.nx + 3, G.ny + 3, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
-    if (capy) k_bc_capture_y<<<grid3(G.nx + 3, G.nz + 3, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
+    step_launch(c, k_bc_y, grid3(G.nx + 3, G.nz + 3, 1, b2), b2, G, c->bc, A);
+    step_launch(c, k_bc_x, grid3(G.ny + 3, G.nz + 3, 1, b2), b2, G, c->bc, A);
+    step_launch(c, k_bc_z, grid3(G.nx + 3, G.ny + 3, 1, b2), b2, G, c->bc, A);
+    if (capy) step_launch(c, k_bc_capture_y, grid3(G.nx + 3, G.nz + 3, 1, b2), b2, G, c->bc, A);
     if (obst) {
         const ObstMasks M{c->obst_ku, c->obst_kv, c->obst_kw};
-        k_bc_obst<<<grid3(G.nx + 3, G.ny + 3, 1, b2), b2, 0, c->stream>>>(G, M, A);
+        step_launch(c, k_bc_obst, grid3(G.nx + 3, G.ny + 3, 1, b2), b2, G, M, A);
     }
     if (nlock == 2) {
-        k_bc_ny<<<grid3(G.nx + 2, G.nz + 2, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
-        k_bc_nx<<<grid3(G.ny + 3, G.nz + 3, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
-        k_bc_nz<<<grid3(G.nx + 2, G.ny + 2, 1, b2), b2, 0, c->stream>>>(G, c->bc, A);
+        step_launch(c, k_bc_ny, grid3(G.nx + 2, G.nz + 2, 1, b2), b2, G, c->bc, A);
+        step_launch(c, k_bc_nx, grid3(G.ny + 3, G.nz + 3, 1, b2), b2, G, c->bc, A);
+        step_launch(c, k_bc_nz, grid3(G.nx + 2, G.ny + 2, 1, b2), b2, G, c->bc, A);
         if (c->P.outflow_fix == 1 && c->bc.xf == 4)
-            k_outflow_fix<<<1, kFixThreads, 0, c->stream>>>(G, A, obst ? c->obst_ku : nullptr, c->P.dx, c->P.dy,
+            step_launch(c, k_outflow_fix, 1, kFixThreads, G, A, obst ? c->obst_ku : nullptr, c->P.dx, c->P.dy,
                                                             c->P.dz);
     }
 }
@@ -1710,13 +1767,12 @@ void launch_cg_setup(suli_ctx* c, bool mixed, bool mixed_residual) {
     // face scratch: the CG direction and product vectors, written again before the iterations read them
     double *sx = c->cg_pa, *sy = c->cg_pb, *sz = c->cg_q;
     const auto faces = mixed ? k_cg_faces<true> : k_cg_faces<false>;
-    faces<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->bc, K, c->f[SULI_F_RHO], sx, sy, sz, M);
-    k_cg_diag<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->bc, K, sx, sy, sz, c->f[SULI_F_U], c->f[SULI_F_V], c->f[SULI_F_W],
+    step_launch(c, faces, cells_grid(G), kBlk, G, c->bc, K, c->f[SULI_F_RHO], sx, sy, sz, M);
+    step_launch(c, k_cg_diag, cells_grid(G), kBlk, G, c->bc, K, sx, sy, sz, c->f[SULI_F_U], c->f[SULI_F_V], c->f[SULI_F_W],
                                                       c->f[SULI_F_PRD1], c->rec_in ? c->cg_d : nullptr, c->cg_e, c->cg_b,
                                                       c->cg_sd, c->cg_isd);
     const auto coef = mixed_residual ? k_cg_coef<true> : k_cg_coef<false>;
-    coef<<<grid3(G.nx, G.ny, (G.nz + kCoefZ - 1) / kCoefZ, kBlk), kBlk, 0, c->stream>>>(
-        G, c->bc, K, sx, sy, sz, c->cg_sd, c->cg_isd, c->cg_e, c->cg_b, c->f[SULI_F_PRD1], c->cg_ax, c->cg_ay, c->cg_az,
+    step_launch(c, coef, grid3(G.nx, G.ny, (G.nz + kCoefZ - 1) / kCoefZ, kBlk), kBlk, G, c->bc, K, sx, sy, sz, c->cg_sd, c->cg_isd, c->cg_e, c->cg_b, c->f[SULI_F_PRD1], c->cg_ax, c->cg_ay, c->cg_az,
         c->cg_r, c->cg, c->red_partial, c->red_counter, M);
 }
 void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
@@ -1797,26 +1853,26 @@ cudaError_t launch_cg_coop(suli_ctx* c) {
 void launch_cg_divcheck(suli_ctx* c) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_CG_FINAL, 1);
-    k_cg_divcheck<<<cells_grid(G), kBlk, 0, c->stream>>>(G, c->cg_sd, c->cg_r, c->cg, c->red_partial, c->red_counter);
+    step_launch(c, k_cg_divcheck, cells_grid(G), kBlk, G, c->cg_sd, c->cg_r, c->cg, c->red_partial, c->red_counter);
 }
 void launch_cg_final(suli_ctx* c, const double* e) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_CG_FINAL, 1);
-    k_cg_final<<<grid3(G.nx + 2, G.ny + 2, G.nz + 2, kBlk), kBlk, 0, c->stream>>>(G, c->bc, c->cg_sd, e,
+    step_launch(c, k_cg_final, grid3(G.nx + 2, G.ny + 2, G.nz + 2, kBlk), kBlk, G, c->bc, c->cg_sd, e,
                                                                                    c->f[SULI_F_PRD1], c->cg);
 }
 void launch_posdin(suli_ctx* c) {
     const Geo& G = c->g;
     const double aux1 = c->dt / c->P.dx, aux2 = c->dt / c->P.dy, aux3 = c->dt / c->P.dz;
     ProfScope ps(c, SULI_K_POSDIN, 1);
-    k_posdin<<<grid3(G.nx + 1, G.ny + 1, (G.nz + 1 + kPosZ - 1) / kPosZ, kBlk), kBlk, 0, c->stream>>>(G, c->bc, aux1, aux2, aux3, c->f[SULI_F_RHO], c->f[SULI_F_PRD1],
-                                                     c->f[SULI_F_U], c->f[SULI_F_V], c->f[SULI_F_W]);
-    cudaMemcpyAsync(c->f[SULI_F_PRD], c->f[SULI_F_PRD1], G.n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
+    step_launch(c, k_posdin, grid3(G.nx + 1, G.ny + 1, (G.nz + 1 + kPosZ - 1) / kPosZ, kBlk), kBlk, G, c->bc, aux1, aux2,
+                aux3, c->f[SULI_F_RHO], c->f[SULI_F_PRD1], c->f[SULI_F_U], c->f[SULI_F_V], c->f[SULI_F_W],
+                c->f[SULI_F_PRD]);
 }
 void launch_est(suli_ctx* c) {
     const Geo& G = c->g;
     ProfScope ps(c, SULI_K_EST, 1);
-    k_est<<<grid3(G.nx, G.ny, (G.nz + kEstZ * kEstChunks - 1) / (kEstZ * kEstChunks), kBlk), kBlk, 0, c->stream>>>(G, 1. / c->P.dx, 1. / c->P.dy, 1. / c->P.dz, c->f[SULI_F_U],
+    step_launch(c, k_est, grid3(G.nx, G.ny, (G.nz + kEstZ * kEstChunks - 1) / (kEstZ * kEstChunks), kBlk), kBlk, G, 1. / c->P.dx, 1. / c->P.dy, 1. / c->P.dz, c->f[SULI_F_U],
                                                   c->f[SULI_F_V], c->f[SULI_F_W], c->red_partial, c->red_counter,
                                                   c->red_out);
 }

@@ -4,12 +4,21 @@
 // the stream is still draining; it waits in pdl_wait() (griddepcontrol.wait) before reading
 // anything the predecessor wrote, which overlaps the launch and block ramp-up of consecutive
 // iteration kernels.  For a plain launch pdl_wait() is a no-op.
+//
+// A grid of at most one block an SM also lets its successor start as soon as it has waited itself
+// (griddepcontrol.launch_dependents), instead of when its blocks have exited: a 64x32x32 mixed
+// step 3.31 -> 3.20 ms.  Larger grids need the SMs' slots for their own blocks: with the early start
+// for up to 300 blocks the 256x128x128 step went from 13.80 to 14.17 ms, for all grids 14.41.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace suli {
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+constexpr unsigned int kPdlEarlyBlocks = 148;   // one a B200 SM
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (gridDim.x * gridDim.y * gridDim.z <= kPdlEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // launch with programmatic stream serialisation (the kernel calls pdl_wait before its loads)
 template <typename... KArgs, typename... Args>

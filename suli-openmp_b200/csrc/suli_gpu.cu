@@ -25,6 +25,13 @@ int fail(suli_ctx* c, int code, const std::string& msg) {
     return code;
 }
 
+// start of a call that launches kernels of the step: what a caller put on the stream before it is not
+// ours, so the first kernel is launched plainly (step_launch)
+void enter(suli_ctx* c) {
+    cudaSetDevice(c->device);
+    if (!c->in_step) c->chained = false;
+}
+
 #define CUDA_TRY(c, expr)                                                                       \
     do {                                                                                        \
         cudaError_t e_ = (expr);                                                                \
@@ -482,7 +489,7 @@ int suli_set_obstacle(suli_ctx* c, const int* ku, const int* kv, const int* kw) 
 int suli_boundary_waves(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
     if (c->P.wave_t == 0) return fail(c, SULI_ERR_ARG, "boundary_waves: wave_t is 0");
-    cudaSetDevice(c->device);
+    enter(c);
     if (c->wave.type != c->P.wave_t) c->wave = wave_coefficients(c->P.wave_t, c->P.gz);
     launch_boundary_waves(c);
     CHECK_LAUNCH(c);
@@ -534,7 +541,7 @@ int suli_iniciais(suli_ctx* c, double u_init) {
 
 int suli_heaviside(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     launch_lsprops(c, c->f[SULI_F_LS], false, true, false);
     CHECK_LAUNCH(c);
     return SULI_OK;
@@ -542,7 +549,7 @@ int suli_heaviside(suli_ctx* c) {
 
 int suli_mod_ls1(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     launch_lsprops(c, c->f[SULI_F_LS], true, false, false);
     launch_curv(c);
     CHECK_LAUNCH(c);
@@ -551,7 +558,7 @@ int suli_mod_ls1(suli_ctx* c) {
 
 int suli_level_set_ini(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     if (c->P.t_hs != 0) {   // the preset shifted by ls_m for the geometric mix (14_level_set.f90:47-51, 196-202)
         const double dx1 = fmax(c->P.dx, fmax(c->P.dy, c->P.dz));
         launch_ls_shift(c, 0.481803535 * dx1 * c->P.alpha1);
@@ -568,7 +575,7 @@ int suli_level_set_ini(suli_ctx* c) {
 // level_set (14_level_set.f90:221-285)
 int suli_level_set(suli_ctx* c, double* vol_ins) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     const double adtl[3] = {1., 3. / 4., 1. / 3.}, bdtl[3] = {0., 1. / 4., 2. / 3.}, gdtl[3] = {1., 1. / 4., 2. / 3.};
     double* L0 = c->f[SULI_F_LS];
     double* L1 = c->ls1;
@@ -629,7 +636,7 @@ int suli_level_set(suli_ctx* c, double* vol_ins) {
 
 int suli_visco(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     launch_visco(c);
     CHECK_LAUNCH(c);
     return SULI_OK;
@@ -637,7 +644,7 @@ int suli_visco(suli_ctx* c) {
 
 int suli_convdiff(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     launch_convdiff(c);
     CHECK_LAUNCH(c);
     return SULI_OK;
@@ -646,7 +653,7 @@ int suli_convdiff(suli_ctx* c) {
 int suli_tempo(suli_ctx* c, int tt, int it) {
     if (!c) return SULI_ERR_ARG;
     if (tt < 1 || tt > 3) return fail(c, SULI_ERR_ARG, "tempo: tt must be 1..3");
-    cudaSetDevice(c->device);
+    enter(c);
     launch_tempo(c, tt, it);
     CHECK_LAUNCH(c);
     return SULI_OK;
@@ -656,7 +663,7 @@ int suli_contorno(suli_ctx* c, int nlock) {
     if (!c) return SULI_ERR_ARG;
     if (nlock < 1 || nlock > 3) return fail(c, SULI_ERR_ARG, "contorno: nlock must be 1..3");
     if (c->P.obst_t != 0 && !c->obst_k) return fail(c, SULI_ERR_ARG, "contorno: obst_t != 0 needs suli_set_obstacle first");
-    cudaSetDevice(c->device);
+    enter(c);
     launch_contorno(c, nlock);
     CHECK_LAUNCH(c);
     return SULI_OK;
@@ -938,7 +945,7 @@ extern "C" {
 
 int suli_graddin(suli_ctx* c, int* iters, double* resid) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     if (c->P.precision == 1) return graddin_mixed(c, iters, resid);
     return graddin_fp64(c, iters, resid, true);
 }
@@ -977,7 +984,7 @@ int suli_graddin_record(suli_ctx* c, float* d_in3, float* d_target, int* iters, 
 
 int suli_posdin(suli_ctx* c) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     launch_posdin(c);
     CHECK_LAUNCH(c);
     return SULI_OK;
@@ -985,7 +992,7 @@ int suli_posdin(suli_ctx* c) {
 
 int suli_est(suli_ctx* c, double* max_div) {
     if (!c) return SULI_ERR_ARG;
-    cudaSetDevice(c->device);
+    enter(c);
     launch_est(c);
     CHECK_LAUNCH(c);
     int r = sync_read(c, c->red_out, c->host_scalars, sizeof(double));
@@ -1066,6 +1073,9 @@ static int io_send(suli_ctx* c, int slot, int field, double* host) {
 // The time step (1_principal.f90:64-108); `io` (suli_step_host) places the overlapped copies.
 static int step_body(suli_ctx* c, int it, suli_step_stats* st, const StepIO* io) {
     int status = SULI_OK;
+    c->chained = false;
+    c->in_step = true;
+    struct Leave { suli_ctx* c; ~Leave() { c->in_step = false; } } leave{c};
     c->t = it * c->dt;
     int r = suli_level_set(c, nullptr);
     if (r < 0) return r;

@@ -17,9 +17,21 @@
 //
 // Per cell the arithmetic is the vectorised kernels' (the same operator, faces and update
 // expressions in the same order), so the values are the same bits; the FP64 dot products sum
-// in another grouping.  Used on level 0 when no x or y axis is periodic (a wrapped neighbour
+// in another grouping.  Used on level 0 when the x axis is not periodic (a wrapped neighbour
 // would lie outside the tile), nx is a multiple of 16 (the row pitch then holds the tile's
 // last x neighbour) and the device grants the shared memory.
+//
+// On a periodic y axis (more than 8 rows) the first tile's row below is row ny and the last tile's
+// row above is row 1, outside the box: one bulk copy a field and plane brings that row behind the
+// box (slot row kSBoxY; no tile needs both), and the neighbour's row number points there.  (The
+// density needs none: faces at the box's end take the next interior face's value.)  The inner
+// solves of a 512x256x256 channel step, on the vectorised kernels before: 58.9 -> 49.0 ms.
+//
+// Issue-bound as much as bandwidth-bound (50-56 % of issue slots at 256x128x128), so a march keeps
+// the quad's values below and at the plane, and the density at it, in registers (SCol, SZCarry):
+// one shared-memory quad and its arithmetic a plane instead of three (inner solves of a 256x128x128
+// step 8.38 -> 8.21 ms).  A deeper ring, loads of the fixed fields ahead of the wait for the
+// preceding kernel, and three CTAs an SM with a ring of four gave nothing or cost 1-4 %.
 //
 // Every wait on a slot is bounded: a wait that runs out makes the CTA wait (bounded again) for
 // the loads it issued, sets the inner solve's status to SULI_ERR_CUDA and done, and return; the
@@ -36,14 +48,16 @@ constexpr int kSTX = 32, kSTY = 8;                             // threads: quads
 constexpr int kSTileX = kSTX * kVX;                            // 128 cells along x
 constexpr int kSBoxX = kSTileX + 8;                            // 4 cells before the tile .. 4 after
 constexpr int kSBoxY = kSTY + 2;                               // one row on each side
-constexpr int kSBoxBytes = kSBoxX * kSBoxY * 4;                // 5440
-constexpr int kSSlotBytes = (kSBoxBytes + 127) / 128 * 128;    // TMA destinations 128-byte aligned
 constexpr int kSR = 5;                                         // ring: planes k-1, k, k+1 + 2 ahead
+constexpr int kSBoxBytes = kSBoxX * kSBoxY * 4;                // 5440
+constexpr int kSRowBytes = kSBoxX * 4;                         // the wrapped row behind the box
+constexpr int kSSlotBytes = (kSBoxBytes + kSRowBytes + 127) / 128 * 128;   // TMA destinations 128-byte aligned
 // the coarse level's box (the prolongation source of the post-smoothing): the parents of the
 // tile's cells and of their neighbours, 72 floats x 6 rows from coarse cell 64 bx - 3, row 4 by
 constexpr int kSCBoxX = 72, kSCBoxY = 6;
 constexpr int kSCBoxBytes = kSCBoxX * kSCBoxY * 4;              // 1728
-constexpr int kSCSlotBytes = (kSCBoxBytes + 127) / 128 * 128;
+constexpr int kSCRowBytes = kSCBoxX * 4;
+constexpr int kSCSlotBytes = (kSCBoxBytes + kSCRowBytes + 127) / 128 * 128;
 
 // a field read only at the thread's own cells: the tile without halo, 128 floats x 8 rows
 constexpr int kSOBoxX = kSTileX, kSOBoxY = kSTY;
@@ -82,10 +96,22 @@ __device__ __forceinline__ void s_tma3(uint32_t dst, const CUtensorMap* map, int
         : "memory");
 }
 
+// one row by an untiled bulk copy (both addresses and the size multiples of 16 bytes)
+__device__ __forceinline__ void s_row(uint32_t dst, const float* src, int bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
 // a quad / one value of a slot at tile row ly, tile column lx (lx of a quad a multiple of 4)
 __device__ __forceinline__ V4 sq(const float* s, int ly, int lx) {
     const float4 t = *reinterpret_cast<const float4*>(s + ly * kSBoxX + lx);
     return V4{{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ void sqa(const float* s, int ly, int lx, float (&o)[kVX]) {
+    const V4 t = sq(s, ly, lx);
+#pragma unroll
+    for (int e = 0; e < kVX; ++e) o[e] = t.v[e];
 }
 __device__ __forceinline__ float ss(const float* s, int ly, int lx) { return s[ly * kSBoxX + lx]; }
 // the thread's quad in a slot of a field read at its own cells only
@@ -97,7 +123,8 @@ __device__ __forceinline__ V4 sqo(const float* s) {
 __device__ __forceinline__ float ssc(const float* s, int ly, int lx) { return s[ly * kSCBoxX + lx]; }
 
 // A thread's quad in the tile and the tile positions of its neighbours: the unknowns' Neumann
-// map (a neighbour outside the box is the cell itself) and the faces' clamped end rule (the
+// map (a neighbour outside the box is the cell itself, or on a periodic y axis in the slot's wrapped
+// row) and the faces' clamped end rule (the
 // face at the box's end is the next interior face), as vquad and OpRho4::faces take them
 struct STile {
     int i0, j, c0;        // first cell of the quad, its index in plane 0
@@ -106,7 +133,7 @@ struct STile {
     int fxm, fxp, fym, fyp;   // faces: x neighbours (scalars), rows
     bool in;
 };
-__device__ __forceinline__ STile s_tile(const Geo& G) {
+__device__ __forceinline__ STile s_tile(const Geo& G, const BC& bc) {
     STile t;
     const int tx = threadIdx.x, ty = threadIdx.y;
     t.i0 = kSTileX * blockIdx.x + kVX * tx + 1;
@@ -117,8 +144,8 @@ __device__ __forceinline__ STile s_tile(const Geo& G) {
     t.ly = 1 + ty;
     t.uxm = (t.i0 > 1) ? t.qx - 1 : t.qx;
     t.uxp = (t.i0 + kVX - 1 < G.nx) ? t.qx + kVX : t.qx + kVX - 1;
-    t.uym = (t.j > 1) ? t.ly - 1 : t.ly;
-    t.uyp = (t.j < G.ny) ? t.ly + 1 : t.ly;
+    t.uym = (t.j > 1) ? t.ly - 1 : (bc.pery ? kSBoxY : t.ly);
+    t.uyp = (t.j < G.ny) ? t.ly + 1 : (bc.pery ? kSBoxY : t.ly);
     t.fxm = (t.i0 > 1) ? t.qx - 1 : t.qx + 1;
     t.fxp = (t.i0 + kVX - 1 < G.nx) ? t.qx + kVX : t.qx + kVX - 2;
     t.fym = (t.j > 1) ? t.ly - 1 : t.ly + 1;
@@ -132,12 +159,32 @@ __device__ __forceinline__ STile s_tile(const Geo& G) {
 // previous plane of the same march (carried in zc while zk records that plane).
 struct SZCarry {
     float f[kVX];
+    V4 rc;   // the density of plane k + 1
     int k = -1;
+};
+// a quad's values below, at and above the plane of a march: the upper one is loaded, the others are
+// the last plane's (all three at the first plane, from = its three quads)
+struct SCol {
+    float m[kVX], c[kVX], p[kVX];
+    int k = -1;
+    template <class F>
+    __device__ __forceinline__ void next(int kk, F from) {
+        if (k == kk - 1) {
+#pragma unroll
+            for (int e = 0; e < kVX; ++e) { m[e] = c[e]; c[e] = p[e]; }
+        } else {
+            from(0, m);
+            from(1, c);
+        }
+        from(2, p);
+        k = kk;
+    }
 };
 __device__ __forceinline__ void s_faces(const STile& t, int k, int nz, const float* rm, const float* r0,
                                         const float* rp, float cx2, float cy2, float cz2, Faces (&F)[kVX],
                                         SZCarry& zc) {
-    const V4 rc = sq(r0, t.ly, t.qx);
+    const bool up = k > 1 && zc.k == k - 1;
+    const V4 rc = up ? zc.rc : sq(r0, t.ly, t.qx);
     const V4 rym = sq(r0, t.fym, t.qx), ryp = sq(r0, t.fyp, t.qx);
     const float rxm0 = ss(r0, t.ly, t.fxm), rxp3 = ss(r0, t.ly, t.fxp);
     float fx[kVX + 1];
@@ -146,7 +193,7 @@ __device__ __forceinline__ void s_faces(const STile& t, int k, int nz, const flo
     for (int e = 1; e < kVX; ++e) fx[e] = face_div(cx2, rc.v[e - 1] + rc.v[e]);
     fx[kVX] = face_div(cx2, rc.v[kVX - 1] + rxp3);
     float fzm[kVX];
-    if (k > 1 && zc.k == k - 1) {
+    if (up) {
 #pragma unroll
         for (int e = 0; e < kVX; ++e) fzm[e] = zc.f[e];
     } else {
@@ -161,8 +208,17 @@ __device__ __forceinline__ void s_faces(const STile& t, int k, int nz, const flo
         zc.f[e] = face_div(cz2, r + rzp.v[e]);
         F[e] = Faces{fx[e], fx[e + 1], face_div(cy2, r + rym.v[e]), face_div(cy2, r + ryp.v[e]), fzm[e], zc.f[e]};
     }
+    zc.rc = rzp;
     zc.k = k;
 }
+
+// the arrays whose wrapped row a periodic y axis needs: the fine fields with the halo before the
+// density (the last of them), and the coarse field with its row and plane pitch and rows
+struct SWrap {
+    const float* f[2];
+    const float* c;
+    int cpx, cpxy, cny;
+};
 
 // The plane engine.  NF fine fields with the halo, NO fine fields at the tile's own cells (box
 // kSOBox) and NC coarse fields (the parent planes, box kSCBox) are loaded for every plane of the
@@ -180,7 +236,7 @@ struct SSlots {
 };
 template <int NF, int NO, int NC, class Body>
 __device__ __forceinline__ int s_march(const Geo& G, const BC& bc, const CUtensorMap* const (&maps)[NF + NO + NC],
-                                       int chunk, Body& body, PCGState* st) {
+                                       const SWrap& wrap, int chunk, Body& body, PCGState* st) {
     extern __shared__ __align__(128) unsigned char s_smem[];
     constexpr size_t kStage = (size_t)NF * kSSlotBytes + (size_t)NO * kSOSlotBytes + (size_t)NC * kSCSlotBytes;
     const int tid = threadIdx.x + kSTX * threadIdx.y;
@@ -208,12 +264,15 @@ __device__ __forceinline__ int s_march(const Geo& G, const BC& bc, const CUtenso
     auto slot_at = [&](int sidx, int f) -> const float* {
         return reinterpret_cast<const float*>(s_smem + (size_t)sidx * kStage + off(f));
     };
+    // the tile with the first or the last row of a periodic y axis, and the row on its other side
+    const bool edge = bc.pery && (blockIdx.y == 0 || y0 + kSBoxY - 1 > G.ny);
+    const int wrow = (blockIdx.y == 0) ? G.ny : 1;
+    const int slot_bytes = NF * kSBoxBytes + NO * kSOBoxBytes + NC * kSCBoxBytes +
+                           (edge ? (NF - 1) * kSRowBytes + NC * kSCRowBytes : 0);
     auto issue = [&](int q) {
         const int s = q % kSR;
         const uint32_t bar = s_addr(&bars[s]);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(NF * kSBoxBytes + NO * kSOBoxBytes + NC * kSCBoxBytes)
-                     : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(slot_bytes) : "memory");
         const int z = map_any(k0 - 1 + q, G.nz, bc.perz);
         unsigned char* b = s_smem + (size_t)s * kStage;
 #pragma unroll
@@ -222,6 +281,15 @@ __device__ __forceinline__ int s_march(const Geo& G, const BC& bc, const CUtenso
         for (int f = NF; f < NF + NO; ++f) s_tma3(s_addr(b + off(f)), maps[f], x0 + 4, y0 + 1, z, bar);
 #pragma unroll
         for (int f = NF + NO; f < NF + NO + NC; ++f) s_tma3(s_addr(b + off(f)), maps[f], x0c, y0c, (z + 1) >> 1, bar);
+        if (edge) {
+#pragma unroll
+            for (int f = 0; f < NF - 1; ++f)
+                s_row(s_addr(b + off(f) + kSBoxBytes), wrap.f[f] + x0 + G.px * wrow + (int)G.pxy * z, kSRowBytes, bar);
+            if (NC > 0)
+                s_row(s_addr(b + off(NF + NO) + kSCBoxBytes),
+                      wrap.c + x0c + wrap.cpx * (blockIdx.y == 0 ? wrap.cny : 1) + wrap.cpxy * ((z + 1) >> 1), kSCRowBytes,
+                      bar);
+        }
     };
     if (tid == 0)
         for (int q = 0; q < min(kSR, nseq); ++q) issue(q);
@@ -274,8 +342,9 @@ struct SBase {
     float cx2, cy2, cz2;
     float* xbuf;
     SZCarry zc;
-    __device__ __forceinline__ void init(const Geo& G, const float* c2) {
-        t = s_tile(G);
+    SCol col;
+    __device__ __forceinline__ void init(const Geo& G, const BC& bc, const float* c2) {
+        t = s_tile(G, bc);
         nz = G.nz;
         pxy = (int)G.pxy;
         cx2 = c2[0]; cy2 = c2[1]; cz2 = c2[2];
@@ -298,18 +367,16 @@ struct SPreBody : SBase {
     }
     __device__ __forceinline__ void plane(int k, const SSlots<3, 0, 0>& sm, const SSlots<3, 0, 0>& s0, const SSlots<3, 0, 0>& sp) {
         if (!t.in) return;
-        float zm[kVX], xc[kVX], zp[kVX], ym[kVX], yp[kVX], ax[kVX], out[kVX];
-        x1(sm, t.ly, t.qx, zm);
-        x1(s0, t.ly, t.qx, xc);
-        x1(sp, t.ly, t.qx, zp);
+        float ym[kVX], yp[kVX], ax[kVX], out[kVX];
+        col.next(k, [&](int q, float (&o)[kVX]) { x1(q == 0 ? sm : q == 1 ? s0 : sp, t.ly, t.qx, o); });
         Faces F[kVX];
         s_faces(t, k, nz, sm.f[2], s0.f[2], sp.f[2], cx2, cy2, cz2, F, zc);
         x1(s0, t.uym, t.qx, ym);
         x1(s0, t.uyp, t.qx, yp);
-        apply4(F, xc, x1s(s0, t.ly, t.uxm), x1s(s0, t.ly, t.uxp), ym, yp, zm, zp, ax);
+        apply4(F, col.c, x1s(s0, t.ly, t.uxm), x1s(s0, t.ly, t.uxp), ym, yp, col.m, col.p, ax);
         const V4 fc = sq(s0.f[0], t.ly, t.qx), dc = sq(s0.f[1], t.ly, t.qx);
 #pragma unroll
-        for (int e = 0; e < kVX; ++e) out[e] = xc[e] + omega2 * (fc.v[e] - ax[e]) * dc.v[e];
+        for (int e = 0; e < kVX; ++e) out[e] = col.c[e] + omega2 * (fc.v[e] - ax[e]) * dc.v[e];
         st4(y, t.c0 + pxy * k, out);
     }
 };
@@ -317,14 +384,14 @@ __global__ void __launch_bounds__(kSTX * kSTY, 2) k_mgs_pre(Geo G, BC bc, const 
                                                          const __grid_constant__ CUtensorMap md,
                                                          const __grid_constant__ CUtensorMap mr, const float* c2,
                                                          float* y, float omega, float omega2, int chunk,
-                                                         PCGState* st) {
+                                                         SWrap wrap, PCGState* st) {
     SPreBody b;
-    b.init(G, c2);
+    b.init(G, bc, c2);
     b.omega = omega;
     b.omega2 = omega2;
     b.y = y;
     const CUtensorMap* const maps[3] = {&mf, &md, &mr};
-    s_march<3, 0, 0>(G, bc, maps, chunk, b, st);
+    s_march<3, 0, 0>(G, bc, maps, wrap, chunk, b, st);
 }
 
 // ---- x_out = x_in + w (f - A x_in)/dg, f.x_out -> rz, beta (k_mgv_jacc on level 0, with the
@@ -336,16 +403,16 @@ struct SJaccBody : SBase {
     __device__ __forceinline__ void plane(int k, const SSlots<2, 2, 0>& sm, const SSlots<2, 2, 0>& s0,
                                           const SSlots<2, 2, 0>& sp) {
         if (!t.in) return;
-        const V4 zm = sq(sm.f[0], t.ly, t.qx), xc = sq(s0.f[0], t.ly, t.qx), zp = sq(sp.f[0], t.ly, t.qx);
+        col.next(k, [&](int q, float (&o)[kVX]) { sqa((q == 0 ? sm : q == 1 ? s0 : sp).f[0], t.ly, t.qx, o); });
         Faces F[kVX];
         s_faces(t, k, nz, sm.f[1], s0.f[1], sp.f[1], cx2, cy2, cz2, F, zc);
         const V4 y1 = sq(s0.f[0], t.uym, t.qx), y2 = sq(s0.f[0], t.uyp, t.qx);
         float ax[kVX], out[kVX];
-        apply4(F, xc.v, ss(s0.f[0], t.ly, t.uxm), ss(s0.f[0], t.ly, t.uxp), y1.v, y2.v, zm.v, zp.v, ax);
+        apply4(F, col.c, ss(s0.f[0], t.ly, t.uxm), ss(s0.f[0], t.ly, t.uxp), y1.v, y2.v, col.m, col.p, ax);
         const V4 fc = sqo(s0.f[2]), dc = sqo(s0.f[3]);
 #pragma unroll
         for (int e = 0; e < kVX; ++e) {
-            out[e] = xc.v[e] + omega * (fc.v[e] - ax[e]) * dc.v[e];
+            out[e] = col.c[e] + omega * (fc.v[e] - ax[e]) * dc.v[e];
             dot += (double)fc.v[e] * (double)out[e];
         }
         st4(xout, t.c0 + pxy * k, out);
@@ -355,16 +422,16 @@ __global__ void __launch_bounds__(kSTX * kSTY, 2) k_mgs_jacc(Geo G, BC bc, const
                                                           const __grid_constant__ CUtensorMap mr,
                                                           const __grid_constant__ CUtensorMap mf,
                                                           const __grid_constant__ CUtensorMap md, const float* c2,
-                                                          float* xout, float omega, int chunk, PCGState* st,
+                                                          float* xout, float omega, int chunk, SWrap wrap, PCGState* st,
                                                           double* partial, unsigned int* counter) {
     SJaccBody b;
-    b.init(G, c2);
+    b.init(G, bc, c2);
     b.omega = omega;
     b.xout = xout;
     b.dot = 0.;
     const CUtensorMap* const maps[4] = {&mx, &mr, &mf, &md};
     // every CTA joins the reduction, even one that gave up; none when the solve is done
-    if (s_march<2, 2, 0>(G, bc, maps, chunk, b, st) < 0) return;
+    if (s_march<2, 2, 0>(G, bc, maps, wrap, chunk, b, st) < 0) return;
     double t, u;
     if (reduce2_last(b.dot, 0.0, partial, counter, t, u) && flat_tid() == 0) {
         const double rz_old = st->rz;
@@ -393,36 +460,34 @@ struct SSpmvBody : SBase {
     }
     __device__ __forceinline__ void plane(int k, const SSlots<3, 0, 0>& sm, const SSlots<3, 0, 0>& s0, const SSlots<3, 0, 0>& sp) {
         if (!t.in) return;
-        float zm[kVX], xc[kVX], zp[kVX], ym[kVX], yp[kVX], ax[kVX];
-        pn(sm, t.ly, t.qx, zm);
-        pn(s0, t.ly, t.qx, xc);
-        pn(sp, t.ly, t.qx, zp);
+        float ym[kVX], yp[kVX], ax[kVX];
+        col.next(k, [&](int q, float (&o)[kVX]) { pn(q == 0 ? sm : q == 1 ? s0 : sp, t.ly, t.qx, o); });
         Faces F[kVX];
         s_faces(t, k, nz, sm.f[2], s0.f[2], sp.f[2], cx2, cy2, cz2, F, zc);
         pn(s0, t.uym, t.qx, ym);
         pn(s0, t.uyp, t.qx, yp);
-        apply4(F, xc, pns(s0, t.ly, t.uxm), pns(s0, t.ly, t.uxp), ym, yp, zm, zp, ax);
+        apply4(F, col.c, pns(s0, t.ly, t.uxm), pns(s0, t.ly, t.uxp), ym, yp, col.m, col.p, ax);
         const int c = t.c0 + pxy * k;
-        st4(p_new, c, xc);
+        st4(p_new, c, col.c);
         st4(qv, c, ax);
 #pragma unroll
-        for (int e = 0; e < kVX; ++e) dot += (double)xc[e] * (double)ax[e];
+        for (int e = 0; e < kVX; ++e) dot += (double)col.c[e] * (double)ax[e];
     }
 };
 __global__ void __launch_bounds__(kSTX * kSTY, 2) k_pcgs_spmvc(Geo G, BC bc, const __grid_constant__ CUtensorMap mz,
                                                             const __grid_constant__ CUtensorMap mp,
                                                             const __grid_constant__ CUtensorMap mr, const float* c2,
-                                                            float* p_new, float* qv, int chunk, PCGState* st,
+                                                            float* p_new, float* qv, int chunk, SWrap wrap, PCGState* st,
                                                             double* partial, unsigned int* counter) {
     SSpmvBody b;
-    b.init(G, c2);
+    b.init(G, bc, c2);
     b.pst = st;
     b.p_new = p_new;
     b.qv = qv;
     b.dot = 0.;
     const CUtensorMap* const maps[3] = {&mz, &mp, &mr};
     // every CTA joins the reduction, even one that gave up; none when the solve is done
-    if (s_march<3, 0, 0>(G, bc, maps, chunk, b, st) < 0) return;
+    if (s_march<3, 0, 0>(G, bc, maps, wrap, chunk, b, st) < 0) return;
     double t, u;
     if (reduce2_last(b.dot, 0.0, partial, counter, t, u) && flat_tid() == 0) {
         st->pq = t;
@@ -467,12 +532,12 @@ struct SRestrictBody : SBase {
             s1 = 0.f;
         }
         if (!t.in) return;
-        const V4 zm = sq(sm.f[0], t.ly, t.qx), xc = sq(s0s.f[0], t.ly, t.qx), zp = sq(sp.f[0], t.ly, t.qx);
+        col.next(k, [&](int q, float (&o)[kVX]) { sqa((q == 0 ? sm : q == 1 ? s0s : sp).f[0], t.ly, t.qx, o); });
         Faces F[kVX];
         s_faces(t, k, nz, sm.f[1], s0s.f[1], sp.f[1], cx2, cy2, cz2, F, zc);
         const V4 y1 = sq(s0s.f[0], t.uym, t.qx), y2 = sq(s0s.f[0], t.uyp, t.qx);
         float ax[kVX];
-        apply4(F, xc.v, ss(s0s.f[0], t.ly, t.uxm), ss(s0s.f[0], t.ly, t.uxp), y1.v, y2.v, zm.v, zp.v, ax);
+        apply4(F, col.c, ss(s0s.f[0], t.ly, t.uxm), ss(s0s.f[0], t.ly, t.uxp), y1.v, y2.v, col.m, col.p, ax);
         const V4 fv = sqo(s0s.f[2]);
         s0 += fv.v[0] - ax[0];
         s0 += fv.v[1] - ax[1];
@@ -493,13 +558,13 @@ __global__ void __launch_bounds__(kSTX * kSTY, 2) k_mgs_restrict(Geo G, Geo Gc, 
                                                               const __grid_constant__ CUtensorMap mx,
                                                               const __grid_constant__ CUtensorMap mr,
                                                               const __grid_constant__ CUtensorMap mf, const float* c2,
-                                                              float* fc, int chunk, PCGState* st) {
+                                                              float* fc, int chunk, SWrap wrap, PCGState* st) {
     SRestrictBody b;
-    b.init(G, c2);
+    b.init(G, bc, c2);
     b.Gc = Gc;
     b.fc = fc;
     const CUtensorMap* const maps[3] = {&mx, &mr, &mf};
-    s_march<2, 1, 0>(G, bc, maps, chunk, b, st);
+    s_march<2, 1, 0>(G, bc, maps, wrap, chunk, b, st);
 }
 
 // ---- x_out = x' + w (f - A x')/dg with x' = y + a P xc (k_mgv_post on level 0): slots y,
@@ -512,7 +577,7 @@ struct SPostBody : SBase {
     // x' of the quad at tile row ly from the y slot and the coarse slot of its plane
     __device__ __forceinline__ void xq(const float* ys, const float* cs, int ly, float (&o)[kVX]) const {
         const V4 yv = sq(ys, ly, t.qx);
-        const int cx = (t.qx >> 1) + 2, cy = (ly + 1) >> 1;
+        const int cx = (t.qx >> 1) + 2, cy = (ly == kSBoxY) ? kSCBoxY : (ly + 1) >> 1;   // wrapped row: its parent's
         const float p0 = alpha * ssc(cs, cy, cx), p1 = alpha * ssc(cs, cy, cx + 1);
         o[0] = yv.v[0] + p0; o[1] = yv.v[1] + p0; o[2] = yv.v[2] + p1; o[3] = yv.v[3] + p1;
     }
@@ -522,18 +587,19 @@ struct SPostBody : SBase {
     __device__ __forceinline__ void plane(int k, const SSlots<2, 2, 1>& sm, const SSlots<2, 2, 1>& s0,
                                           const SSlots<2, 2, 1>& sp) {
         if (!t.in) return;
-        float zm[kVX], xc[kVX], zp[kVX], ym[kVX], yp[kVX], ax[kVX], out[kVX];
-        xq(sm.f[0], sm.f[4], t.ly, zm);
-        xq(s0.f[0], s0.f[4], t.ly, xc);
-        xq(sp.f[0], sp.f[4], t.ly, zp);
+        float ym[kVX], yp[kVX], ax[kVX], out[kVX];
+        col.next(k, [&](int q, float (&o)[kVX]) {
+            const SSlots<2, 2, 1>& s = q == 0 ? sm : q == 1 ? s0 : sp;
+            xq(s.f[0], s.f[4], t.ly, o);
+        });
         Faces F[kVX];
         s_faces(t, k, nz, sm.f[1], s0.f[1], sp.f[1], cx2, cy2, cz2, F, zc);
         xq(s0.f[0], s0.f[4], t.uym, ym);
         xq(s0.f[0], s0.f[4], t.uyp, yp);
-        apply4(F, xc, xs(s0.f[0], s0.f[4], t.ly, t.uxm), xs(s0.f[0], s0.f[4], t.ly, t.uxp), ym, yp, zm, zp, ax);
+        apply4(F, col.c, xs(s0.f[0], s0.f[4], t.ly, t.uxm), xs(s0.f[0], s0.f[4], t.ly, t.uxp), ym, yp, col.m, col.p, ax);
         const V4 fc = sqo(s0.f[2]), dc = sqo(s0.f[3]);
 #pragma unroll
-        for (int e = 0; e < kVX; ++e) out[e] = xc[e] + omega * (fc.v[e] - ax[e]) * dc.v[e];
+        for (int e = 0; e < kVX; ++e) out[e] = col.c[e] + omega * (fc.v[e] - ax[e]) * dc.v[e];
         st4(xout, t.c0 + pxy * k, out);
     }
 };
@@ -543,14 +609,14 @@ __global__ void __launch_bounds__(kSTX * kSTY, 2) k_mgs_post(Geo G, BC bc, const
                                                           const __grid_constant__ CUtensorMap md,
                                                           const __grid_constant__ CUtensorMap mc, const float* c2,
                                                           float* xout, float omega, float alpha, int chunk,
-                                                          PCGState* st) {
+                                                          SWrap wrap, PCGState* st) {
     SPostBody b;
-    b.init(G, c2);
+    b.init(G, bc, c2);
     b.omega = omega;
     b.alpha = alpha;
     b.xout = xout;
     const CUtensorMap* const maps[5] = {&my, &mr, &mf, &md, &mc};
-    s_march<2, 2, 1>(G, bc, maps, chunk, b, st);
+    s_march<2, 2, 1>(G, bc, maps, wrap, chunk, b, st);
 }
 static inline dim3 sgrid(const Geo& g, int chunk) {
     return dim3((g.nx + kSTileX - 1) / kSTileX, (g.ny + kSTY - 1) / kSTY, (g.nz + chunk - 1) / chunk);

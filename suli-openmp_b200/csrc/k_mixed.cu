@@ -766,9 +766,10 @@ static const CUtensorMap& own_map(const suli_ctx* c, const float* a) {
 }
 
 // Decide once per context whether level 0 runs the streaming kernels: vectorised kernels on a
-// multigrid hierarchy (mg_kernels 0), nx a multiple of 16, no periodic x or y axis, a tensor map
-// for every level-0 array they read, and two CTAs' shared memory an SM.  SULI_NO_STREAM=1
-// keeps the vectorised level-0 kernels; SULI_STREAM_CHUNK sets the planes a CTA computes.
+// multigrid hierarchy (mg_kernels 0), nx a multiple of 16, no periodic x axis, more than 8 rows on a
+// periodic y axis (no tile then holds both its ends), a tensor map for every level-0 array they
+// read, and two CTAs' shared memory an SM.  SULI_NO_STREAM=1 keeps the vectorised level-0
+// kernels; SULI_STREAM_CHUNK sets the planes a CTA computes.
 int stream_ready(suli_ctx* c) {
     c->stream_ok = false;
     c->stream_post_ok = false;
@@ -777,7 +778,7 @@ int stream_ready(suli_ctx* c) {
         if (std::strcmp(ev, "1") == 0) return SULI_OK;
     if (c->mg.size() < 2 || c->P.mg_kernels != 0) return SULI_OK;
     const Geo& g = c->mg[0].g;
-    if (g.nx % 16 != 0 || g.px < g.nx + 16 || c->bc.perx || c->bc.pery) return SULI_OK;
+    if (g.nx % 16 != 0 || g.px < g.nx + 16 || c->bc.perx || (c->bc.pery && g.ny <= kSTY)) return SULI_OK;
     const MGLevel& M0 = c->mg[0];
     const float* arrays[] = {c->pc_r, c->pc_r2, M0.x, M0.y, c->pc_pa, c->pc_pb, M0.idg, M0.rho};
     for (const float* a : arrays)
@@ -817,6 +818,10 @@ int stream_ready(suli_ctx* c) {
     return SULI_OK;
 }
 
+static SWrap stream_wrap(const suli_ctx* c, const float* f0, const float* f1 = nullptr) {
+    const Geo& g = c->mg[1].g;
+    return SWrap{{f0, f1}, mg_corr(c, 1), g.px, (int)g.pxy, g.ny};
+}
 template <typename... KArgs, typename... Args>
 static void stream_launch(suli_ctx* c, void (*kernel)(KArgs...), size_t smem, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -834,13 +839,13 @@ static void stream_launch(suli_ctx* c, void (*kernel)(KArgs...), size_t smem, Ar
 static void launch_stream_pre(suli_ctx* c, const float* f, float om, float om2) {
     const MGLevel& M = c->mg[0];
     stream_launch(c, k_mgs_pre, stream_smem_bytes(3), M.g, c->bc, plane_map(c, f), plane_map(c, M.idg),
-                  plane_map(c, M.rho), (const float*)M.c2, M.y, om, om2, c->stream_chunk, c->pcg);
+                  plane_map(c, M.rho), (const float*)M.c2, M.y, om, om2, c->stream_chunk, stream_wrap(c, f, M.idg), c->pcg);
 }
 static void launch_stream_jacc(suli_ctx* c, const float* f, float om) {
     const MGLevel& M = c->mg[0];
     stream_launch(c, k_mgs_jacc, stream_smem_bytes(2, 2), M.g, c->bc, plane_map(c, M.x), plane_map(c, M.rho),
-                  own_map(c, f), own_map(c, M.idg), (const float*)M.c2, M.y, om, c->stream_chunk, c->pcg,
-                  c->red_partial, c->red_counter);
+                  own_map(c, f), own_map(c, M.idg), (const float*)M.c2, M.y, om, c->stream_chunk,
+                  stream_wrap(c, M.x), c->pcg, c->red_partial, c->red_counter);
 }
 // the restriction's chunk is even (a coarse plane's two fine planes in one CTA)
 static void launch_stream_restrict(suli_ctx* c, const float* f) {
@@ -858,19 +863,19 @@ static void launch_stream_restrict(suli_ctx* c, const float* f) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k_mgs_restrict, M.g, C.g, c->bc, plane_map(c, M.y), plane_map(c, M.rho), own_map(c, f),
-                       (const float*)M.c2, C.f, ch, c->pcg);
+                       (const float*)M.c2, C.f, ch, stream_wrap(c, M.y), c->pcg);
 }
 static void launch_stream_post(suli_ctx* c, const float* f, float om2, float alpha) {
     const MGLevel& M = c->mg[0];
     stream_launch(c, k_mgs_post, stream_smem_bytes(2, 2, 1), M.g, c->bc, plane_map(c, M.y), plane_map(c, M.rho),
                   own_map(c, f), own_map(c, M.idg), c->smap_c, (const float*)M.c2, M.x, om2, alpha, c->stream_chunk,
-                  c->pcg);
+                  stream_wrap(c, M.y), c->pcg);
 }
 static void launch_stream_spmvc(suli_ctx* c, const float* p_old, float* p_new) {
     const MGLevel& M = c->mg[0];
     stream_launch(c, k_pcgs_spmvc, stream_smem_bytes(3), M.g, c->bc, plane_map(c, M.y), plane_map(c, p_old),
-                  plane_map(c, M.rho), (const float*)M.c2, p_new, c->pc_q, c->stream_chunk, c->pcg, c->red_partial,
-                  c->red_counter);
+                  plane_map(c, M.rho), (const float*)M.c2, p_new, c->pc_q, c->stream_chunk, stream_wrap(c, M.y, p_old),
+                  c->pcg, c->red_partial, c->red_counter);
 }
 
 // pre-smoothing (weights om, then om2) and restriction of level l (level 0 forms its faces from

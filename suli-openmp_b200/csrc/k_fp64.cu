@@ -482,8 +482,12 @@ __device__ __forceinline__ R classico_hi(const double* __restrict__ a, int c, co
 }
 
 // DER: classico's scheme (adv_type = 1); ADV: 2 rotacional, 3 antissim (advect.cuh; der = 1)
+// About 1500 instructions and 110 loads a face (measured: half of issue, 22 % of the FP64 pipe, a third
+// of L1; 60 % of the stalls wait for loads), so blocks an SM against registers decide: FP32 five
+// blocks (6 at the compiler's own 40 registers: 0.75 -> 0.68 ms a 256x128x128 step; 4: 0.70), FP64 four
+// (3 at 78: 181 -> 162 us at 150x133x90 with der = 2; 5: 173).
 template <typename R, int DER, int ADV>
-__global__ void __launch_bounds__(256) k_convdiff(Geo G, CDConst C, CDFields F) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G, CDConst C, CDFields F) {
     pdl_wait();
     const Thread3 t = tid3(1, 1, 1);
     const int i = t.i, j = t.j, k = t.k, nx = G.nx, ny = G.ny, nz = G.nz;

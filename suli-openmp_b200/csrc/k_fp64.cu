@@ -187,14 +187,26 @@ __global__ void __launch_bounds__(256) k_ls_advect(Geo G, LsConst L, const doubl
     const Thread3 t = tid3(1, 1, 1);
     if (t.i > G.nx || t.j > G.ny || t.k > G.nz) return;
     const int i = t.i, j = t.j, k = t.k;
-    const Weno3<R> W = der_weno_at<R>(G, cur, i, j, k, L.ihx, L.ihy, L.ihz, L.rcp<R>(0), L.rcp<R>(1), L.rcp<R>(2));
     const R ua = (RLD(u, i, j, k) + RLD(u, i + 1, j, k)) * R(0.5);
     const R va = (RLD(v, i, j, k) + RLD(v, i, j + 1, k)) * R(0.5);
     const R wa = (RLD(w, i, j, k) + RLD(w, i, j, k + 1)) * R(0.5);
     const R apos = pmax(ua, R(0)), aneg = pmin(ua, R(0));
     const R bpos = pmax(va, R(0)), bneg = pmin(va, R(0));
     const R cpos = pmax(wa, R(0)), cneg = pmin(wa, R(0));
-    const R sy7 = -(apos * W.dnx + aneg * W.dpx + bpos * W.dny + bneg * W.dpy + cpos * W.dnz + cneg * W.dpz);
+    R sy7;
+    if constexpr (sizeof(R) == 8) {
+        R P[7];
+        pencil7<R>([&](int q) { return R(FIDX(cur, q, j, k)); }, i, G.nx, L.ihx, P);
+        R adv = weno_upwind(P, L.rcp<R>(0), apos + aneg);
+        pencil7<R>([&](int q) { return R(FIDX(cur, i, q, k)); }, j, G.ny, L.ihy, P);
+        adv += weno_upwind(P, L.rcp<R>(1), bpos + bneg);
+        pencil7<R>([&](int q) { return R(FIDX(cur, i, j, q)); }, k, G.nz, L.ihz, P);
+        adv += weno_upwind(P, L.rcp<R>(2), cpos + cneg);
+        sy7 = -adv;
+    } else {   // memory- and issue-bound alike: the upwind side alone saved little and rounds differently
+        const Weno3<R> W = der_weno_at<R>(G, cur, i, j, k, L.ihx, L.ihy, L.ihz, L.rcp<R>(0), L.rcp<R>(1), L.rcp<R>(2));
+        sy7 = -(apos * W.dnx + aneg * W.dpx + bpos * W.dny + bneg * W.dpy + cpos * W.dnz + cneg * W.dpz);
+    }
     const long long c = G.idx(i, j, k);
     const double p0 = phi0[c];
     const double gxv = cur[c];

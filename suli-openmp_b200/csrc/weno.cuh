@@ -8,6 +8,12 @@
 // 2 the 1/11 "zero derivative" rows at both ends.  The arithmetic is the reference's with its
 // divisions rearranged: the reciprocal of h formed once on the host, and in FP64 the nonlinear
 // weights w_k/q_k^2 / sum_m w_m/q_m^2 formed over a common denominator (one division per side).
+//
+// The FP64 kernels are bound by the FP64 pipe (70 % busy at 150 instructions a one-sided pair), so
+// FP64 forms the pair from the differences E of the divided differences D: the second differences
+// and smoothness terms of the stencils that both sides share once, the smoothness indicators up to
+// a common factor, and each candidate as the centre D plus a combination of E, which needs the
+// weights' ratios only (about 100 instructions).  FP32 keeps the reference's expressions.
 #pragma once
 
 namespace suli {
@@ -53,25 +59,49 @@ __device__ __forceinline__ void pencil7(F at, int i, int n, int ihs, T P[7]) {
     }
 }
 
-// omega_k = (w_k/q_k^2) / sum_m (w_m/q_m^2), q_k = eps + is_k.  FP64: over the common
-// denominator q_1^2 q_2^2 q_3^2 (q >= eps = 1e-8, so the products stay far inside the FP64
-// range); FP32 (the mixed path's arithmetic, where that product can underflow): the three
-// quotients and one reciprocal of their sum, each with the hardware reciprocal (__fdividef, 2
-// ulp; q^2 stays far below the 2^126 where it would flush), since IEEE FP32 divisions were a
-// third of the WENO kernels' instructions.
-template <typename T>
-__device__ __forceinline__ void nonlinear_weights(T is1, T is2, T is3, T eps, T w1, T w2, T w3, T& o1, T& o2,
-                                                  T& o3) {
-    const T a = (eps + is1) * (eps + is1), b = (eps + is2) * (eps + is2), c = (eps + is3) * (eps + is3);
-    if constexpr (sizeof(T) == 8) {
-        const T n1 = w1 * (b * c), n2 = w2 * (a * c), n3 = w3 * (a * b);
-        const T inv = T(1) / (n1 + n2 + n3);
-        o1 = n1 * inv; o2 = n2 * inv; o3 = n3 * inv;
-    } else {
-        const T al1 = __fdividef(w1, a), al2 = __fdividef(w2, b), al3 = __fdividef(w3, c);
-        const T inv = __fdividef(T(1), al1 + al2 + al3);
-        o1 = al1 * inv; o2 = al2 * inv; o3 = al3 * inv;
-    }
+// FP32 (the mixed path's arithmetic), the reference's expressions: the derivative at the middle of
+// the five divided differences v0..v4 (left-biased; reversed, right-biased).  The weights
+// omega_k = (w_k/q_k^2) / sum_m (w_m/q_m^2), q_k = eps + is_k, as three quotients and one
+// reciprocal of their sum, each with the hardware reciprocal (__fdividef, 2 ulp; q^2 stays far below
+// the 2^126 where it would flush, and a common denominator could underflow), since IEEE FP32
+// divisions were a third of the WENO kernels' instructions.
+__device__ __forceinline__ float weno_side(float v0, float v1, float v2, float v3, float v4) {
+    using T = float;
+    const T aux1 = T(13. / 12.), aux2 = T(1. / 4.), aux3 = T(1. / 6.), eps = T(0.00000001);
+    const T w1 = T(0.1), w2 = T(0.6), w3 = T(0.3);
+    T a, b;
+    a = v0 - 2 * v1 + v2; b = v0 - 4 * v1 + 3 * v2;
+    const T is1 = aux1 * a * a + aux2 * b * b;
+    a = v1 - 2 * v2 + v3; b = v1 - v3;
+    const T is2 = aux1 * a * a + aux2 * b * b;
+    a = v2 - 2 * v3 + v4; b = 3 * v2 - 4 * v3 + v4;
+    const T is3 = aux1 * a * a + aux2 * b * b;
+    const T q1 = (eps + is1) * (eps + is1), q2 = (eps + is2) * (eps + is2), q3 = (eps + is3) * (eps + is3);
+    const T al1 = __fdividef(w1, q1), al2 = __fdividef(w2, q2), al3 = __fdividef(w3, q3);
+    const T inv = __fdividef(T(1), al1 + al2 + al3);
+    const T o1 = al1 * inv, o2 = al2 * inv, o3 = al3 * inv;
+    return aux3 * (o1 * (2 * v0 - 7 * v1 + 11 * v2) + o2 * (-v1 + 5 * v2 + 2 * v3) + o3 * (2 * v2 + 5 * v3 - v4));
+}
+
+// FP64: what the weighted candidates add to v2, from the differences e_m = v_{m+1} - v_m and
+// x_k = 12/13 eps + (second difference of stencil k)^2.  q_k = x_k + 3/13 b_k^2 is 12/13 (eps + is_k);
+// the factor and the weights' (0.1, 0.6, 0.3) = (1, 6, 3)/10 cancel in the ratios, formed over the
+// common denominator q_1^2 q_2^2 q_3^2 (q >= 9e-9, so the products stay far inside the FP64 range).
+// Odd in e: the reversed differences, which change sign, give the right-biased side's with -.
+constexpr double kWenoEps = 12. / 13. * 0.00000001, kWenoB = 3. / 13.;
+__device__ __forceinline__ double weno_blend(double e0, double e1, double e2, double e3, double x1, double x2,
+                                             double x3) {
+    const double b1 = 3. * e1 - e0, b2 = e1 + e2, b3 = e3 - 3. * e2;
+    const double q1 = x1 + (kWenoB * b1) * b1, q2 = x2 + (kWenoB * b2) * b2, q3 = x3 + (kWenoB * b3) * b3;
+    const double a = q1 * q1, b = q2 * q2, c = q3 * q3;
+    const double n1 = b * c, n2 = 6. * (a * c), n3 = 3. * (a * b);
+    const double num = n1 * (5. * e1 - 2. * e0) + n2 * (e1 + 2. * e2) + n3 * (4. * e2 - e3);
+    return num * (1. / (6. * (n1 + n2 + n3)));
+}
+__device__ __forceinline__ double weno_side(double v0, double v1, double v2, double v3, double v4) {
+    const double e0 = v1 - v0, e1 = v2 - v1, e2 = v3 - v2, e3 = v4 - v3;
+    const double s1 = e1 - e0, s2 = e2 - e1, s3 = e3 - e2;
+    return v2 + weno_blend(e0, e1, e2, e3, kWenoEps + s1 * s1, kWenoEps + s2 * s2, kWenoEps + s3 * s3);
 }
 
 // One-sided derivatives from the seven values P[0..6] = phi(i-3..i+3) and ih = 1/h (formed
@@ -83,38 +113,30 @@ __device__ __forceinline__ void weno_pair(const T P[7], T ih, T& dp, T& dn) {
     T D[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) D[m] = (P[m + 1] - P[m]) * ih;
-    const T aux1 = T(13. / 12.), aux2 = T(1. / 4.), aux3 = T(1. / 6.), aux6 = T(0.00000001);
-    const T w1 = T(0.1), w2 = T(0.6), w3 = T(0.3);
-    // right-biased: up(i)=D5, up(i-1)=D4, up(i-2)=D3, up(i-3)=D2, up(i-4)=D1
-    {
-        const T u0 = D[5], u1 = D[4], u2 = D[3], u3 = D[2], u4 = D[1];
-        T a, b;
-        a = u0 - 2 * u1 + u2; b = u0 - 4 * u1 + 3 * u2;
-        const T is1 = aux1 * a * a + aux2 * b * b;
-        a = u1 - 2 * u2 + u3; b = u1 - u3;
-        const T is2 = aux1 * a * a + aux2 * b * b;
-        a = u2 - 2 * u3 + u4; b = 3 * u2 - 4 * u3 + u4;
-        const T is3 = aux1 * a * a + aux2 * b * b;
-        T o1, o2, o3;
-        nonlinear_weights(is1, is2, is3, aux6, w1, w2, w3, o1, o2, o3);
-        dp = aux3 * (o1 * (2 * u0 - 7 * u1 + 11 * u2) + o2 * (-u1 + 5 * u2 + 2 * u3) +
-                     o3 * (2 * u2 + 5 * u3 - u4));
+    if constexpr (sizeof(T) == 8) {
+        const T e0 = D[1] - D[0], e1 = D[2] - D[1], e2 = D[3] - D[2], e3 = D[4] - D[3], e4 = D[5] - D[4];
+        const T s1 = e1 - e0, s2 = e2 - e1, s3 = e3 - e2, s4 = e4 - e3;
+        const T x1 = kWenoEps + s1 * s1, x2 = kWenoEps + s2 * s2, x3 = kWenoEps + s3 * s3, x4 = kWenoEps + s4 * s4;
+        dn = D[2] + weno_blend(e0, e1, e2, e3, x1, x2, x3);
+        dp = D[3] - weno_blend(e4, e3, e2, e1, x4, x3, x2);
+    } else {
+        dp = weno_side(D[5], D[4], D[3], D[2], D[1]);
+        dn = weno_side(D[0], D[1], D[2], D[3], D[4]);
     }
-    // left-biased: un(i)=D0, un(i+1)=D1, un(i+2)=D2, un(i+3)=D3, un(i+4)=D4
-    {
-        const T v0 = D[0], v1 = D[1], v2 = D[2], v3 = D[3], v4 = D[4];
-        T a, b;
-        a = v0 - 2 * v1 + v2; b = v0 - 4 * v1 + 3 * v2;
-        const T is1 = aux1 * a * a + aux2 * b * b;
-        a = v1 - 2 * v2 + v3; b = v1 - v3;
-        const T is2 = aux1 * a * a + aux2 * b * b;
-        a = v2 - 2 * v3 + v4; b = 3 * v2 - 4 * v3 + v4;
-        const T is3 = aux1 * a * a + aux2 * b * b;
-        T o1, o2, o3;
-        nonlinear_weights(is1, is2, is3, aux6, w1, w2, w3, o1, o2, o3);
-        dn = aux3 * (o1 * (2 * v0 - 7 * v1 + 11 * v2) + o2 * (-v1 + 5 * v2 + 2 * v3) +
-                     o3 * (2 * v2 + 5 * v3 - v4));
-    }
+}
+
+// FP64: max(vel, 0) phi_x^- + min(vel, 0) phi_x^+ with the upwind side alone formed (the other has
+// the factor 0; its outermost value still enters with that factor, so that one that is not finite
+// is carried on).  A transport stage at 191x97x113: 79 -> 58 us; the reinitialisation's nine
+// kernels, which need both sides: 612 -> 516 us.
+__device__ __forceinline__ double weno_upwind(const double P[7], double ih, double vel) {
+    const bool left = vel > 0.;
+    double v[6];   // the values from the outermost upwind one on
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v[m] = left ? P[m] : P[6 - m];
+    const double h = left ? ih : -ih;
+    const double d = weno_side((v[1] - v[0]) * h, (v[2] - v[1]) * h, (v[3] - v[2]) * h, (v[4] - v[3]) * h, (v[5] - v[4]) * h);
+    return vel * (d + 0. * (left ? P[6] : P[0]));
 }
 
 }  // namespace suli

@@ -989,44 +989,44 @@ __global__ void k_bc_nz(Geo G, BC bc, BCArgs A) {
     if (bc.zf == 3) FIDX(w, i, j, nz1) = A.pl.bzzf[i + lv * j];
 }
 
-// outflow_fix = 1 (an extension, after contorno(2) with ccxf = 4): one block sums the net
-// volume flux through the boundary planes (the sum of graddin's right-hand side over the cells,
-// telescoped), then shifts the outflow faces u(nx+1, j, k) above the obstacle mask ku(nx+1, j)
-// by one uniform value so that the net flux vanishes.  Fixed-order tree sums (deterministic).
-constexpr int kFixThreads = 1024;
-__global__ void __launch_bounds__(kFixThreads) k_outflow_fix(Geo G, BCArgs A, const int* __restrict__ ku, double dx,
-                                                            double dy, double dz) {
+// outflow_fix = 1 (an extension, after contorno(2) with ccxf = 4): sum the net volume flux through
+// the boundary planes (the sum of graddin's right-hand side over the cells, telescoped), then shift
+// the outflow faces u(nx+1, j, k) above the obstacle mask ku(nx+1, j) by one uniform value so that
+// the net flux vanishes.  Fixed-order tree sums (deterministic).  Bound by the latency of the strided
+// loads, so the planes are spread over the SMs: one block for everything took 339 us at 512x256x256,
+// the two kernels about 35.
+constexpr int kFixBlocks = 128;
+__global__ void __launch_bounds__(256) k_outflow_sum(Geo G, BCArgs A, const int* __restrict__ ku, double dx, double dy,
+                                                    double dz, double* partial, unsigned int* counter, double* delta) {
     pdl_wait();
-    __shared__ double s_delta;
-    const int nx = G.nx, ny = G.ny, nz = G.nz, tid = threadIdx.x;
-    double fx = 0., fy = 0., fz = 0., open = 0.;
-    for (int q = tid; q < ny * nz; q += kFixThreads) {
+    const int nx = G.nx, ny = G.ny, nz = G.nz, first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    double s[4] = {0., 0., 0., 0.};   // x, y and z fluxes, open outflow faces
+    for (int q = first; q < ny * nz; q += step) {
         const int j = 1 + q % ny, k = 1 + q / ny;
-        fx += FIDX(A.u, nx + 1, j, k) - FIDX(A.u, 1, j, k);
-        open += (!ku || k > ku[(nx + 1) + (nx + 3) * j]) ? 1. : 0.;
+        s[0] += FIDX(A.u, nx + 1, j, k) - FIDX(A.u, 1, j, k);
+        s[3] += (!ku || k > ku[(nx + 1) + (nx + 3) * j]) ? 1. : 0.;
     }
-    for (int q = tid; q < nx * nz; q += kFixThreads) {
+    for (int q = first; q < nx * nz; q += step) {
         const int i = 1 + q % nx, k = 1 + q / nx;
-        fy += FIDX(A.v, i, ny + 1, k) - FIDX(A.v, i, 1, k);
+        s[1] += FIDX(A.v, i, ny + 1, k) - FIDX(A.v, i, 1, k);
     }
-    for (int q = tid; q < nx * ny; q += kFixThreads) {
+    for (int q = first; q < nx * ny; q += step) {
         const int i = 1 + q % nx, j = 1 + q / nx;
-        fz += FIDX(A.w, i, j, nz + 1) - FIDX(A.w, i, j, 1);
+        s[2] += FIDX(A.w, i, j, nz + 1) - FIDX(A.w, i, j, 1);
     }
-    fx = block_sum(fx);
-    fy = block_sum(fy);
-    fz = block_sum(fz);
-    open = block_sum(open);
-    if (tid == 0) {
-        const double net = fx * (dy * dz) + fy * (dx * dz) + fz * (dx * dy);
-        s_delta = (open > 0.) ? -net / (open * (dy * dz)) : 0.;
+    double t[4], m;
+    if (reduce_sums_max_last<4>(s, 0., partial, counter, t, m) && flat_tid() == 0) {
+        const double net = t[0] * (dy * dz) + t[1] * (dx * dz) + t[2] * (dx * dy);
+        *delta = (t[3] > 0.) ? -net / (t[3] * (dy * dz)) : 0.;
     }
-    __syncthreads();
-    const double delta = s_delta;
-    for (int q = tid; q < ny * nz; q += kFixThreads) {
-        const int j = 1 + q % ny, k = 1 + q / ny;
-        if (!ku || k > ku[(nx + 1) + (nx + 3) * j]) FIDX(A.u, nx + 1, j, k) += delta;
-    }
+}
+__global__ void __launch_bounds__(256) k_outflow_shift(Geo G, double* u, const int* __restrict__ ku,
+                                                      const double* __restrict__ delta) {
+    pdl_wait();
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, nx = G.nx, ny = G.ny;
+    if (q >= ny * G.nz) return;
+    const int j = 1 + q % ny, k = 1 + q / ny;
+    if (!ku || k > ku[(nx + 1) + (nx + 3) * j]) FIDX(u, nx + 1, j, k) += *delta;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1731,7 +1731,7 @@ void launch_contorno(suli_ctx* c, int nlock) {
     A.nlock = nlock;
     A.obst = obst ? 1 : 0;
     const bool capy = !obst && (c->bc.y0 == 2 || c->bc.yf == 2);
-    ProfScope ps(c, SULI_K_CONTORNO, (nlock == 2 ? 7 + (c->P.outflow_fix == 1 && c->bc.xf == 4 ? 1 : 0) : 4) +
+    ProfScope ps(c, SULI_K_CONTORNO, (nlock == 2 ? 7 + (c->P.outflow_fix == 1 && c->bc.xf == 4 ? 2 : 0) : 4) +
                                          (capy || obst ? 1 : 0));
     {
         const long long ng = 2LL * (G.ny + 2) * (G.nz + 2) + 2LL * G.nx * (G.nz + 2) + 2LL * G.nx * G.ny;
@@ -1749,9 +1749,14 @@ void launch_contorno(suli_ctx* c, int nlock) {
         step_launch(c, k_bc_ny, grid3(G.nx + 2, G.nz + 2, 1, b2), b2, G, c->bc, A);
         step_launch(c, k_bc_nx, grid3(G.ny + 3, G.nz + 3, 1, b2), b2, G, c->bc, A);
         step_launch(c, k_bc_nz, grid3(G.nx + 2, G.ny + 2, 1, b2), b2, G, c->bc, A);
-        if (c->P.outflow_fix == 1 && c->bc.xf == 4)
-            step_launch(c, k_outflow_fix, 1, kFixThreads, G, A, obst ? c->obst_ku : nullptr, c->P.dx, c->P.dy,
-                                                            c->P.dz);
+        if (c->P.outflow_fix == 1 && c->bc.xf == 4) {
+            const int* ku = obst ? c->obst_ku : nullptr;
+            double* delta = c->red_out + 8;
+            const int plane = std::max(G.ny * G.nz, std::max(G.nx * G.nz, G.nx * G.ny));
+            step_launch(c, k_outflow_sum, std::min(kFixBlocks, (plane + 255) / 256), 256, G, A, ku, c->P.dx, c->P.dy,
+                        c->P.dz, c->red_partial, c->red_counter, delta);
+            step_launch(c, k_outflow_shift, (G.ny * G.nz + 255) / 256, 256, G, A.u, ku, delta);
+        }
     }
 }
 static CGConst cg_const(const suli_ctx* c) {

@@ -256,7 +256,8 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
         if ((e = cudaMalloc(&c->f[f], n * sizeof(double))) != cudaSuccess) return bail(e, "plane");
         if ((e = cudaMemsetAsync(c->f[f], 0, n * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
     }
-    const long long nb = (long long)((p->nx + 1 + 31) / 32) * ((p->ny + 1 + 7) / 8) * (p->nz + 1) + 64;
+    // block partials: up to four a block of the face grids; five for at most 128 blocks (outflow_fix)
+    const long long nb = (long long)((p->nx + 1 + 31) / 32) * ((p->ny + 1 + 7) / 8) * (p->nz + 1) + 256;
     if ((e = cudaMalloc(&c->red_partial, (size_t)nb * 4 * sizeof(double))) != cudaSuccess) return bail(e, "partial");
     if ((e = cudaMalloc(&c->red_counter, 64 * sizeof(unsigned int))) != cudaSuccess) return bail(e, "counter");
     if ((e = cudaMemsetAsync(c->red_counter, 0, 64 * sizeof(unsigned int), c->stream)) != cudaSuccess) return bail(e, "memset");

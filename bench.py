@@ -266,7 +266,7 @@ CLASS_PASSES = {
     "visco": 5,        # nut: u, v, w, rho in, nut out; faces: nut, ls_nu in, xnut..znut out
     "convdiff": 20,    # u, v, w, rho, hsx..z, kurv, nut, xnut..znut in, Fu..Fw out; prd0 = prd1 copy
     "tempo": 15,       # per component: velocity, F in; velocity and two stage stores out
-    "posdin": 10,      # u, v, w, prd1, rho in; u, v, w out; the prd = prd1 copy timed with it
+    "posdin": 9,       # u, v, w, prd1, rho in; u, v, w, prd out
     "est": 3,          # u, v, w in
 }
 
@@ -501,7 +501,9 @@ def cg_roofline(p, prof):
     N = p.nx * p.ny * p.nz
     faces = (p.nx + 1) * p.ny * p.nz + p.nx * (p.ny + 1) * p.nz + p.nx * p.ny * (p.nz + 1)
     bytes_spmv = 8 * (4 * N + faces)
-    bytes_upd = 8 * 5 * N   # e, r, q in, e, r out: the e update's p is read by the first pass
+    # r, q in, r out; every other iteration e in and out and the older direction (the newer one is
+    # read by the first pass)
+    bytes_upd = int(8 * 4.5 * N)
     n_it = max(prof["cg_iterations"], 1)
     t_it = (prof["cg_spmv"]["ms"] + prof["cg_update"]["ms"]) / n_it / 1e3
     share = launch_share("launches_sloshing_256x128x128_fp64", "k_cg_spmv2", ("k_cg_spmv2", "k_cg_update"))

@@ -259,11 +259,13 @@ __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, doubl
 }
 
 // Larger grids: the iteration's two passes over units dealt to the threads in turn (a unit is a
-// pair of x cells, 16-byte loads, and a column of KZ planes).  The first pass also applies the
-// previous iteration's e -= alpha p, whose p it reads anyway, so the second only forms r; it
-// takes the units in reverse order, newest in the L2 first.  Iteration n (from 1) writes its
-// direction into pa for odd n, pb for even n.  Bound by the loads a thread's 64 registers keep in
-// flight: 12 passes in 83.4 us at 256x128x128, 4.8 TB/s (the two kernels' 13 passes: 103.4 us).
+// pair of x cells, 16-byte loads, and a column of KZ planes).  Every other iteration the first pass
+// also applies the last two iterations' e -= alpha p (it reads the newer p anyway, and the older
+// where it writes its own), so the second only forms r; it takes the units in reverse order,
+// newest in the L2 first.  Iteration n (from 1) writes its direction into pa for odd n, pb for even
+// n.  Bound by the loads a thread's 64 registers keep in flight: 11.5 passes in 80 us at
+// 256x128x128, 4.8 TB/s (e updated in every iteration, 12 passes: 83.4; the two kernels' 13 passes:
+// 103.4).
 // Measured there: 512 threads of the same 87.7-97, 4 planes a unit 96, 8 planes 105, 1 plane 89.
 template <int KZ, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, double* pa, double* pb, double* q, double* e,
@@ -287,7 +289,8 @@ __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, doubl
         if (two) __stcg(reinterpret_cast<double2*>(a), v);
         else __stcg(a, v.x);
     };
-    bool pending = false;   // e lacks the previous iteration's update
+    int pending = 0;          // iterations whose update e lacks, the older with step alpha_old
+    double alpha_old = 0.;
     while (!s.done && !S.failed) {
         double* pn_ = (s.iters & 1) ? pb : pa;                                   // iteration s.iters + 1
         const double* po = (s.iters == 0) ? r : ((s.iters & 1) ? pa : pb);
@@ -325,20 +328,20 @@ __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, doubl
                                   pzp.x * azp.x - pzm.x * azc.x;
                 const double q1 = pc.y - pxp * ax2 - pc.x * axc.y - pyp.y * ayp.y - pym.y * ayc.y - pzp.y * azp.y -
                                   pzm.y * azc.y;
+                if (pending == 2) {   // the older direction is the one this iteration's replaces
+                    double2 ev = lg2(e + c);
+                    const double2 pw = lg2(pn_ + c), pv = lg2(po + c);
+                    ev.x = (ev.x - alpha_old * pw.x) - alpha0 * pv.x;
+                    ev.y = (ev.y - alpha_old * pw.y) - alpha0 * pv.y;
+                    put(e + c, ev, two);
+                }
                 put(q + c, make_double2(q0, q1), two);
                 put(pn_ + c, pc, two);
                 dot += pc.x * q0;
                 if (two) dot += pc.y * q1;
-                if (pending) {
-                    double2 ev = lg2(e + c);
-                    const double2 pv = lg2(po + c);
-                    ev.x = ev.x - alpha0 * pv.x;
-                    ev.y = ev.y - alpha0 * pv.y;
-                    put(e + c, ev, two);
-                }
             }
         }
-        pending = false;
+        if (pending == 2) pending = 0;
         s.dot(coop_sum(S, dot));
         if (s.done || S.failed) break;
         const double alpha = s.alpha;
@@ -361,19 +364,26 @@ __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, doubl
                 if (two) rr += rv.y * rv.y;
             }
         }
-        pending = true;
+        if (pending == 0) alpha_old = alpha;
+        ++pending;
         s.residual(coop_sum(S, rr), mode, thr, maxit);
     }
-    if (pending) {   // the last iteration's e -= alpha p
-        const double* p = (s.iters & 1) ? pa : pb;
+    if (pending > 0) {   // the last iterations' updates of e
+        const double* p1 = ((s.iters - pending + 1) & 1) ? pa : pb;
+        const double* p2 = (s.iters & 1) ? pa : pb;
         for (int u = first; u < units; u += step) {
             const int kz = u / uxy, rem = u - kz * uxy, jj = rem / ux, i0 = 2 * (rem - jj * ux) + 1, k0 = kz * KZ + 1;
             for (int k = k0; k < k0 + KZ && k <= nz; ++k) {
                 const int c = kBase + (i0 - 1) + px * (jj + 1) + pxy * k;
                 double2 ev = lg2(e + c);
-                const double2 pv = lg2(p + c);
-                ev.x = ev.x - s.alpha * pv.x;
-                ev.y = ev.y - s.alpha * pv.y;
+                double2 pv = lg2(p1 + c);
+                ev.x = ev.x - alpha_old * pv.x;
+                ev.y = ev.y - alpha_old * pv.y;
+                if (pending == 2) {
+                    pv = lg2(p2 + c);
+                    ev.x = ev.x - s.alpha * pv.x;
+                    ev.y = ev.y - s.alpha * pv.y;
+                }
                 put(e + c, ev, i0 < nx);
             }
         }

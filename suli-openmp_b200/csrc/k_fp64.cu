@@ -1823,7 +1823,8 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
 // iteration on a B200 (two kernels an iteration in a graph loop in brackets): k_cg_one 3.9 us at
 // 25x50x45 (17.5; k_cg_reg 5.5), 4.1 at 64x32x48 (16.5; 6.0), 5.4 at 57x49x53 (17.9); above its
 // 151,552 cells on 148 SMs k_cg_two 12.9 at 64x64x48 (16.8), 14.9 at 80^3 (20.4), 31.0 at
-// 111x110x110 (41.8), 47.2 at 128^3 (55.8), 83.4 at 256x128x128 (103.4), 617 at 512x256x256 (708).
+// 111x110x110 (41.8), 47.2 at 128^3 (55.8), 83.4 at 256x128x128 (103.4), 617 at 512x256x256 (708); since then
+// k_cg_two updates e every other iteration, 80 at 256x128x128.
 constexpr int kRegU = 4, kRegNT = 256, kOneU = 4, kOneNT = 256, kTwoKZ = 2, kTwoNT = 1024;
 static_assert(kRegU * kRegNT == kOneU * kOneNT, "the register kernels hold the same grids");
 constexpr int kOneSmem = 8 * kOneU * kOneNT * (int)sizeof(double);

@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
 // asymmetric operator (a periodic axis with the reference's clamped end faces, 8_derivadas.f90:318-323,
 // when the density varies across it) makes p.A~p another number, so those solves keep k_cg_reg.
 // A resumed solve reads p and s, which end in cg_pa and cg_q.
-// Bound by the latency of its one sum, whose last part the neighbours' loads overlap: 3.9 us an
-// iteration at 25x50x45 where k_cg_reg takes 5.5, 4.1 at 64x32x48 against 6.0.
+// Bound by the latency of its one sum, whose last part the neighbours' loads overlap: 3.4 us an
+// iteration at 25x50x45 where k_cg_reg takes 5.5, 3.8 at 64x32x48 against 6.0.
 template <int U, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, double* pa, double* wa, double* wb, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,

@@ -1820,31 +1820,40 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
 }
 // The cooperative solve: a register kernel while every cell fits the device's threads (one sum an
 // iteration where the operator is symmetric, else two), else the two-pass kernel.  Measured per
-// iteration on a B200 (two kernels an iteration in a graph loop in brackets): k_cg_one 3.9 us at
-// 25x50x45 (17.5; k_cg_reg 5.5), 4.1 at 64x32x48 (16.5; 6.0), 5.4 at 57x49x53 (17.9); above its
+// iteration on a B200 (two kernels an iteration in a graph loop in brackets): k_cg_one 3.4 us at
+// 25x50x45 (17.5; k_cg_reg 5.5), 3.8 at 64x32x48 (16.5; 6.0), 5.3 at 57x49x53 (17.9); above its
 // 151,552 cells on 148 SMs k_cg_two 12.9 at 64x64x48 (16.8), 14.9 at 80^3 (20.4), 31.0 at
 // 111x110x110 (41.8), 47.2 at 128^3 (55.8), 83.4 at 256x128x128 (103.4), 617 at 512x256x256 (708); since then
 // k_cg_two updates e every other iteration, 80 at 256x128x128.
-constexpr int kRegU = 4, kRegNT = 256, kOneU = 4, kOneNT = 256, kTwoKZ = 2, kTwoNT = 1024;
-static_assert(kRegU * kRegNT == kOneU * kOneNT, "the register kernels hold the same grids");
-constexpr int kOneSmem = 8 * kOneU * kOneNT * (int)sizeof(double);
+// The register kernels hold three cells a thread while that fits (113,664 cells), else four, at
+// which they spill: k_cg_one 2.8 us instead of 3.5 at 40x20x24, 3.43 instead of 3.84 at 25x50x45,
+// 3.77 instead of 4.07 at 64x32x48.  Two cells a thread, or 192 to 384 threads: no better.
+constexpr int kRegNT = 256, kRegMaxU = 4, kTwoKZ = 2, kTwoNT = 1024;
+constexpr int one_smem(int u) { return 8 * u * kRegNT * (int)sizeof(double); }
 static bool cg_symmetric(const suli_ctx* c) { return c->bc.wrapf || !(c->bc.perx || c->bc.pery || c->bc.perz); }
 // whether the device runs them; returns their work area's 8-byte elements
 size_t coop_ready(suli_ctx* c) {
     c->coop_ctas = 0;
     if (const char* ev = std::getenv("SULI_NO_COOP"))
         if (std::strcmp(ev, "1") == 0) return 0;
-    int ok = 0, nsm = 0, a = 0, b = 0, d = 0;
+    int ok = 0, nsm = 0;
     if (cudaDeviceGetAttribute(&ok, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess || !ok ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_cg_reg<kRegU, kRegNT>, kRegNT, 0) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_two<kTwoKZ, kTwoNT>, kTwoNT, 0) != cudaSuccess ||
-        cudaFuncSetAttribute(k_cg_one<kOneU, kOneNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_cg_one<kOneU, kOneNT>, kOneNT, kOneSmem) != cudaSuccess ||
-        a < 1 || b < 1 || d < 1) {
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
+    auto fits = [&](const void* k, int threads, int smem) {
+        int n = 0;
+        const bool r = (smem == 0 || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess) &&
+                       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) == cudaSuccess && n >= 1;
+        if (!r) cudaGetLastError();
+        return r;
+    };
+    if (!fits((const void*)k_cg_reg<3, kRegNT>, kRegNT, 0) || !fits((const void*)k_cg_reg<kRegMaxU, kRegNT>, kRegNT, 0) ||
+        !fits((const void*)k_cg_one<3, kRegNT>, kRegNT, one_smem(3)) ||
+        !fits((const void*)k_cg_one<kRegMaxU, kRegNT>, kRegNT, one_smem(kRegMaxU)) ||
+        !fits((const void*)k_cg_two<kTwoKZ, kTwoNT>, kTwoNT, 0))
+        return 0;
     c->coop_ctas = nsm;
     return coop_work(nsm);
 }
@@ -1854,17 +1863,20 @@ cudaError_t launch_cg_coop(suli_ctx* c) {
     cudaError_t e = cudaMemsetAsync(c->coop_area, 0, sizeof(double), c->stream);   // the arrival counter
     if (e != cudaSuccess) return e;
     const double *ax = c->cg_ax, *ay = c->cg_ay, *az = c->cg_az;
-    const long long cells = (long long)G.nx * G.ny * G.nz, per = (long long)kRegU * kRegNT;
-    if (cells <= per * c->coop_ctas && cg_symmetric(c)) {
-        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_q, &c->cg_pb, &c->cg_e, &ax, &ay, &az, &c->cg,
-                        &c->coop_area};
-        return cudaLaunchCooperativeKernel(k_cg_one<kOneU, kOneNT>, dim3((unsigned)((cells + per - 1) / per)),
-                                           dim3(kOneNT), args, kOneSmem, c->stream);
-    }
+    const long long cells = (long long)G.nx * G.ny * G.nz;
+    const int u = cells <= 3LL * kRegNT * c->coop_ctas ? 3 : kRegMaxU;
+    const long long per = (long long)u * kRegNT;
     if (cells <= per * c->coop_ctas) {
+        const dim3 ctas((unsigned)((cells + per - 1) / per));
+        if (cg_symmetric(c)) {
+            void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_q, &c->cg_pb, &c->cg_e, &ax, &ay, &az, &c->cg,
+                            &c->coop_area};
+            const void* k = u == 3 ? (const void*)k_cg_one<3, kRegNT> : (const void*)k_cg_one<kRegMaxU, kRegNT>;
+            return cudaLaunchCooperativeKernel(k, ctas, dim3(kRegNT), args, one_smem(u), c->stream);
+        }
         void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_area};
-        return cudaLaunchCooperativeKernel(k_cg_reg<kRegU, kRegNT>, dim3((unsigned)((cells + per - 1) / per)),
-                                           dim3(kRegNT), args, 0, c->stream);
+        const void* k = u == 3 ? (const void*)k_cg_reg<3, kRegNT> : (const void*)k_cg_reg<kRegMaxU, kRegNT>;
+        return cudaLaunchCooperativeKernel(k, ctas, dim3(kRegNT), args, 0, c->stream);
     }
     const long long units = (long long)((G.nx + 1) / 2) * G.ny * ((G.nz + kTwoKZ - 1) / kTwoKZ);
     const long long ctas = std::min<long long>(c->coop_ctas, (units + kTwoNT - 1) / kTwoNT);

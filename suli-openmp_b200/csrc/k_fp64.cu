@@ -494,17 +494,11 @@ __device__ __forceinline__ R classico_hi(const double* __restrict__ a, int c, co
 }
 
 // DER: classico's scheme (adv_type = 1); ADV: 2 rotacional, 3 antissim (advect.cuh; der = 1)
-// About 1500 instructions and 110 loads a face (measured: half of issue, 22 % of the FP64 pipe, a third
-// of L1; 60 % of the stalls wait for loads), so blocks an SM against registers decide: FP32 five
-// blocks (6 at the compiler's own 40 registers: 0.75 -> 0.68 ms a 256x128x128 step; 4: 0.70), FP64 four
-// (3 at 78: 181 -> 162 us at 150x133x90 with der = 2; 5: 173).
-template <typename R, int DER, int ADV>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G, CDConst C, CDFields F) {
-    pdl_wait();
-    const Thread3 t = tid3(1, 1, 1);
-    const int i = t.i, j = t.j, k = t.k, nx = G.nx, ny = G.ny, nz = G.nz;
-    if (i > nx + 1 || j > ny + 1 || k > nz + 1) return;
-    copy_box(G, F.prd1, F.prd0, i, j, k);
+// The right-hand sides at face (i, j, k).  YZ: a row away from the y and z ends (the same for a whole
+// warp), where no index along them is clamped, so the loads there are at constant offsets.
+template <typename R, int DER, int ADV, bool YZ>
+__device__ __forceinline__ void convdiff_at(const Geo& G, const CDConst& C, const CDFields& F, int i, int j, int k) {
+    const int nx = G.nx, ny = G.ny, nz = G.nz;
     const R idx = R(C.idx), idy = R(C.idy), idz = R(C.idz);   // 1/dx, 1/dy, 1/dz
     // every load is the face's own index plus a constant offset (32-bit): a field value at
     // (i + di, j + dj, k + dk), read in the compute type R
@@ -545,10 +539,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G,
         const R dhsdx = (tx1 + tx0) * R(0.5);
         const R ama_i = AT(F.nut, (clampi(i, 1, nx)) - i, 0, 0) * idx;
         const R ama_m = AT(F.nut, (clampi(i - 1, 1, nx)) - i, 0, 0) * idx;
-        const int jp = clampi(j + 1, 2, ny), jm = clampi(j, 2, ny);
+        const int jp = (YZ ? j + 1 : clampi(j + 1, 2, ny)), jm = (YZ ? j : clampi(j, 2, ny));
         const R bma_p = ((AT(F.xnut, 0, (jp) - j, 0) + AT(F.xnut, 0, (jp - 1) - j, 0)) * R(0.5)) * idy;
         const R bma_m = ((AT(F.xnut, 0, (jm) - j, 0) + AT(F.xnut, 0, (jm - 1) - j, 0)) * R(0.5)) * idy;
-        const int kp = clampi(k + 1, 2, nz), km = clampi(k, 2, nz);
+        const int kp = (YZ ? k + 1 : clampi(k + 1, 2, nz)), km = (YZ ? k : clampi(k, 2, nz));
         const R dma_p = ((AT(F.xnut, 0, 0, (kp) - k) + AT(F.xnut, 0, 0, (kp - 1) - k)) * R(0.5)) * idz;
         const R dma_m = ((AT(F.xnut, 0, 0, (km) - k) + AT(F.xnut, 0, 0, (km - 1) - k)) * R(0.5)) * idz;
         const R Gv = (ama_i * R(2.) * (AT(u, 1, 0, 0) - uc) - ama_m * R(2.) * (uc - AT(u, -1, 0, 0))) * idx +
@@ -564,7 +558,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G,
     // ---- Fv on v-faces (i = 1..nx, j = 1..ny+1, k = 1..nz)
     if (i <= nx && k <= nz) {
         const R vc = AT(v, 0, 0, 0);
-        const int jc = clampi(j, 2, ny);
+        const int jc = (YZ ? j : clampi(j, 2, ny));
         R vint;
         if constexpr (ADV != 1) {
             vint = split_form_v<R, ADV>(FaceTaps<R>{c0, px, pxy}, u, v, w, i, j, k, ny, idx, idy, idz);
@@ -593,9 +587,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G,
         const int ip = clampi(i + 1, 2, nx), im = clampi(i, 2, nx);
         const R amb_p = ((AT(F.ynut, (ip) - i, 0, 0) + AT(F.ynut, (ip - 1) - i, 0, 0)) * R(0.5)) * idx;
         const R amb_m = ((AT(F.ynut, (im) - i, 0, 0) + AT(F.ynut, (im - 1) - i, 0, 0)) * R(0.5)) * idx;
-        const R bmb_j = AT(F.nut, 0, (clampi(j, 1, ny)) - j, 0) * idy;
-        const R bmb_m = AT(F.nut, 0, (clampi(j - 1, 1, ny)) - j, 0) * idy;
-        const int kp = clampi(k + 1, 2, nz), km = clampi(k, 2, nz);
+        const R bmb_j = AT(F.nut, 0, ((YZ ? j : clampi(j, 1, ny))) - j, 0) * idy;
+        const R bmb_m = AT(F.nut, 0, ((YZ ? j - 1 : clampi(j - 1, 1, ny))) - j, 0) * idy;
+        const int kp = (YZ ? k + 1 : clampi(k + 1, 2, nz)), km = (YZ ? k : clampi(k, 2, nz));
         const R dmb_p = ((AT(F.ynut, 0, 0, (kp) - k) + AT(F.ynut, 0, 0, (kp - 1) - k)) * R(0.5)) * idz;
         const R dmb_m = ((AT(F.ynut, 0, 0, (km) - k) + AT(F.ynut, 0, 0, (km - 1) - k)) * R(0.5)) * idz;
         const R Gv = amb_p * ((AT(v, 1, 0, 0) - vc) * idx + (AT(u, 1, 0, 0) - AT(u, 1, -1, 0)) * idy) -
@@ -611,7 +605,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G,
     // ---- Fw on w-faces (i = 1..nx, j = 1..ny, k = 1..nz+1)
     if (i <= nx && j <= ny) {
         const R wc = AT(w, 0, 0, 0);
-        const int kc = clampi(k, 2, nz);
+        const int kc = (YZ ? k : clampi(k, 2, nz));
         R wint;
         if constexpr (ADV != 1) {
             wint = split_form_w<R, ADV>(FaceTaps<R>{c0, px, pxy}, u, v, w, i, j, k, nz, idx, idy, idz);
@@ -640,11 +634,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G,
         const int ip = clampi(i + 1, 2, nx), im = clampi(i, 2, nx);
         const R amd_p = ((AT(F.znut, (ip) - i, 0, 0) + AT(F.znut, (ip - 1) - i, 0, 0)) * R(0.5)) * idx;
         const R amd_m = ((AT(F.znut, (im) - i, 0, 0) + AT(F.znut, (im - 1) - i, 0, 0)) * R(0.5)) * idx;
-        const int jp = clampi(j + 1, 2, ny), jm = clampi(j, 2, ny);
+        const int jp = (YZ ? j + 1 : clampi(j + 1, 2, ny)), jm = (YZ ? j : clampi(j, 2, ny));
         const R bmd_p = ((AT(F.znut, 0, (jp) - j, 0) + AT(F.znut, 0, (jp - 1) - j, 0)) * R(0.5)) * idy;
         const R bmd_m = ((AT(F.znut, 0, (jm) - j, 0) + AT(F.znut, 0, (jm - 1) - j, 0)) * R(0.5)) * idy;
-        const R dmd_k = AT(F.nut, 0, 0, (clampi(k, 1, nz)) - k) * idz;
-        const R dmd_m = AT(F.nut, 0, 0, (clampi(k - 1, 1, nz)) - k) * idz;
+        const R dmd_k = AT(F.nut, 0, 0, ((YZ ? k : clampi(k, 1, nz))) - k) * idz;
+        const R dmd_m = AT(F.nut, 0, 0, ((YZ ? k - 1 : clampi(k - 1, 1, nz))) - k) * idz;
         const R Gv = amd_p * ((AT(w, 1, 0, 0) - wc) * idx + (AT(u, 1, 0, 0) - AT(u, 1, 0, -1)) * idz) -
                           amd_m * ((wc - AT(w, -1, 0, 0)) * idx + (AT(u, 0, 0, 0) - AT(u, 0, 0, -1)) * idz) +
                           bmd_p * ((AT(w, 0, 1, 0) - wc) * idy + (AT(v, 0, 1, 0) - AT(v, 0, 1, -1)) * idz) -
@@ -656,6 +650,27 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G,
         F.Fw[c0] = (double)r;
     }
 #undef AT
+}
+
+// About 1500 instructions and 110 loads a face (measured: half of issue, 22 % of the FP64 pipe, a third
+// of L1; 60 % of the stalls wait for loads), so blocks an SM against registers decide: FP32 five
+// blocks (6 at the compiler's own 40 registers: 0.75 -> 0.68 ms a 256x128x128 step; 4: 0.70), FP64 four
+// (3 at 78: 181 -> 162 us at 150x133x90 with der = 2; 5: 173).  In FP64 the rows away from the y and
+// z ends take loads at constant offsets (162 -> 148 us); in FP32 that spills and gave nothing.
+template <typename R, int DER, int ADV>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 4) k_convdiff(Geo G, CDConst C, CDFields F) {
+    pdl_wait();
+    const Thread3 t = tid3(1, 1, 1);
+    const int i = t.i, j = t.j, k = t.k;
+    if (i > G.nx + 1 || j > G.ny + 1 || k > G.nz + 1) return;
+    copy_box(G, F.prd1, F.prd0, i, j, k);
+    if constexpr (sizeof(R) == 8) {
+        if (j >= 2 && j < G.ny && k >= 2 && k < G.nz) {
+            convdiff_at<R, DER, ADV, true>(G, C, F, i, j, k);
+            return;
+        }
+    }
+    convdiff_at<R, DER, ADV, false>(G, C, F, i, j, k);
 }
 
 // ------------------------------------------------------------------------------------

@@ -330,13 +330,13 @@ enum suli_kernel {
     SULI_K_TEMPO,
     SULI_K_CONTORNO,
     SULI_K_CG_SETUP,
-    SULI_K_CG_SPMV,        /* CG kernel A: p = r + beta p, q = A p, p.q */
+    SULI_K_CG_SPMV,        /* the cooperative FP64 CG; CG kernel A: p = r + beta p, q = A p, p.q */
     SULI_K_CG_UPDATE,      /* CG kernel B: e -= alpha p, r -= alpha q, r.r */
     SULI_K_CG_FINAL,
     SULI_K_POSDIN,
     SULI_K_EST,
-    SULI_K_MG,             /* precision 1: FP32 inner PCG iterations (SpMV, update, multigrid
-                              V-cycle), launched as one CUDA graph per iteration */
+    SULI_K_MG,             /* precision 1: FP32 inner PCG iterations (multigrid V-cycle, SpMV,
+                              update), an inner solve launched as one CUDA graph */
     SULI_K_REFINE,         /* precision 1: FP64 residual and correction of the refinement */
     SULI_K_NN,             /* learned initial guess: the network's forward pass (its input
                               features and the FP64 step count as CG_SETUP) */

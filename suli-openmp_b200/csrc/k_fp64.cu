@@ -441,6 +441,10 @@ struct CDConst {
 // that axis: the halo box 0..n+1 copied by a kernel over the faces
 __device__ __forceinline__ void copy_box(const Geo& G, const double* __restrict__ src, double* __restrict__ dst, int i,
                                          int j, int k) {
+    if (i > 1 && j > 1 && k > 1) {
+        FIDX(dst, i, j, k) = FIDX(src, i, j, k);
+        return;
+    }
     for (int kk = (k == 1) ? 0 : k; kk <= k; ++kk)
         for (int jj = (j == 1) ? 0 : j; jj <= j; ++jj)
             for (int ii = (i == 1) ? 0 : i; ii <= i; ++ii) FIDX(dst, ii, jj, kk) = FIDX(src, ii, jj, kk);
@@ -1465,8 +1469,9 @@ __global__ void k_cg_final(Geo G, BC bc, const double* __restrict__ sdv, const d
 // ------------------------------------------------------------------------------------
 // A thread owns a column of kPosZ faces (i, j, k0 .. k0 + kPosZ - 1) and walks it in z, so the
 // plane below (prd1 and rho at k - 1) was read by the same thread a step earlier and comes from
-// L1 instead of being fetched again from DRAM by another block.
-constexpr int kPosZ = 8;
+// L1 instead of being fetched again from DRAM by another block.  At 256x128x128, three launches: 265
+// us with eight planes a thread, 250 with four or two (copy_box's loops at every face: 283).
+constexpr int kPosZ = 4;
 __global__ void __launch_bounds__(256) k_posdin(Geo G, BC bc, double aux1, double aux2, double aux3,
                                                 const double* __restrict__ rho, const double* __restrict__ prd1,
                                                 double* __restrict__ u, double* __restrict__ v,

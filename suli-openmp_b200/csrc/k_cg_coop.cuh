@@ -49,12 +49,10 @@ __device__ __forceinline__ void coop_store(const CoopCG& s, bool failed, CGState
 // Cells are numbered along x, so the loads of a warp run along rows.  Bound by the latencies of
 // its two sums and of the neighbours' loads (25x50x45: 5.5 us an iteration, 17.5 with two kernels).
 template <int U, int NT>
-__global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, double* pa, double* e,
-                                                  const double* __restrict__ ax, const double* __restrict__ ay,
-                                                  const double* __restrict__ az, CGState* st, double* work) {
-    __shared__ double sh[kCoopShared];
+__device__ __forceinline__ void cg_reg(const Geo& G, const BC& bc, double* r, double* pa, double* e,
+                                       const double* __restrict__ ax, const double* __restrict__ ay,
+                                       const double* __restrict__ az, CGState* st, double* work, double* sh) {
     CoopCG s = coop_load(st);
-    if (s.done) return;
     const double thr = st->thr;
     const int mode = st->mode, maxit = st->maxit;
     CoopGrid S(work, sh);
@@ -129,6 +127,14 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
         }
     if (blockIdx.x == 0 && threadIdx.x == 0) coop_store(s, S.failed, st);
 }
+template <int U, int NT>
+__global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, double* pa, double* e,
+                                                  const double* __restrict__ ax, const double* __restrict__ ay,
+                                                  const double* __restrict__ az, CGState* st, double* work) {
+    __shared__ double sh[kCoopShared];
+    if (st->done) return;
+    cg_reg<U, NT>(G, bc, r, pa, e, ax, ay, az, st, work, sh);
+}
 
 // Small grids whose operator is symmetric: the same iteration in Chronopoulos and Gear's form
 // (J. Comput. Appl. Math. 25, 1989), which needs one grid-wide sum: with w = A~ r,
@@ -137,22 +143,35 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
 // and r and s at their six neighbours, which it advances itself (the owner's expressions), so an
 // iteration loads only w at the neighbours and stores only w, in two arrays in turn (a CTA may be
 // one sum ahead).  e, p and the coefficients sit in shared memory, the rest in registers.
-// In exact arithmetic the iterates are k_cg_reg's; measured on tanks with density ratio 833, the
-// iteration counts and the true residuals agree down to a relative residual of 1e-12.  An
-// asymmetric operator (a periodic axis with the reference's clamped end faces, 8_derivadas.f90:318-323,
-// when the density varies across it) makes p.A~p another number, so those solves keep k_cg_reg.
-// A resumed solve reads p and s, which end in cg_pa and cg_q.
+// In exact arithmetic the iterates are k_cg_reg's.  An asymmetric operator (a periodic axis with the
+// reference's clamped end faces, 8_derivadas.f90:318-323, when the density varies across it) makes p.A~p
+// another number, so those solves keep k_cg_reg.  So does a system without a solution: every
+// boundary is a Neumann one, the null vector of A~ is sqrt(d), and the part of r along it
+// (CGState.null2, its square) stays in r for good.  Once r is little more than that part, p.A~p is
+// the small difference of two large terms and can come out negative: a channel with an unbalanced
+// outflow took up to ten times the iterations and left three to ten times the divergence of the two-sum
+// form.  Restated on the CPU (density ratio 833, tolerances 1e-4 to 1e-18, warm and cold starts),
+// the two forms agree in iterations and in the true residual wherever null2 <= 1e-2 thr, and part from
+// 1e-1 thr on; kNullPart leaves a factor of ten.  A balanced system has null2 of rounding, about
+// 1e-38 b~.b~.
+// A resumed solve reads p and s, which end in cg_pa and cg_q; one whose threshold the divergence test
+// lowered past the rule goes on in the two-sum form from r, e and p.
 // Bound by the latency of its one sum, whose last part the neighbours' loads overlap: 3.4 us an
 // iteration at 25x50x45 where k_cg_reg takes 5.5, 3.8 at 64x32x48 against 6.0.
+constexpr double kNullPart = 1e-3;
 template <int U, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, double* pa, double* wa, double* wb, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
                                                   const double* __restrict__ az, CGState* st, double* work) {
     extern __shared__ double cells[];   // [8 U][NT]: six coefficients, e, p
     __shared__ double sh[kCoopShared];
-    CoopCG t = coop_load(st);
-    if (t.done) return;
+    if (st->done) return;
     const double thr = st->thr;
+    if (!(st->null2 <= kNullPart * thr)) {   // the same for every CTA
+        cg_reg<U, NT>(G, bc, r, pa, e, ax, ay, az, st, work, sh);
+        return;
+    }
+    CoopCG t = coop_load(st);
     const int mode = st->mode, maxit = st->maxit;
     CoopGrid S(work, sh);
     const int px = G.px, pxy = (int)G.pxy;

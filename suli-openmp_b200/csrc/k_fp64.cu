@@ -1172,7 +1172,7 @@ __global__ void __launch_bounds__(256) k_cg_diag(Geo G, BC bc, CGConst K, const 
 
 // scaled face coefficients s/sqrt(d_c d_nb) = s * (1/sqrt(d_c)) * (1/sqrt(d_nb)) and the first
 // residual (:126-151); reduction of r.r and b.b.  Plain: the reference's residual, whose
-// neighbours outside the box are prd1's ghosts.  MX: the refinement's residual (k_mx_outer: ghosts
+// neighbours outside the box are prd1's ghosts, and its part along the null vector (null2).  MX: the refinement's residual (k_mx_outer: ghosts
 // map to cells), rounded to FP32 as the inner solve's right-hand side r_u = sqrt(d) r~, with
 // its sums; the refinement's own first pass over the coefficients is saved (set-up and refinement
 // of a 256x128x128 step 1.86 -> 1.59 ms).  Forming the faces from the density here and in
@@ -1189,7 +1189,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
-    double rr = 0.0, bbv = 0.0, ru2 = 0.0, um = 0.0;
+    double rr = 0.0, bbv = 0.0, ru2 = 0.0, um = 0.0, zr = 0.0, zz = 0.0;
     // a thread owns kCoefZ cells of a column: 4x fewer blocks than one cell a thread, whose
     // partials the grid reduction (one counter) would otherwise take in turn
 #pragma unroll
@@ -1231,17 +1231,21 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
             um = fmax(um, fabs(uv));
         } else {
             r[c] = rv;
+            zr += sd[c] * rv;
+            zz += sd[c] * sd[c];
         }
     }
     }
-    double trr, tbb, tru2 = 0.0, tum = 0.0;
+    double trr, tbb, tru2 = 0.0, tum = 0.0, tnull = 0.0;
     bool last;
     if (MX) {
         double s[3] = {rr, bbv, ru2}, t[3];
         last = reduce_sums_max_last<3>(s, um, partial, counter, t, tum);
         trr = t[0]; tbb = t[1]; tru2 = t[2];
     } else {
-        last = reduce2_last(rr, bbv, partial, counter, trr, tbb);
+        double s[4] = {rr, bbv, zr, zz}, t[4];
+        last = reduce_sums_max_last<4>(s, 0.0, partial, counter, t, tum);
+        trr = t[0]; tbb = t[1]; tnull = t[2] * (t[2] / t[3]);
     }
     if (last && flat_tid() == 0) {
         st->rr = trr;
@@ -1255,6 +1259,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
         st->status = 0;
         st->div_tol = K.div_tol;
         st->rmax = tum;
+        st->null2 = tnull;
         const bool go = MX ? (trr > st->thr || (K.div_tol > 0. && !(tum <= K.div_tol)))
                            : (fabs(trr) > st->thr) && (K.maxit > 0);
         st->done = go ? 0 : 1;
@@ -1839,7 +1844,8 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
                c->red_partial, c->red_counter);
 }
 // The cooperative solve: a register kernel while every cell fits the device's threads (one sum an
-// iteration where the operator is symmetric, else two), else the two-pass kernel.  Measured per
+// iteration where the operator is symmetric and, as k_cg_one sees on the device, the system has a
+// solution; else two), else the two-pass kernel.  Measured per
 // iteration on a B200 (two kernels an iteration in a graph loop in brackets): k_cg_one 3.4 us at
 // 25x50x45 (17.5; k_cg_reg 5.5), 3.8 at 64x32x48 (16.5; 6.0), 5.3 at 57x49x53 (17.9); above its
 // 151,552 cells on 148 SMs k_cg_two 12.9 at 64x64x48 (16.8), 14.9 at 80^3 (20.4), 31.0 at

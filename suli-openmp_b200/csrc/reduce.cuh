@@ -123,8 +123,9 @@ static __device__ bool reduce_sums_max_last(double (&a)[NS], double m, double* p
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    // partials tid, tid + nt, ... in that order, eight blocks' loads ahead of the folds
-    constexpr int U = 8;
+    // partials tid, tid + nt, ... in that order, eight blocks' loads ahead of the folds (four with
+    // four sums: eight would spill at 64 registers)
+    constexpr int U = NS < 4 ? 8 : 4;
     double sa[NS] = {}, sm = 0.0;
     for (int q0 = tid; q0 < nb; q0 += U * nt) {
         double pa[U][NS], pm[U];

@@ -35,7 +35,7 @@ struct CGState {
     int maxit;
     int mode;         // suli_params.cg_stop
     int status;       // 0 ok, SULI_WARN_CG_MAXIT, SULI_ERR_NAN
-    int pad;
+    int gave_up;      // a CTA's wait in the cooperative CG ran out (k_coop.cuh)
     double div_tol;   // suli_params.div_tol (0: off)
     double rmax;      // max |sqrt(d) r~| of the last check: the max |div u| projection leaves
     double null2;     // square of r~'s part along the null vector sqrt(d) (plain set-up), which no

@@ -35,7 +35,11 @@ struct CoopCG {
 __device__ __forceinline__ CoopCG coop_load(const CGState* st) {
     return CoopCG{st->rr, st->rr_start, st->alpha, st->beta, st->pq, st->iters, st->done, st->status};
 }
+// the end of a CTA's part of the solve: its failure, and from CTA 0 the state
 __device__ __forceinline__ void coop_store(const CoopCG& s, bool failed, CGState* st) {
+    if (threadIdx.x != 0) return;
+    if (failed) st->gave_up = 1;
+    if (blockIdx.x != 0) return;
     st->rr = s.rr; st->rr_start = s.rr_start; st->alpha = s.alpha; st->beta = s.beta; st->pq = s.pq;
     st->iters = s.iters;
     st->done = 1;
@@ -51,11 +55,11 @@ __device__ __forceinline__ void coop_store(const CoopCG& s, bool failed, CGState
 template <int U, int NT>
 __device__ __forceinline__ void cg_reg(const Geo& G, const BC& bc, double* r, double* pa, double* e,
                                        const double* __restrict__ ax, const double* __restrict__ ay,
-                                       const double* __restrict__ az, CGState* st, double* work, double* sh) {
+                                       const double* __restrict__ az, CGState* st, double* work, int polls, double* sh) {
     CoopCG s = coop_load(st);
     const double thr = st->thr;
     const int mode = st->mode, maxit = st->maxit;
-    CoopGrid S(work, sh);
+    CoopGrid S(work, sh, polls);
     const int px = G.px, pxy = (int)G.pxy;
     const int total = G.nx * G.ny * G.nz, step = gridDim.x * NT;
     int c[U], nb[U][6];
@@ -125,15 +129,15 @@ __device__ __forceinline__ void cg_reg(const Geo& G, const BC& bc, double* r, do
             e[c[u]] = ec[u];
             pa[c[u]] = p[u];
         }
-    if (blockIdx.x == 0 && threadIdx.x == 0) coop_store(s, S.failed, st);
+    coop_store(s, S.failed, st);
 }
 template <int U, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, double* pa, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
-                                                  const double* __restrict__ az, CGState* st, double* work) {
+                                                  const double* __restrict__ az, CGState* st, double* work, int polls) {
     __shared__ double sh[kCoopShared];
     if (st->done) return;
-    cg_reg<U, NT>(G, bc, r, pa, e, ax, ay, az, st, work, sh);
+    cg_reg<U, NT>(G, bc, r, pa, e, ax, ay, az, st, work, polls, sh);
 }
 
 // Small grids whose operator is symmetric: the same iteration in Chronopoulos and Gear's form
@@ -162,18 +166,18 @@ constexpr double kNullPart = 1e-3;
 template <int U, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, double* pa, double* wa, double* wb, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
-                                                  const double* __restrict__ az, CGState* st, double* work) {
+                                                  const double* __restrict__ az, CGState* st, double* work, int polls) {
     extern __shared__ double cells[];   // [8 U][NT]: six coefficients, e, p
     __shared__ double sh[kCoopShared];
     if (st->done) return;
     const double thr = st->thr;
     if (!(st->null2 <= kNullPart * thr)) {   // the same for every CTA
-        cg_reg<U, NT>(G, bc, r, pa, e, ax, ay, az, st, work, sh);
+        cg_reg<U, NT>(G, bc, r, pa, e, ax, ay, az, st, work, polls, sh);
         return;
     }
     CoopCG t = coop_load(st);
     const int mode = st->mode, maxit = st->maxit;
-    CoopGrid S(work, sh);
+    CoopGrid S(work, sh, polls);
     const int px = G.px, pxy = (int)G.pxy;
     const int total = G.nx * G.ny * G.nz, step = gridDim.x * NT;
     const bool fresh = (t.iters == 0);
@@ -274,7 +278,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, doubl
             pa[c[u]] = own[(8 * u + 7) * NT];
             wa[c[u]] = sc[u];
         }
-    if (blockIdx.x == 0 && threadIdx.x == 0) coop_store(t, S.failed, st);
+    coop_store(t, S.failed, st);
 }
 
 // Larger grids: the iteration's two passes over units dealt to the threads in turn (a unit is a
@@ -289,13 +293,13 @@ __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, doubl
 template <int KZ, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, double* pa, double* pb, double* q, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,
-                                                  const double* __restrict__ az, CGState* st, double* work) {
+                                                  const double* __restrict__ az, CGState* st, double* work, int polls) {
     __shared__ double sh[kCoopShared];
     CoopCG s = coop_load(st);
     if (s.done) return;
     const double thr = st->thr;
     const int mode = st->mode, maxit = st->maxit;
-    CoopGrid S(work, sh);
+    CoopGrid S(work, sh, polls);
     const int nx = G.nx, ny = G.ny, nz = G.nz, px = G.px, pxy = (int)G.pxy;
     const int ux = (nx + 1) / 2, uxy = ux * ny, units = uxy * ((nz + KZ - 1) / KZ);
     const int first = blockIdx.x * NT + threadIdx.x, step = gridDim.x * NT;
@@ -407,7 +411,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, doubl
             }
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) coop_store(s, S.failed, st);
+    coop_store(s, S.failed, st);
 }
 
 }  // namespace suli

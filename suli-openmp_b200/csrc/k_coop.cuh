@@ -7,13 +7,15 @@
 // order, once every CTA has (fixed order, so a run is bit-reproducible, and no floating-point
 // atomics).  Two sets of partials take turns: a CTA overwrites a set two sums on, when every CTA has
 // arrived at the sum between and so has read it.
-// Each wait is bounded; a wait that runs out ends the solve with SULI_ERR_CUDA.
+// Each wait is bounded by a number of polls (kCoopPolls, a few seconds).  A CTA whose wait runs out
+// leaves the solve, and those that need its next arrival leave after it; any one of them fails the
+// solve with SULI_ERR_CUDA (CGState.gave_up), also where the rest went on to converge.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace suli {
 
-constexpr int kCoopSpin = 1 << 22;   // polls of a bounded wait (each about an L2 latency)
+constexpr int kCoopPolls = 1 << 22;   // polls of a bounded wait (each about an L2 latency)
 constexpr int kCoopShared = 68;      // shared doubles: warp partials, the totals, the failure flag
 // the work area: the counter (zero at launch) and two sets of partial pairs, in 8-byte elements
 __host__ __device__ inline size_t coop_work(int ctas) { return 16 + 4 * (size_t)ctas; }
@@ -24,9 +26,11 @@ struct CoopGrid {
     double* sh;            // [kCoopShared]
     unsigned int target;   // arrivals that end the next wait
     int set;
+    int polls;             // the most a wait polls
     bool failed;
-    __device__ __forceinline__ CoopGrid(double* work, double* shared)
-        : count(reinterpret_cast<unsigned int*>(work)), part(work + 16), sh(shared), target(0), set(0), failed(false) {}
+    __device__ __forceinline__ CoopGrid(double* work, double* shared, int limit)
+        : count(reinterpret_cast<unsigned int*>(work)), part(work + 16), sh(shared), target(0), set(0), polls(limit),
+          failed(false) {}
 };
 
 // the first warp's part: arrive for the CTA and wait for all (after a __syncthreads: every global
@@ -40,7 +44,7 @@ __device__ __forceinline__ void coop_wait(CoopGrid& S) {
         int spin = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(S.count) : "memory");
-        } while ((int)(v - S.target) < 0 && ++spin < kCoopSpin);
+        } while ((int)(v - S.target) < 0 && ++spin < S.polls);
         ok = (int)(v - S.target) >= 0;
         S.sh[66] = ok ? 0. : 1.;
     }

@@ -1257,6 +1257,7 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
         st->maxit = K.maxit;
         st->mode = K.mode;
         st->status = 0;
+        st->gave_up = 0;
         st->div_tol = K.div_tol;
         st->rmax = tum;
         st->null2 = tnull;
@@ -1431,7 +1432,7 @@ __global__ void __launch_bounds__(256) k_cg_divcheck(Geo G, const double* __rest
                                                      const double* __restrict__ r, CGState* st, double* partial,
                                                      unsigned int* counter) {
     pdl_wait();
-    if (!st->done || st->status != 0 || !(st->div_tol > 0.)) return;
+    if (!st->done || st->status != 0 || st->gave_up || !(st->div_tol > 0.)) return;
     const Thread3 t = tid3(1, 1, 1);
     double m = 0.;
     if (t.i <= G.nx && t.j <= G.ny && t.k <= G.nz) {
@@ -1883,8 +1884,14 @@ size_t coop_ready(suli_ctx* c) {
     c->coop_ctas = nsm;
     return coop_work(nsm);
 }
+// the most a grid-wide sum's wait polls; SULI_COOP_POLLS: a smaller number, for tests
+static int coop_polls() {
+    const char* ev = std::getenv("SULI_COOP_POLLS");
+    return ev ? std::max(1, std::min(std::atoi(ev), kCoopPolls)) : kCoopPolls;
+}
 cudaError_t launch_cg_coop(suli_ctx* c) {
     const Geo& G = c->g;
+    int polls = coop_polls();
     ProfScope ps(c, SULI_K_CG_SPMV, 1);
     cudaError_t e = cudaMemsetAsync(c->coop_area, 0, sizeof(double), c->stream);   // the arrival counter
     if (e != cudaSuccess) return e;
@@ -1896,18 +1903,18 @@ cudaError_t launch_cg_coop(suli_ctx* c) {
         const dim3 ctas((unsigned)((cells + per - 1) / per));
         if (cg_symmetric(c)) {
             void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_q, &c->cg_pb, &c->cg_e, &ax, &ay, &az, &c->cg,
-                            &c->coop_area};
+                            &c->coop_area, &polls};
             const void* k = u == 3 ? (const void*)k_cg_one<3, kRegNT> : (const void*)k_cg_one<kRegMaxU, kRegNT>;
             return cudaLaunchCooperativeKernel(k, ctas, dim3(kRegNT), args, one_smem(u), c->stream);
         }
-        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_area};
+        void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_area, &polls};
         const void* k = u == 3 ? (const void*)k_cg_reg<3, kRegNT> : (const void*)k_cg_reg<kRegMaxU, kRegNT>;
         return cudaLaunchCooperativeKernel(k, ctas, dim3(kRegNT), args, 0, c->stream);
     }
     const long long units = (long long)((G.nx + 1) / 2) * G.ny * ((G.nz + kTwoKZ - 1) / kTwoKZ);
     const long long ctas = std::min<long long>(c->coop_ctas, (units + kTwoNT - 1) / kTwoNT);
     void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_pb, &c->cg_q, &c->cg_e, &ax, &ay, &az, &c->cg,
-                    &c->coop_area};
+                    &c->coop_area, &polls};
     return cudaLaunchCooperativeKernel(k_cg_two<kTwoKZ, kTwoNT>, dim3((unsigned)ctas), dim3(kTwoNT), args, 0, c->stream);
 }
 void launch_cg_divcheck(suli_ctx* c) {

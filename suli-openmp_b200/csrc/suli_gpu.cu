@@ -808,7 +808,7 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
     if (iters) *iters = s.iters;
     if (resid) *resid = (s.bb > 0.) ? std::sqrt(s.rr / s.bb) : 0.;
     if (s.status == SULI_ERR_NAN) return fail(c, SULI_ERR_NAN, "graddin: NaN/Inf in the Poisson solve");
-    if (s.status == SULI_ERR_CUDA) return fail(c, SULI_ERR_CUDA, "graddin: a grid-wide sum's wait ran out");
+    if (s.status == SULI_ERR_CUDA || s.gave_up) return fail(c, SULI_ERR_CUDA, "graddin: a grid-wide sum's wait ran out");
     return s.status;
 }
 

@@ -5,6 +5,8 @@
 // flow of the reference (the reinitialisation error loop, the volume-correction loop and the
 // Poisson stopping test) is decided from device-resident scalars; the host reads them back
 // only where the reference branches on them.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -14,6 +16,7 @@
 #include <string>
 #include <vector>
 #include "ctx.cuh"
+#include "devrange.h"
 #include "nn_api.cuh"
 
 using namespace suli;
@@ -360,15 +363,33 @@ static bool host_memory(const void* p) {
     return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
 }
 
-// memory of the context's own GPU that a kernel can read and write in place of a staged copy
-static bool own_memory(const suli_ctx* c, const void* p) {
+// How a field is copied from or to the caller's memory: by a kernel straight from or to it (8-byte
+// aligned memory of the context's own GPU inside one allocation), staged through cg_q by a copy,
+// which knows every other kind of address and refuses one that it cannot read or write, or not at
+// all (device memory that ends before the field does: a kernel would fault).
+enum class Way { direct, staged, none };
+static Way copy_way(const suli_ctx* c, const void* p, size_t bytes) {
     cudaPointerAttributes a{};
-    if (reinterpret_cast<uintptr_t>(p) % sizeof(double) != 0) return false;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return Way::staged;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == c->device;
+    if (a.type != cudaMemoryTypeDevice || a.device != c->device) return Way::staged;
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return Way::staged;
+    }
+    const RangeKind kind = range_kind(reinterpret_cast<uintptr_t>(p), bytes, [&](uintptr_t at, uintptr_t* base, size_t* size) {
+        CUdeviceptr b = 0;
+        if (reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(fn)(&b, size, (CUdeviceptr)at) != CUDA_SUCCESS) return false;
+        *base = (uintptr_t)b;
+        return true;
+    });
+    if (kind == kRangeUnmapped) return Way::none;
+    return kind == kRangeOne && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0 ? Way::direct : Way::staged;
 }
 
 int suli_upload(suli_ctx* c, int field, const double* host) {
@@ -391,7 +412,9 @@ int suli_upload(suli_ctx* c, int field, const double* host) {
                 if (host[q] != 0.0) { c->tf_active = true; break; }
         }
     }
-    if (own_memory(c, host)) {
+    const Way way = copy_way(c, host, n * sizeof(double));
+    if (way == Way::none) return fail(c, SULI_ERR_ARG, "upload: the device array is shorter than the field");
+    if (way == Way::direct) {
         repack<true>(c, field, host, c->f[field]);
     } else {   // stage through the CG q buffer (same size class as any field, free between calls)
         CUDA_TRY(c, cudaMemcpyAsync(c->cg_q, host, n * sizeof(double), cudaMemcpyDefault, c->stream));
@@ -414,7 +437,9 @@ int suli_download(suli_ctx* c, int field, double* host) {
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         return SULI_OK;
     }
-    const bool direct = own_memory(c, host);
+    const Way way = copy_way(c, host, n * sizeof(double));
+    if (way == Way::none) return fail(c, SULI_ERR_ARG, "download: the device array is shorter than the field");
+    const bool direct = way == Way::direct;
     repack<false>(c, field, c->f[field], direct ? host : c->cg_q);
     CHECK_LAUNCH(c);
     if (!direct) CUDA_TRY(c, cudaMemcpyAsync(host, c->cg_q, n * sizeof(double), cudaMemcpyDefault, c->stream));

@@ -860,15 +860,19 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
     // The inner solve's state is copied to the host right after its loop and read at the next
     // synchronisation, so the refinement residual is launched without waiting for the host.
     bool pcg_pending = false;
+    // An error leaves the context as a solve expects it: the next one's first iteration reads the old
+    // direction (times 0), which must be finite, and a kernel that gave up in one CTA while others had
+    // yet to start (they skip a solve that is done) has not all arrivals of its reduction.
+    auto abandon = [&](int code, const char* why) -> int {
+        CUDA_TRY(c, cudaMemsetAsync(c->pc_pb, 0, c->g.n * sizeof(float), c->stream));
+        CUDA_TRY(c, cudaMemsetAsync(c->red_counter, 0, 64 * sizeof(unsigned int), c->stream));
+        return fail(c, code, why);
+    };
     auto take_inner = [&]() -> int {
         pcg_pending = false;
-        if (c->pcg_host[0].status == SULI_ERR_NAN) {
-            // the next solve's first iteration reads the old direction (times 0): leave it finite
-            cudaMemsetAsync(c->pc_pb, 0, c->g.n * sizeof(float), c->stream);
-            return fail(c, SULI_ERR_NAN, "graddin: NaN/Inf in the inner solve");
-        }
+        if (c->pcg_host[0].status == SULI_ERR_NAN) return abandon(SULI_ERR_NAN, "graddin: NaN/Inf in the inner solve");
         if (c->pcg_host[0].status == SULI_ERR_CUDA)
-            return fail(c, SULI_ERR_CUDA, "graddin: a streaming multigrid kernel's wait for its loads ran out");
+            return abandon(SULI_ERR_CUDA, "graddin: a streaming multigrid kernel's wait for its loads ran out");
         inner_total += c->pcg_host[0].iters;
         inner_capped = (c->pcg_host[0].iters >= c->inner_maxit);
         if (c->use_graphs) {   // eager launches were counted as they went
@@ -881,7 +885,7 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
         if (r != SULI_OK) return r;
         if (pcg_pending)
             if (int ri = take_inner()) return ri;
-        if (c->cg_host[0].status == SULI_ERR_NAN) return fail(c, SULI_ERR_NAN, "graddin: NaN/Inf in the Poisson solve");
+        if (c->cg_host[0].status == SULI_ERR_NAN) return abandon(SULI_ERR_NAN, "graddin: NaN/Inf in the Poisson solve");
         if (c->cg_host[0].done) break;
         // a pass that did not halve the FP64 residual, or an inner solve that hit its cap: the
         // FP32 inner solve no longer helps; the plain FP64 CG finishes from the better iterate

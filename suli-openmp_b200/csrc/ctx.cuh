@@ -176,8 +176,8 @@ struct suli_ctx {
     CUtensorMap smap[12];          // boxes with the halo
     CUtensorMap smap_own[12];      // the same arrays, boxes of the tile's own cells
     const float* smap_ptr[12] = {nullptr};
-    // the last thing put on the stream is a kernel of this call (step_launch); the calls suli_step is
-    // made of count as one
+    // the last thing put on the stream is a kernel of this call (step_launch; stream_copy and the like
+    // clear it); the calls suli_step is made of count as one
     bool chained = false, in_step = false;
     int inner_maxit = 200;
     int inner_batch = 4;
@@ -235,6 +235,26 @@ inline void prof_resolve(suli_ctx* c) {
     }
     P.used = 0;
 }
+// Everything on the context's stream that is not a kernel goes through these: a kernel launched as
+// dependent on the work before it waits for kernels only, so the next step_launch must be plain (one
+// behind a device-to-device copy has been seen to read the copy's target before it was written).
+inline cudaError_t stream_copy(suli_ctx* c, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+    c->chained = false;
+    return cudaMemcpyAsync(dst, src, bytes, kind, c->stream);
+}
+inline cudaError_t stream_zero(suli_ctx* c, void* dst, size_t bytes) {
+    c->chained = false;
+    return cudaMemsetAsync(dst, 0, bytes, c->stream);
+}
+inline cudaError_t stream_graph(suli_ctx* c, cudaGraphExec_t g) {
+    c->chained = false;
+    return cudaGraphLaunch(g, c->stream);
+}
+inline cudaError_t stream_wait(suli_ctx* c, cudaEvent_t e) {
+    c->chained = false;
+    return cudaStreamWaitEvent(c->stream, e, 0);
+}
+
 // RAII timer of one kernel class around `n` launches on the context's stream.
 struct ProfScope {
     suli_ctx* c;

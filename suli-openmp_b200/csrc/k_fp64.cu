@@ -1572,7 +1572,7 @@ static dim3 faces_grid(const Geo& g) { return grid3(g.nx + 1, g.ny + 1, g.nz + 1
 // Launch a kernel of the step (each calls pdl_wait first).  Behind another kernel of the same call
 // (c->chained) it is a dependent launch, which overlaps its start with the end of the one before:
 // the grids of a small step run shorter than a plain launch takes.  Behind anything else (a copy,
-// a memset, work a caller put on the stream) it is a plain launch.
+// a memset, a graph, an event's wait, work a caller put on the stream) it is a plain launch.
 template <typename... KArgs, typename... Args>
 static void step_launch(suli_ctx* c, void (*kernel)(KArgs...), dim3 grid, dim3 block, Args... args) {
     if (c->chained) pdl_launch(kernel, grid, block, c->stream, args...);
@@ -1730,8 +1730,7 @@ void launch_boundary_waves(suli_ctx* c) {
     const dim3 b2(32, 8);
     ProfScope ps(c, SULI_K_CONTORNO, 2);
     step_launch(c, k_ls_round_float, cells_grid(G), kBlk, G, c->f[SULI_F_LS]);
-    cudaMemsetAsync(c->f[SULI_F_BXY0], 0, c->plane_elems[SULI_F_BXY0] * sizeof(double), c->stream);   // v1 never set
-    c->chained = false;
+    stream_zero(c, c->f[SULI_F_BXY0], c->plane_elems[SULI_F_BXY0] * sizeof(double));   // v1 never set
     step_launch(c, k_waves, grid3(G.ny + 2, G.nz + 3, 1, b2), b2, G, c->wave, c->P.dx, c->P.dz, c->t, c->f[SULI_F_LS],
                                                                      c->f[SULI_F_BXX0], c->f[SULI_F_BXX1], c->f[SULI_F_BXZ0]);
 }
@@ -1831,17 +1830,17 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
         ProfScope ps(c, SULI_K_CG_SPMV, 1);
         if (G.nx % 2 == 0) {
             const dim3 g2((G.nx / 2 + kTX - 1) / kTX, (G.ny + kTY - 1) / kTY, (G.nz + kCGZA - 1) / kCGZA);
-            pdl_launch(k_cg_spmv2, g2, b, c->stream, G, c->bc, (const double*)c->cg_r, p_old, p_new, c->cg_q,
+            step_launch(c, k_cg_spmv2, g2, b, G, c->bc, (const double*)c->cg_r, p_old, p_new, c->cg_q,
                        (const double*)c->cg_ax, (const double*)c->cg_ay, (const double*)c->cg_az, c->cg,
                        c->red_partial, c->red_counter);
         } else {
-            pdl_launch(k_cg_spmv, ga, b, c->stream, G, c->bc, (const double*)c->cg_r, p_old, p_new, c->cg_q,
+            step_launch(c, k_cg_spmv, ga, b, G, c->bc, (const double*)c->cg_r, p_old, p_new, c->cg_q,
                        (const double*)c->cg_ax, (const double*)c->cg_ay, (const double*)c->cg_az, c->cg,
                        c->red_partial, c->red_counter);
         }
     }
     ProfScope ps(c, SULI_K_CG_UPDATE, 1);
-    pdl_launch(k_cg_update, gb, b, c->stream, G, c->cg_e, c->cg_r, (const double*)p_new, (const double*)c->cg_q, c->cg,
+    step_launch(c, k_cg_update, gb, b, G, c->cg_e, c->cg_r, (const double*)p_new, (const double*)c->cg_q, c->cg,
                c->red_partial, c->red_counter);
 }
 // The cooperative solve: a register kernel while every cell fits the device's threads (one sum an
@@ -1893,8 +1892,13 @@ cudaError_t launch_cg_coop(suli_ctx* c) {
     const Geo& G = c->g;
     int polls = coop_polls();
     ProfScope ps(c, SULI_K_CG_SPMV, 1);
-    cudaError_t e = cudaMemsetAsync(c->coop_area, 0, sizeof(double), c->stream);   // the arrival counter
+    cudaError_t e = stream_zero(c, c->coop_area, sizeof(double));   // the arrival counter
     if (e != cudaSuccess) return e;
+    auto launch = [&](const void* k, dim3 ctas, int threads, void** args, int smem) {
+        const cudaError_t r = cudaLaunchCooperativeKernel(k, ctas, dim3(threads), args, smem, c->stream);
+        c->chained = r == cudaSuccess;
+        return r;
+    };
     const double *ax = c->cg_ax, *ay = c->cg_ay, *az = c->cg_az;
     const long long cells = (long long)G.nx * G.ny * G.nz;
     const int u = cells <= 3LL * kRegNT * c->coop_ctas ? 3 : kRegMaxU;
@@ -1905,17 +1909,17 @@ cudaError_t launch_cg_coop(suli_ctx* c) {
             void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_q, &c->cg_pb, &c->cg_e, &ax, &ay, &az, &c->cg,
                             &c->coop_area, &polls};
             const void* k = u == 3 ? (const void*)k_cg_one<3, kRegNT> : (const void*)k_cg_one<kRegMaxU, kRegNT>;
-            return cudaLaunchCooperativeKernel(k, ctas, dim3(kRegNT), args, one_smem(u), c->stream);
+            return launch(k, ctas, kRegNT, args, one_smem(u));
         }
         void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_e, &ax, &ay, &az, &c->cg, &c->coop_area, &polls};
         const void* k = u == 3 ? (const void*)k_cg_reg<3, kRegNT> : (const void*)k_cg_reg<kRegMaxU, kRegNT>;
-        return cudaLaunchCooperativeKernel(k, ctas, dim3(kRegNT), args, 0, c->stream);
+        return launch(k, ctas, kRegNT, args, 0);
     }
     const long long units = (long long)((G.nx + 1) / 2) * G.ny * ((G.nz + kTwoKZ - 1) / kTwoKZ);
     const long long ctas = std::min<long long>(c->coop_ctas, (units + kTwoNT - 1) / kTwoNT);
     void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_pb, &c->cg_q, &c->cg_e, &ax, &ay, &az, &c->cg,
                     &c->coop_area, &polls};
-    return cudaLaunchCooperativeKernel(k_cg_two<kTwoKZ, kTwoNT>, dim3((unsigned)ctas), dim3(kTwoNT), args, 0, c->stream);
+    return launch((const void*)k_cg_two<kTwoKZ, kTwoNT>, dim3((unsigned)ctas), kTwoNT, args, 0);
 }
 void launch_cg_divcheck(suli_ctx* c) {
     const Geo& G = c->g;

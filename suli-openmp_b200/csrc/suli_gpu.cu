@@ -111,7 +111,7 @@ void repack(suli_ctx* c, int field, const double* src, double* dst) {
 }
 
 int sync_read(suli_ctx* c, const void* dev, void* host, size_t bytes) {
-    CUDA_TRY(c, cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, stream_copy(c, host, dev, bytes, cudaMemcpyDeviceToHost));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return SULI_OK;
 }
@@ -243,7 +243,7 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
     const size_t coop = coop_ready(c);   // the cooperative CG's work area, after the fields
     c->arena_elems = per * (size_t)(n3d + nwork) + coop;
     if ((e = cudaMalloc(&c->arena, c->arena_elems * sizeof(double))) != cudaSuccess) return bail(e, "arena");
-    if ((e = cudaMemsetAsync(c->arena, 0, c->arena_elems * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
+    if ((e = stream_zero(c, c->arena, c->arena_elems * sizeof(double))) != cudaSuccess) return bail(e, "memset");
     c->coop_area = c->arena + per * (size_t)(n3d + nwork);
     for (int f = 0; f < n3d; ++f) c->f[f] = c->arena + per * f;
     double* wk = c->arena + per * n3d;
@@ -257,16 +257,16 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
         const size_t n = (size_t)(hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1);
         c->plane_elems[f] = n;
         if ((e = cudaMalloc(&c->f[f], n * sizeof(double))) != cudaSuccess) return bail(e, "plane");
-        if ((e = cudaMemsetAsync(c->f[f], 0, n * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
+        if ((e = stream_zero(c, c->f[f], n * sizeof(double))) != cudaSuccess) return bail(e, "memset");
     }
     // block partials: up to four a block of the face grids; five for at most 128 blocks (outflow_fix)
     const long long nb = (long long)((p->nx + 1 + 31) / 32) * ((p->ny + 1 + 7) / 8) * (p->nz + 1) + 256;
     if ((e = cudaMalloc(&c->red_partial, (size_t)nb * 4 * sizeof(double))) != cudaSuccess) return bail(e, "partial");
     if ((e = cudaMalloc(&c->red_counter, 64 * sizeof(unsigned int))) != cudaSuccess) return bail(e, "counter");
-    if ((e = cudaMemsetAsync(c->red_counter, 0, 64 * sizeof(unsigned int), c->stream)) != cudaSuccess) return bail(e, "memset");
+    if ((e = stream_zero(c, c->red_counter, 64 * sizeof(unsigned int))) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMalloc(&c->red_out, 16 * sizeof(double))) != cudaSuccess) return bail(e, "red_out");
     if ((e = cudaMalloc(&c->cg, sizeof(CGState))) != cudaSuccess) return bail(e, "cg state");
-    if ((e = cudaMemsetAsync(c->cg, 0, sizeof(CGState), c->stream)) != cudaSuccess) return bail(e, "memset");
+    if ((e = stream_zero(c, c->cg, sizeof(CGState))) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMallocHost(&c->cg_host, 2 * sizeof(CGState))) != cudaSuccess) return bail(e, "pinned");
     if ((e = cudaMallocHost(&c->host_scalars, 16 * sizeof(double))) != cudaSuccess) return bail(e, "pinned");
     if (p->precision == 1) {
@@ -281,7 +281,7 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
         size_t tot = 7 * (size_t)gs[0].n + 64;
         for (auto& g : gs) tot += 7 * (size_t)g.n;
         if ((e = cudaMalloc(&c->f32_arena, tot * sizeof(float))) != cudaSuccess) return bail(e, "f32 arena");
-        if ((e = cudaMemsetAsync(c->f32_arena, 0, tot * sizeof(float), c->stream)) != cudaSuccess) return bail(e, "memset");
+        if ((e = stream_zero(c, c->f32_arena, tot * sizeof(float))) != cudaSuccess) return bail(e, "memset");
         float* q = c->f32_arena;
         auto take = [&](size_t n) { float* r = q; q += n; return r; };
         c->pc_x = take(gs[0].n); c->pc_r = take(gs[0].n); c->pc_pa = take(gs[0].n); c->pc_pb = take(gs[0].n);
@@ -295,9 +295,9 @@ int suli_create(const suli_params* p, int device, suli_ctx** out) {
             c->mg.push_back(L);
         }
         if ((e = cudaMalloc(&c->cg_e2, per * sizeof(double))) != cudaSuccess) return bail(e, "e2");
-        if ((e = cudaMemsetAsync(c->cg_e2, 0, per * sizeof(double), c->stream)) != cudaSuccess) return bail(e, "memset");
+        if ((e = stream_zero(c, c->cg_e2, per * sizeof(double))) != cudaSuccess) return bail(e, "memset");
         if ((e = cudaMalloc(&c->pcg, sizeof(PCGState))) != cudaSuccess) return bail(e, "pcg state");
-        if ((e = cudaMemsetAsync(c->pcg, 0, sizeof(PCGState), c->stream)) != cudaSuccess) return bail(e, "memset");
+        if ((e = stream_zero(c, c->pcg, sizeof(PCGState))) != cudaSuccess) return bail(e, "memset");
         if ((e = cudaMallocHost(&c->pcg_host, 2 * sizeof(PCGState))) != cudaSuccess) return bail(e, "pinned");
         cluster_ready(c);
         stream_ready(c);
@@ -400,7 +400,7 @@ int suli_upload(suli_ctx* c, int field, const double* host) {
     const int n0 = hi[0] - lo[0] + 1, n1 = hi[1] - lo[1] + 1, n2 = hi[2] - lo[2] + 1;
     const size_t n = (size_t)n0 * n1 * n2;
     if (is_plane(field)) {
-        CUDA_TRY(c, cudaMemcpyAsync(c->f[field], host, n * sizeof(double), cudaMemcpyDefault, c->stream));
+        CUDA_TRY(c, stream_copy(c, c->f[field], host, n * sizeof(double), cudaMemcpyDefault));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         return SULI_OK;
     }
@@ -417,7 +417,7 @@ int suli_upload(suli_ctx* c, int field, const double* host) {
     if (way == Way::direct) {
         repack<true>(c, field, host, c->f[field]);
     } else {   // stage through the CG q buffer (same size class as any field, free between calls)
-        CUDA_TRY(c, cudaMemcpyAsync(c->cg_q, host, n * sizeof(double), cudaMemcpyDefault, c->stream));
+        CUDA_TRY(c, stream_copy(c, c->cg_q, host, n * sizeof(double), cudaMemcpyDefault));
         repack<true>(c, field, c->cg_q, c->f[field]);
     }
     CHECK_LAUNCH(c);
@@ -433,7 +433,7 @@ int suli_download(suli_ctx* c, int field, double* host) {
     const int n0 = hi[0] - lo[0] + 1, n1 = hi[1] - lo[1] + 1, n2 = hi[2] - lo[2] + 1;
     const size_t n = (size_t)n0 * n1 * n2;
     if (is_plane(field)) {
-        CUDA_TRY(c, cudaMemcpyAsync(host, c->f[field], n * sizeof(double), cudaMemcpyDefault, c->stream));
+        CUDA_TRY(c, stream_copy(c, host, c->f[field], n * sizeof(double), cudaMemcpyDefault));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         return SULI_OK;
     }
@@ -442,7 +442,7 @@ int suli_download(suli_ctx* c, int field, double* host) {
     const bool direct = way == Way::direct;
     repack<false>(c, field, c->f[field], direct ? host : c->cg_q);
     CHECK_LAUNCH(c);
-    if (!direct) CUDA_TRY(c, cudaMemcpyAsync(host, c->cg_q, n * sizeof(double), cudaMemcpyDefault, c->stream));
+    if (!direct) CUDA_TRY(c, stream_copy(c, host, c->cg_q, n * sizeof(double), cudaMemcpyDefault));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return SULI_OK;
 }
@@ -504,9 +504,9 @@ int suli_set_obstacle(suli_ctx* c, const int* ku, const int* kv, const int* kw) 
         c->obst_kv = c->obst_k + nu;
         c->obst_kw = c->obst_k + nu + nv;
     }
-    CUDA_TRY(c, cudaMemcpyAsync(c->obst_k, ku, nu * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(c, cudaMemcpyAsync(c->obst_k + nu, kv, nv * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(c, cudaMemcpyAsync(c->obst_k + nu + nv, kw, nw * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, stream_copy(c, c->obst_k, ku, nu * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, stream_copy(c, c->obst_k + nu, kv, nv * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, stream_copy(c, c->obst_k + nu + nv, kw, nw * sizeof(int), cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->obst_ku_host.assign(ku, ku + nu);
     return SULI_OK;
@@ -552,8 +552,8 @@ int suli_iniciais(suli_ctx* c, double u_init) {
         }
     }
     if (c->P.wave_t == 0) {
-        CUDA_TRY(c, cudaMemcpyAsync(c->f[SULI_F_BXX0], bx0.data(), bx0.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-        CUDA_TRY(c, cudaMemcpyAsync(c->f[SULI_F_BXX1], bx1.data(), bx1.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        CUDA_TRY(c, stream_copy(c, c->f[SULI_F_BXX0], bx0.data(), bx0.size() * sizeof(double), cudaMemcpyHostToDevice));
+        CUDA_TRY(c, stream_copy(c, c->f[SULI_F_BXX1], bx1.data(), bx1.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
     const int tm = c->P.t_tempo;
     const double dt = c->P.dt;
@@ -767,7 +767,7 @@ void nn_begin(suli_ctx* c) {
             ProfScope ps(c, SULI_K_CG_SETUP, 2);
             launch_nn_features(c, c->rec_in);
         }
-        cudaMemcpyAsync(c->nn_e0, c->cg_e, c->g.n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
+        stream_copy(c, c->nn_e0, c->cg_e, c->g.n * sizeof(double), cudaMemcpyDeviceToDevice);
         return;
     }
     {   // the features go straight into the network's BF16 input
@@ -864,8 +864,8 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
     // direction (times 0), which must be finite, and a kernel that gave up in one CTA while others had
     // yet to start (they skip a solve that is done) has not all arrivals of its reduction.
     auto abandon = [&](int code, const char* why) -> int {
-        CUDA_TRY(c, cudaMemsetAsync(c->pc_pb, 0, c->g.n * sizeof(float), c->stream));
-        CUDA_TRY(c, cudaMemsetAsync(c->red_counter, 0, 64 * sizeof(unsigned int), c->stream));
+        CUDA_TRY(c, stream_zero(c, c->pc_pb, c->g.n * sizeof(float)));
+        CUDA_TRY(c, stream_zero(c, c->red_counter, 64 * sizeof(unsigned int)));
         return fail(c, code, why);
     };
     auto take_inner = [&]() -> int {
@@ -900,7 +900,7 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
         launch_pcg_begin(c);
         if (c->use_graphs) {
             ProfScope ps(c, SULI_K_MG, 0);   // kernel launches are counted below, once known
-            CUDA_TRY(c, cudaGraphLaunch(c->pcg_loop, c->stream));
+            CUDA_TRY(c, stream_graph(c, c->pcg_loop));
         } else {
             for (int pair = 0; pair < c->inner_maxit; ++pair) {
                 launch_pcg_pair(c);
@@ -909,7 +909,7 @@ int graddin_mixed(suli_ctx* c, int* iters, double* resid) {
                 if (c->pcg_host[0].done) break;
             }
         }
-        CUDA_TRY(c, cudaMemcpyAsync(c->pcg_host, c->pcg, sizeof(PCGState), cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(c, stream_copy(c, c->pcg_host, c->pcg, sizeof(PCGState), cudaMemcpyDeviceToHost));
         pcg_pending = true;
         launch_mx_residual(c, ecur, enext, true);
         std::swap(ecur, enext);
@@ -1081,7 +1081,7 @@ struct StepIO {
 };
 
 static int io_scatter(suli_ctx* c, int slot, int field) {
-    CUDA_TRY(c, cudaStreamWaitEvent(c->stream, c->io_ev[slot], 0));
+    CUDA_TRY(c, stream_wait(c, c->io_ev[slot]));
     repack<true>(c, field, c->io_stage[slot], c->f[field]);
     CHECK_LAUNCH(c);
     return SULI_OK;

@@ -41,10 +41,10 @@ __device__ __forceinline__ void coop_wait(CoopGrid& S) {
     if (lane == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(S.count) : "memory");
         unsigned int v;
-        int spin = 0;
+        int left = S.polls;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(S.count) : "memory");
-        } while ((int)(v - S.target) < 0 && ++spin < S.polls);
+        } while ((int)(v - S.target) < 0 && --left > 0);
         ok = (int)(v - S.target) >= 0;
         S.sh[66] = ok ? 0. : 1.;
     }

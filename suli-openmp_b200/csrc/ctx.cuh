@@ -176,8 +176,8 @@ struct suli_ctx {
     CUtensorMap smap[12];          // boxes with the halo
     CUtensorMap smap_own[12];      // the same arrays, boxes of the tile's own cells
     const float* smap_ptr[12] = {nullptr};
-    // the last thing put on the stream is a kernel of this call (step_launch; stream_copy and the like
-    // clear it); the calls suli_step is made of count as one
+    // what this call put on the stream last is a kernel, or complete (step_launch; stream_copy and the
+    // like clear it); the calls suli_step is made of count as one
     bool chained = false, in_step = false;
     int inner_maxit = 200;
     int inner_batch = 4;

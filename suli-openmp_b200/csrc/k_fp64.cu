@@ -1572,7 +1572,8 @@ static dim3 faces_grid(const Geo& g) { return grid3(g.nx + 1, g.ny + 1, g.nz + 1
 // Launch a kernel of the step (each calls pdl_wait first).  Behind another kernel of the same call
 // (c->chained) it is a dependent launch, which overlaps its start with the end of the one before:
 // the grids of a small step run shorter than a plain launch takes.  Behind anything else (a copy,
-// a memset, a graph, an event's wait, work a caller put on the stream) it is a plain launch.
+// a memset, a graph, an event's wait, work a caller put on the stream) it is a plain launch, unless the
+// host has waited for that (sync_read).
 template <typename... KArgs, typename... Args>
 static void step_launch(suli_ctx* c, void (*kernel)(KArgs...), dim3 grid, dim3 block, Args... args) {
     if (c->chained) pdl_launch(kernel, grid, block, c->stream, args...);

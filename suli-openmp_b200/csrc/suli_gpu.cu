@@ -113,6 +113,7 @@ void repack(suli_ctx* c, int field, const double* src, double* dst) {
 int sync_read(suli_ctx* c, const void* dev, void* host, size_t bytes) {
     CUDA_TRY(c, stream_copy(c, host, dev, bytes, cudaMemcpyDeviceToHost));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    c->chained = true;   // the copy is complete
     return SULI_OK;
 }
 

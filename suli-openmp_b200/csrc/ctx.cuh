@@ -189,9 +189,10 @@ struct suli_ctx {
     cudaGraphExec_t pcg_loop = nullptr;
     // the plain FP64 CG as one cooperative launch (k_cg_coop.cuh): CTAs the device holds at once and
     // their work area; 0 CTAs (the device cannot launch it, or SULI_NO_COOP=1): two kernels an
-    // iteration, launched from the host, whose sums are grouped differently
+    // iteration in a device-side loop, whose sums are grouped differently
     int coop_ctas = 0;
     double* coop_area = nullptr;   // in the arena
+    cudaGraphExec_t cg_loop = nullptr;
     int pcg_graph_kernels = 0;   // kernels of one inner iteration
     // learned initial guess (suli_attach_nn) and training-pair recording (suli_graddin_record)
     suli_nn* nn = nullptr;
@@ -200,7 +201,7 @@ struct suli_ctx {
     double* nn_e0 = nullptr;                     // e0 of a recorded solve (box layout)
     suli::NNScale* nn_scale = nullptr;
     float *rec_in = nullptr, *rec_target = nullptr;
-    // false (environment SULI_EAGER_LOOPS=1, for per-kernel profiling): the inner PCG
+    // false (environment SULI_EAGER_LOOPS=1, for per-kernel profiling): the inner PCG and the two-kernel CG
     // iterations are launched one by one from the host, two at a time with a check of the
     // device state after each pair, in place of the device-side graph loop; same kernels, same
     // order, same results
@@ -307,6 +308,7 @@ void launch_tempo(suli_ctx* c, int tt, int it);
 void launch_contorno(suli_ctx* c, int nlock);
 void launch_cg_setup(suli_ctx* c, bool mixed = false, bool mixed_residual = false);
 void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new);
+void launch_cg_cond(suli_ctx* c, cudaGraphConditionalHandle h);
 size_t coop_ready(suli_ctx* c);
 cudaError_t launch_cg_coop(suli_ctx* c);
 void launch_cg_divcheck(suli_ctx* c);

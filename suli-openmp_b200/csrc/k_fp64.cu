@@ -1451,6 +1451,12 @@ __global__ void __launch_bounds__(256) k_cg_divcheck(Geo G, const double* __rest
     }
 }
 
+// loop condition of the two-kernel iteration's graph: repeat until the state says done
+__global__ void k_cg_cond(cudaGraphConditionalHandle h, const CGState* st) {
+    pdl_wait();
+    cudaGraphSetConditional(h, st->done ? 0u : 1u);
+}
+
 // de-normalisation over the halo box (:268-274)
 __global__ void k_cg_final(Geo G, BC bc, const double* __restrict__ sdv, const double* __restrict__ e,
                            double* prd1, const CGState* st) {
@@ -1844,6 +1850,7 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
     step_launch(c, k_cg_update, gb, b, G, c->cg_e, c->cg_r, (const double*)p_new, (const double*)c->cg_q, c->cg,
                c->red_partial, c->red_counter);
 }
+void launch_cg_cond(suli_ctx* c, cudaGraphConditionalHandle h) { step_launch(c, k_cg_cond, 1, 1, h, c->cg); }
 // The cooperative solve: a register kernel while every cell fits the device's threads (one sum an
 // iteration where the operator is symmetric and, as k_cg_one sees on the device, the system has a
 // solution; else two), else the two-pass kernel.  Measured per

@@ -318,6 +318,7 @@ int suli_destroy(suli_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->pcg_loop) cudaGraphExecDestroy(c->pcg_loop);
+    if (c->cg_loop) cudaGraphExecDestroy(c->cg_loop);
     for (auto& e : c->prof.ev) cudaEventDestroy(e);
     cudaFree(c->arena);
     cudaFree(c->obst_k);
@@ -700,7 +701,7 @@ int suli_contorno(suli_ctx* c, int nlock) {
 }  // extern "C"
 
 namespace {
-// The inner solve's iterations as one graph launch: a WHILE conditional node whose body is two
+// A solver's iterations as one graph launch: a WHILE conditional node whose body is two
 // iterations (the direction vector ping-pongs between two buffers; every kernel reads its
 // scalars from device memory, so the captured parameters never change) and a kernel that clears
 // the condition once the solve has converged or hit its cap.  The GPU iterates without host
@@ -721,12 +722,14 @@ int make_loop_graph(suli_ctx* c, cudaGraphExec_t* out, Body body, Cond cond, con
     if (e == cudaSuccess)
         e = cudaStreamBeginCaptureToGraph(c->stream, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                           cudaStreamCaptureModeThreadLocal);
+    c->chained = false;   // nothing precedes the body's first kernel
     if (e == cudaSuccess) {
         body();
         cond(h);
         cudaGraph_t captured = nullptr;
         e = cudaStreamEndCapture(c->stream, &captured);
     }
+    c->chained = false;
     if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
@@ -746,6 +749,18 @@ int ensure_pcg_loop(suli_ctx* c) {
         return r;
     c->pcg_graph_kernels = pcg_iter_kernels(c);
     return SULI_OK;
+}
+
+// the plain FP64 CG as two kernels an iteration
+int ensure_cg_loop(suli_ctx* c) {
+    if (c->cg_loop) return SULI_OK;
+    return make_loop_graph(
+        c, &c->cg_loop,
+        [&] {
+            launch_cg_iter(c, c->cg_pa, c->cg_pb);
+            launch_cg_iter(c, c->cg_pb, c->cg_pa);
+        },
+        [&](cudaGraphConditionalHandle h) { launch_cg_cond(c, h); }, "CG graph");
 }
 
 // Mixed-precision solve: FP64 refinement around an FP32 multigrid-preconditioned CG.
@@ -790,7 +805,15 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
     launch_cg_setup(c);
     if (record) nn_begin(c);   // recording only: the learned guess needs the refinement loop
     CHECK_LAUNCH(c);
-    int done_iters = 0;   // iterations before this run of the loop (resumed solves)
+    int done_iters = 0;    // iterations before this run of the loop (resumed solves)
+    int graph_from = -1;   // iterations before the graph, its launches not yet counted
+    auto count_graph = [&] {
+        if (graph_from < 0) return;
+        const long long bodies = std::max(1, (c->cg_host[0].iters - graph_from + 1) / 2);
+        c->prof.launches[SULI_K_CG_SPMV] += 2 * bodies;
+        c->prof.launches[SULI_K_CG_UPDATE] += 2 * bodies;
+        graph_from = -1;
+    };
     auto run_loop = [&]() -> int {
         if (c->coop_ctas > 0) {
             const cudaError_t e = launch_cg_coop(c);
@@ -801,7 +824,20 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
         }
         // iteration 1 uses p_old = r with beta = 0 (erroppr = erropr, :172); iteration n writes its
         // direction to cg_pa for odd n, cg_pb for even n
-        for (int n = done_iters;; n += 2) {
+        int n = done_iters;
+        if (c->use_graphs) {   // the loop's body starts from cg_pa
+            if (int rg = ensure_cg_loop(c)) return rg;
+            if (n % 2 == 0) {
+                launch_cg_iter(c, n == 0 ? c->cg_r : c->cg_pb, c->cg_pa);
+                ++n;
+            }
+            CHECK_LAUNCH(c);
+            ProfScope ps(c, SULI_K_CG_SPMV, 0);   // kernel launches are counted below, once known
+            CUDA_TRY(c, stream_graph(c, c->cg_loop));
+            graph_from = n;
+            return SULI_OK;
+        }
+        for (;; n += 2) {
             double* cur = (n & 1) ? c->cg_pa : c->cg_pb;    // direction n (n >= 1), then n + 2
             double* nxt = (n & 1) ? c->cg_pb : c->cg_pa;   // direction n + 1
             launch_cg_iter(c, n == 0 ? c->cg_r : cur, nxt);
@@ -819,6 +855,7 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
         CHECK_LAUNCH(c);
         int rr = sync_read(c, c->cg, c->cg_host, sizeof(CGState));
         if (rr != SULI_OK) return rr;
+        count_graph();
         if (c->cg_host[0].done) break;
         done_iters = c->cg_host[0].iters;
         if (int rl = run_loop()) return rl;
@@ -829,6 +866,7 @@ int graddin_fp64(suli_ctx* c, int* iters, double* resid, bool record) {
     CHECK_LAUNCH(c);
     int r = sync_read(c, c->cg, c->cg_host, sizeof(CGState));
     if (r != SULI_OK) return r;
+    count_graph();
     const CGState& s = c->cg_host[0];
     c->prof.cg_iters += s.iters;
     if (iters) *iters = s.iters;

@@ -411,6 +411,7 @@ struct suli_nn {
     int kernel = 0;                  // convolution kernel: 0 tcgen05 pipeline, 1 mma.sync, 2 tcgen05 one tile per CTA
     float* part = nullptr;           // per-CTA partial sums of the parameter gradient (training)
     long long part_floats = 0;
+    int wg_ctas[3][4] = {{0}};       // CTAs of k_wgrad_tc<MB, NB> an SM holds (0: not asked yet)
     bool grad_error = false;         // the partial-sum buffer could not be allocated
     std::string err;
 };
@@ -620,17 +621,17 @@ void wgrad_tc(suli_nn* N, const Vol& vol, const ConvIn& in, int cout, const __nv
     using G = WgGeo<MB, NB>;
     const int cin = in.ca + in.cb;
     const long long width = 27LL * cout * cin + cout;   // dw then db, contiguous
-    static int ctas[64] = {0};   // CTAs an SM holds
-    if (!ctas[N->device]) {
+    int& ctas = N->wg_ctas[MB][NB];
+    if (!ctas) {
         cudaFuncSetAttribute(k_wgrad_tc<MB, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
         int n = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_wgrad_tc<MB, NB>, kWgThreads, G::SMEM) != cudaSuccess)
             cudaGetLastError();
-        ctas[N->device] = std::max(n, 1);
+        ctas = std::max(n, 1);
     }
     const int blocks = (cout / (16 * MB)) * (cin / (16 * NB));
     const long long columns = (long long)((vol.nx + kWgX - 1) / kWgX) * ((vol.ny + kWgY - 1) / kWgY);
-    const long long want = (long long)ctas[N->device] * sm_count(N->device) / (columns * blocks);
+    const long long want = (long long)ctas * sm_count(N->device) / (columns * blocks);
     const int segs = (int)std::max<long long>(1, std::min<long long>(want, vol.nz / 4));
     int seg = (vol.nz + segs - 1) / segs;
     if (!G::TOTALS) seg = std::min(seg, G::CHAIN);

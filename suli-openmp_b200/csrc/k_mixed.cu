@@ -705,18 +705,15 @@ static inline const float* mg_corr(const suli_ctx* c, int l) { return fused_leve
 
 // ---- level-0 kernels streaming z-planes through shared memory (k_mg_stream.cuh)
 static PFN_cuTensorMapEncodeTiled_v12000 plane_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {   // once, also with several threads
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
             q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        else
-            cudaGetLastError();
-    }
+            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+        cudaGetLastError();
+        return PFN_cuTensorMapEncodeTiled_v12000(nullptr);
+    }();
     return fn;
 }
 // a level-0 FP32 array as a 3-D tensor {px, py, nz + 3} (x = kBase + i - 1 within row j of

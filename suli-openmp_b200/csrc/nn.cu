@@ -463,18 +463,15 @@ void conv_tc(suli_nn* N, const Vol& vol, const ConvIn& in, const __nv_bfloat16* 
 
 // ---- the pipelined tcgen05 convolution (nn_tp.cuh): TMA descriptors and launch shape
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {   // once, also with several threads
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
             q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-        else
-            cudaGetLastError();
-    }
+            return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+        cudaGetLastError();
+        return PFN_cuTensorMapEncodeTiled_v12000(nullptr);
+    }();
     return fn;
 }
 // channels-last volume [nz][ny][nx][C]; box {8 channels, hx, hy, hz}, zero fill outside

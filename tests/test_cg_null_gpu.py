@@ -94,3 +94,24 @@ def test_balanced_system(pkg, monkeypatch, shape, tol):
             out[two] = (n, a - a.mean())
     assert abs(out[False][0] - out[True][0]) <= 3
     assert rel_err(out[False][1], out[True][1]) <= 1e4 * tol
+
+
+@pytest.mark.parametrize("tol", [3e-1, 1e-1, 3e-2, 1e-2])
+def test_threshold_lowered_past_the_rule(pkg, monkeypatch, tol):
+    """A solve that stops in the one-sum form, whose threshold the divergence test then lowers to nothing:
+    it goes on in the two-sum form from there.  Eighty iterations in all; thirty carry a sum's other
+    grouping to 1e-9 at most (test_cg_coop_gpu.py), and the error grows by a factor of ten a
+    thirty at most while the residual falls."""
+    p = small_params(14, 12, 10)
+    p.cg_stop, p.cg_tol, p.cg_maxit, p.div_tol = 1, tol, 80, 1e-30
+    out = []
+    for two in ("0", "1"):
+        monkeypatch.setenv("SULI_NO_COOP", two)
+        with pkg.Solver(p) as s:
+            load_state(s, seeded_state(p, 3))
+            s.heaviside()
+            s.set_dt(1e-3)
+            s.contorno(2)
+            out.append((s.graddin()[0], s.download("prd1")))
+    assert out[0][0] == out[1][0] == 80
+    assert rel_err(out[0][1], out[1][1]) <= 1e-7

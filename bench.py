@@ -494,35 +494,30 @@ def launch_share(profile: str, kernel: str, among: tuple):
 
 
 def cg_roofline(p, prof):
-    """Roofline of the plain path's dominant pass (p, q = A p and p.q) and of a whole CG iteration.
-    The solve is one cooperative launch, so CUDA events time the iteration; the pass's duration
-    is that time times the share of the same work (k_cg_spmv2) in the committed ncu launch list
-    of the form with two kernels an iteration (SULI_NO_COOP=1)."""
+    """Roofline of the plain path's CG: a whole iteration of k_cg_two, whose solve is one cooperative
+    launch, so CUDA events time the solves and the iteration is their mean."""
     N = p.nx * p.ny * p.nz
     faces = (p.nx + 1) * p.ny * p.nz + p.nx * (p.ny + 1) * p.nz + p.nx * p.ny * (p.nz + 1)
-    bytes_spmv = 8 * (4 * N + faces)
-    # r, q in, r out; every other iteration e in and out and the older direction (the newer one is
-    # read by the first pass)
-    bytes_upd = int(8 * 4.5 * N)
+    # first pass: r, the older direction, ax, ay, az in, p, q out, and every other iteration e in and
+    # out and the direction before; second pass: r, q in, r out
+    nbytes = 8 * (4 * N + faces) + int(8 * 1.5 * N) + 8 * 3 * N
     n_it = max(prof["cg_iterations"], 1)
     t_it = (prof["cg_spmv"]["ms"] + prof["cg_update"]["ms"]) / n_it / 1e3
-    share = launch_share("launches_sloshing_256x128x128_fp64", "k_cg_spmv2", ("k_cg_spmv2", "k_cg_update"))
     peak, peak_kind = measured_peaks()
-    it = {"kernels": "k_cg_two (both passes, one cooperative launch a solve)", "bytes": bytes_spmv + bytes_upd, "us": t_it * 1e6,
-          "achieved_gbs": (bytes_spmv + bytes_upd) / t_it / 1e9,
-          "frac": (bytes_spmv + bytes_upd) / t_it / 1e9 / peak}
-    t_spmv = t_it * (share if share else 1.0)
-    ach = bytes_spmv / t_spmv / 1e9
+    ach = nbytes / t_it / 1e9
+    share = launch_share("launches_sloshing_256x128x128_fp64", "k_cg_spmv2", ("k_cg_spmv2", "k_cg_update"))
     return {
-        "kernel": "k_cg_two, first pass (FP64 CG, two cells a thread: p = r + beta p, q = A p, p.q)",
+        "kernel": "k_cg_two (FP64 CG, one cooperative launch a solve), an iteration's two passes",
         "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
         "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback 6.65 TB/s",
-        "traffic": profiled_traffic("cg_spmv2_256x128x128", N), "algorithmic_bytes_per_launch": bytes_spmv,
-        "avg_launch_us": t_spmv * 1e6,
-        "duration": ("CUDA-event time of a CG iteration x k_cg_spmv2's share of the two-kernel form in "
-                     "profiles/launches_sloshing_256x128x128_fp64.txt" if share else
-                     "CUDA-event time of a whole CG iteration (no launch list to apportion it)"),
-        "cg_iteration": it,
+        "traffic": profiled_traffic("cg_two_256x128x128", N), "algorithmic_bytes_per_iteration": nbytes,
+        "duration": "CUDA-event time of the solves over their iterations",
+        "cg_iteration": {"kernels": "k_cg_two (both passes)", "bytes": nbytes, "us": t_it * 1e6, "achieved_gbs": ach,
+                         "frac": ach / peak},
+        # what the first kernel of the two-kernel form (SULI_NO_COOP=1) would take of an iteration as long as
+        # this one, by its share of the committed launch list; no pass of k_cg_two takes that time
+        "avg_launch_us": t_it * (share if share else 1.0) * 1e6,
+        "avg_launch_us_of": "k_cg_spmv2 in the two-kernel form, apportioned",
     }
 
 

@@ -173,7 +173,8 @@ const char* suli_last_error(const suli_ctx* c);
 int suli_synchronize(suli_ctx* c);
 
 /* Fortran-layout copies (c_loc of the module array).  Synchronous.  The pointer may be host
-   memory or device memory of any GPU (unified addressing decides the copy's direction). */
+   memory or device memory of any GPU (unified addressing decides the copy's direction).  An array
+   on the context's own GPU whose memory ends before the field does gives SULI_ERR_ARG. */
 int suli_upload(suli_ctx* c, int field, const double* host);
 int suli_download(suli_ctx* c, int field, double* host);
 int suli_set_scalar(suli_ctx* c, int scalar, double v);

@@ -1,10 +1,9 @@
 // k_cg_coop.cuh — the plain FP64 CG as one cooperative launch (included by k_fp64.cu).
 //
 // The two-kernel iteration (k_cg_spmv*, k_cg_update) costs two launches, two ramps and two
-// last-block reductions, whatever the grid: about 16-20 us on grids whose data the L2 holds and
-// whose arithmetic takes 1-2 us.  Here every CTA stays resident for the whole solve and an
-// iteration is two grid-wide sums (p.q, r.r), each also the barrier that publishes r (or p).
-//
+// last-block reductions, whatever the grid: about 17-20 us on grids whose data the L2 holds and
+// whose arithmetic takes 1-2 us.  Here every CTA stays resident for the whole solve, and an iteration's
+// grid-wide sums, one (k_cg_one) or two (p.q and r.r), are also the barriers that publish its vectors.
 #pragma once
 #include "k_coop.cuh"
 
@@ -51,7 +50,7 @@ __device__ __forceinline__ void coop_store(const CoopCG& s, bool failed, CGState
 // advances itself (p_nb = r_nb + beta p_nb, the owner's expression), so an iteration loads only r
 // at the neighbours and stores only r.  The directions end in cg_pa (resumed solves read it).
 // Cells are numbered along x, so the loads of a warp run along rows.  Bound by the latencies of
-// its two sums and of the neighbours' loads (25x50x45: 5.5 us an iteration, 17.5 with two kernels).
+// its two sums and of the neighbours' loads (25x50x45: 6.1 us an iteration, 19.7 with two kernels).
 template <int U, int NT>
 __device__ __forceinline__ void cg_reg(const Geo& G, const BC& bc, double* r, double* pa, double* e,
                                        const double* __restrict__ ax, const double* __restrict__ ay,
@@ -161,7 +160,7 @@ __global__ void __launch_bounds__(NT, 1) k_cg_reg(Geo G, BC bc, double* r, doubl
 // A resumed solve reads p and s, which end in cg_pa and cg_q; one whose threshold the divergence test
 // lowered past the rule goes on in the two-sum form from r, e and p.
 // Bound by the latency of its one sum, whose last part the neighbours' loads overlap: 3.4 us an
-// iteration at 25x50x45 where k_cg_reg takes 5.5, 3.8 at 64x32x48 against 6.0.
+// iteration at 25x50x45 where k_cg_reg takes 6.1, 3.7 at 64x32x48 against 6.7.
 constexpr double kNullPart = 1e-3;
 template <int U, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, double* pa, double* wa, double* wb, double* e,
@@ -286,10 +285,10 @@ __global__ void __launch_bounds__(NT, 1) k_cg_one(Geo G, BC bc, double* r, doubl
 // also applies the last two iterations' e -= alpha p (it reads the newer p anyway, and the older
 // where it writes its own), so the second only forms r; it takes the units in reverse order,
 // newest in the L2 first.  Iteration n (from 1) writes its direction into pa for odd n, pb for even
-// n.  Bound by the loads a thread's 64 registers keep in flight: 11.5 passes in 80 us at
-// 256x128x128, 4.8 TB/s (e updated in every iteration, 12 passes: 83.4; the two kernels' 13 passes:
-// 103.4).
-// Measured there: 512 threads of the same 87.7-97, 4 planes a unit 96, 8 planes 105, 1 plane 89.
+// n.  Bound by the loads a thread's 64 registers keep in flight: 11.5 passes in 78 us at
+// 256x128x128 (the two kernels' 13 in 110), the first pass 8.5 in 60 us, 4.7 TB/s, the second 3 in 18
+// us, 5.6 TB/s.  Measured there with e updated in every iteration (83.4 us): 512 threads of the same
+// 87.7-97, 4 planes a unit 96, 8 planes 105, 1 plane 89.
 template <int KZ, int NT>
 __global__ void __launch_bounds__(NT, 1) k_cg_two(Geo G, BC bc, double* r, double* pa, double* pb, double* q, double* e,
                                                   const double* __restrict__ ax, const double* __restrict__ ay,

@@ -656,8 +656,8 @@ __device__ __forceinline__ void convdiff_at(const Geo& G, const CDConst& C, cons
 #undef AT
 }
 
-// About 1500 instructions and 110 loads a face (measured: half of issue, 22 % of the FP64 pipe, a third
-// of L1; 60 % of the stalls wait for loads), so blocks an SM against registers decide: FP32 five
+// About 1400 instructions and 110 loads a face in FP64 (measured: 58 % of issue, 28 % of the FP64 pipe,
+// 44 % of L1; most stalls wait for loads), so blocks an SM against registers decide: FP32 five
 // blocks (6 at the compiler's own 40 registers: 0.75 -> 0.68 ms a 256x128x128 step; 4: 0.70), FP64 four
 // (3 at 78: 181 -> 162 us at 150x133x90 with der = 2; 5: 173).  In FP64 the rows away from the y and
 // z ends take loads at constant offsets (162 -> 148 us); in FP32 that spills and gave nothing.
@@ -1853,15 +1853,15 @@ void launch_cg_iter(suli_ctx* c, const double* p_old, double* p_new) {
 void launch_cg_cond(suli_ctx* c, cudaGraphConditionalHandle h) { step_launch(c, k_cg_cond, 1, 1, h, c->cg); }
 // The cooperative solve: a register kernel while every cell fits the device's threads (one sum an
 // iteration where the operator is symmetric and, as k_cg_one sees on the device, the system has a
-// solution; else two), else the two-pass kernel.  Measured per
-// iteration on a B200 (two kernels an iteration in a graph loop in brackets): k_cg_one 3.4 us at
-// 25x50x45 (17.5; k_cg_reg 5.5), 3.8 at 64x32x48 (16.5; 6.0), 5.3 at 57x49x53 (17.9); above its
-// 151,552 cells on 148 SMs k_cg_two 12.9 at 64x64x48 (16.8), 14.9 at 80^3 (20.4), 31.0 at
-// 111x110x110 (41.8), 47.2 at 128^3 (55.8), 83.4 at 256x128x128 (103.4), 617 at 512x256x256 (708); since then
-// k_cg_two updates e every other iteration, 80 at 256x128x128.
+// solution; else two), else the two-pass kernel.  Microseconds an iteration on a B200 (in brackets two
+// kernels an iteration in a device-side loop):
+//   k_cg_one, k_cg_reg: 2.8, 4.7 at 40x20x24 (17.0), 3.4, 6.1 at 25x50x45 (19.7), 3.7, 6.7 at 64x32x48
+//   (18.3), 5.1, 7.8 at 57x49x53 (20.4); they hold up to 151,552 cells on 148 SMs;
+//   k_cg_two: 12.9 at 64x64x48 (18.3), 15.1 at 80^3 (21.7), 31.3 at 111x110x110 (46), 45 at 128^3 (62),
+//   78 at 256x128x128 (110), 538 at 512x256x256 (758).
 // The register kernels hold three cells a thread while that fits (113,664 cells), else four, at
-// which they spill: k_cg_one 2.8 us instead of 3.5 at 40x20x24, 3.43 instead of 3.84 at 25x50x45,
-// 3.77 instead of 4.07 at 64x32x48.  Two cells a thread, or 192 to 384 threads: no better.
+// which k_cg_one spills: with four everywhere it took 3.5 us at 40x20x24, 3.84 at 25x50x45 and 4.07 at
+// 64x32x48.  Two cells a thread, or 192 to 384 threads: no better.
 constexpr int kRegNT = 256, kRegMaxU = 4, kTwoKZ = 2, kTwoNT = 1024;
 constexpr int one_smem(int u) { return 8 * u * kRegNT * (int)sizeof(double); }
 static bool cg_symmetric(const suli_ctx* c) { return c->bc.wrapf || !(c->bc.perx || c->bc.pery || c->bc.perz); }

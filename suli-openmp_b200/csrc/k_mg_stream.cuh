@@ -27,7 +27,7 @@
 // density needs none: faces at the box's end take the next interior face's value.)  The inner
 // solves of a 512x256x256 channel step, on the vectorised kernels before: 58.9 -> 49.0 ms.
 //
-// Issue-bound as much as bandwidth-bound (50-56 % of issue slots at 256x128x128), so a march keeps
+// Issue-bound as much as bandwidth-bound (45-53 % of issue slots and 2.6-3.9 TB/s at 256x128x128), so a march keeps
 // the quad's values below and at the plane, and the density at it, in registers (SCol, SZCarry):
 // one shared-memory quad and its arithmetic a plane instead of three (inner solves of a 256x128x128
 // step 8.38 -> 8.21 ms).  A deeper ring, loads of the fixed fields ahead of the wait for the

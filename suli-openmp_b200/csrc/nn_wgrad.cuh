@@ -10,10 +10,11 @@
 // all 3 x 2 MB NB accumulator tiles in registers, so no partial sums are exchanged.  Rows are padded
 // by 16 bytes, which makes the eight row addresses of an ldmatrix phase hit distinct banks.
 //
-// The earlier kernel gave a CTA one tap and staged both operands again for each of the 27.
-// Measured at 128^3 (before -> here): 16 -> 16 channels 1709 -> 150 us, 48 -> 16 3033 -> 344 us,
-// 96 -> 32 at 64^3 800 -> 240 us; a gradient of the whole network 14.7 -> 4.9 ms.  Bound by the
-// mma.sync rate and the ldmatrix reads (L1 60 % busy; 27 instead of 18 warps an SM change nothing).
+// Measured at 128^3 (in brackets one tap a CTA, which stages both operands 27 times): 16 -> 16 channels
+// 150 us (1709), 48 -> 16 344 (3033), 96 -> 32 at 64^3 240 (800); a gradient of the whole network 4.9
+// ms (14.7).  No unit is full: the tensor pipe is busy 41-52 % of the time, L1 with the ldmatrix reads
+// 38-63 %; the warps wait for fixed latencies and at the plane's barrier (27 instead of 18 warps an SM
+// change nothing).
 // Why mma.sync: 16-channel layers have a 16 x 16 output a tap, far below tcgen05's 64-row minimum,
 // and the taps' shifted operands have no uniform stride that would stack them into its rows.
 //

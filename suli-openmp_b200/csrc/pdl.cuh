@@ -14,7 +14,7 @@
 
 namespace suli {
 
-constexpr unsigned int kPdlEarlyBlocks = 148;   // one a B200 SM
+constexpr unsigned int kPdlEarlyBlocks = 148;   // one an SM of a B200, the only part this is built for
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (gridDim.x * gridDim.y * gridDim.z <= kPdlEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -38,8 +38,8 @@ struct CGState {
     int gave_up;      // a CTA's wait in the cooperative CG ran out (k_coop.cuh)
     double div_tol;   // suli_params.div_tol (0: off)
     double rmax;      // max |sqrt(d) r~| of the last check: the max |div u| projection leaves
-    double null2;     // square of r~'s part along the null vector sqrt(d) (plain set-up), which no
-                      // iteration reduces: the floor of r~.r~
+    double null2;     // square of r~'s part along the null vector sqrt(d), which no iteration reduces:
+                      // the floor of r~.r~ (infinite where the solve's kernel does not ask)
 };
 
 // State of the FP32 inner preconditioned CG of the mixed-precision solve (device resident).

@@ -1172,13 +1172,14 @@ __global__ void __launch_bounds__(256) k_cg_diag(Geo G, BC bc, CGConst K, const 
 
 // scaled face coefficients s/sqrt(d_c d_nb) = s * (1/sqrt(d_c)) * (1/sqrt(d_nb)) and the first
 // residual (:126-151); reduction of r.r and b.b.  Plain: the reference's residual, whose
-// neighbours outside the box are prd1's ghosts, and its part along the null vector (null2).  MX: the refinement's residual (k_mx_outer: ghosts
-// map to cells), rounded to FP32 as the inner solve's right-hand side r_u = sqrt(d) r~, with
+// neighbours outside the box are prd1's ghosts; NP: with its part along the null vector (null2, of
+// the solves that may take k_cg_one; two more sums).  MX: the refinement's residual (k_mx_outer:
+// ghosts map to cells), rounded to FP32 as the inner solve's right-hand side r_u = sqrt(d) r~, with
 // its sums; the refinement's own first pass over the coefficients is saved (set-up and refinement
 // of a 256x128x128 step 1.86 -> 1.59 ms).  Forming the faces from the density here and in
 // k_cg_diag instead of reading them back was no faster: five more FP64 divisions a cell.
 constexpr int kCoefZ = 4;
-template <bool MX>
+template <bool MX, bool NP>
 __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, const double* __restrict__ sx,
                                                     const double* __restrict__ sy, const double* __restrict__ sz,
                                                     const double* __restrict__ sd, const double* __restrict__ isd,
@@ -1231,17 +1232,21 @@ __global__ void __launch_bounds__(256, 4) k_cg_coef(Geo G, BC bc, CGConst K, con
             um = fmax(um, fabs(uv));
         } else {
             r[c] = rv;
-            zr += sd[c] * rv;
-            zz += sd[c] * sd[c];
+            if (NP) {
+                zr += sd[c] * rv;
+                zz += sd[c] * sd[c];
+            }
         }
     }
     }
-    double trr, tbb, tru2 = 0.0, tum = 0.0, tnull = 0.0;
+    double trr, tbb, tru2 = 0.0, tum = 0.0, tnull = INFINITY;
     bool last;
     if (MX) {
         double s[3] = {rr, bbv, ru2}, t[3];
         last = reduce_sums_max_last<3>(s, um, partial, counter, t, tum);
         trr = t[0]; tbb = t[1]; tru2 = t[2];
+    } else if (!NP) {
+        last = reduce2_last(rr, bbv, partial, counter, trr, tbb);
     } else {
         double s[4] = {rr, bbv, zr, zz}, t[4];
         last = reduce_sums_max_last<4>(s, 0.0, partial, counter, t, tum);
@@ -1805,6 +1810,7 @@ static CGConst cg_const(const suli_ctx* c) {
     K.maxit = c->P.cg_maxit;
     return K;
 }
+static bool cg_one_fits(const suli_ctx* c);
 // mixed: also level 0 of the multigrid; mixed_residual: the refinement's first residual in place of
 // the plain path's
 void launch_cg_setup(suli_ctx* c, bool mixed, bool mixed_residual) {
@@ -1824,7 +1830,7 @@ void launch_cg_setup(suli_ctx* c, bool mixed, bool mixed_residual) {
     step_launch(c, k_cg_diag, cells_grid(G), kBlk, G, c->bc, K, sx, sy, sz, c->f[SULI_F_U], c->f[SULI_F_V], c->f[SULI_F_W],
                                                       c->f[SULI_F_PRD1], c->rec_in ? c->cg_d : nullptr, c->cg_e, c->cg_b,
                                                       c->cg_sd, c->cg_isd);
-    const auto coef = mixed_residual ? k_cg_coef<true> : k_cg_coef<false>;
+    const auto coef = mixed_residual ? k_cg_coef<true, false> : !mixed && cg_one_fits(c) ? k_cg_coef<false, true> : k_cg_coef<false, false>;
     step_launch(c, coef, grid3(G.nx, G.ny, (G.nz + kCoefZ - 1) / kCoefZ, kBlk), kBlk, G, c->bc, K, sx, sy, sz, c->cg_sd, c->cg_isd, c->cg_e, c->cg_b, c->f[SULI_F_PRD1], c->cg_ax, c->cg_ay, c->cg_az,
         c->cg_r, c->cg, c->red_partial, c->red_counter, M);
 }
@@ -1865,6 +1871,10 @@ void launch_cg_cond(suli_ctx* c, cudaGraphConditionalHandle h) { step_launch(c, 
 constexpr int kRegNT = 256, kRegMaxU = 4, kTwoKZ = 2, kTwoNT = 1024;
 constexpr int one_smem(int u) { return 8 * u * kRegNT * (int)sizeof(double); }
 static bool cg_symmetric(const suli_ctx* c) { return c->bc.wrapf || !(c->bc.perx || c->bc.pery || c->bc.perz); }
+// solves of which k_cg_one takes those that have a solution
+static bool cg_one_fits(const suli_ctx* c) {
+    return cg_symmetric(c) && (long long)c->P.nx * c->P.ny * c->P.nz <= (long long)kRegMaxU * kRegNT * c->coop_ctas;
+}
 // whether the device runs them; returns their work area's 8-byte elements
 size_t coop_ready(suli_ctx* c) {
     c->coop_ctas = 0;
@@ -1913,7 +1923,7 @@ cudaError_t launch_cg_coop(suli_ctx* c) {
     const long long per = (long long)u * kRegNT;
     if (cells <= per * c->coop_ctas) {
         const dim3 ctas((unsigned)((cells + per - 1) / per));
-        if (cg_symmetric(c)) {
+        if (cg_one_fits(c)) {
             void* args[] = {(void*)&G, &c->bc, &c->cg_r, &c->cg_pa, &c->cg_q, &c->cg_pb, &c->cg_e, &ax, &ay, &az, &c->cg,
                             &c->coop_area, &polls};
             const void* k = u == 3 ? (const void*)k_cg_one<3, kRegNT> : (const void*)k_cg_one<kRegMaxU, kRegNT>;

@@ -377,16 +377,19 @@ static Way copy_way(const suli_ctx* c, const void* p, size_t bytes) {
         return Way::staged;
     }
     if (a.type != cudaMemoryTypeDevice || a.device != c->device) return Way::staged;
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
+    static const PFN_cuMemGetAddressRange_v3020 fn = [] {   // once, also with several threads
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
         cudaGetLastError();
-        return Way::staged;
-    }
+        return PFN_cuMemGetAddressRange_v3020(nullptr);
+    }();
+    if (!fn) return Way::staged;
     const RangeKind kind = range_kind(reinterpret_cast<uintptr_t>(p), bytes, [&](uintptr_t at, uintptr_t* base, size_t* size) {
         CUdeviceptr b = 0;
-        if (reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(fn)(&b, size, (CUdeviceptr)at) != CUDA_SUCCESS) return false;
+        if (fn(&b, size, (CUdeviceptr)at) != CUDA_SUCCESS) return false;
         *base = (uintptr_t)b;
         return true;
     });
